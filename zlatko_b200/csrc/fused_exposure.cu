@@ -4,8 +4,8 @@
 // src/gpu/fused_kernels.cpp:224-530, and its CPU mirror simulatePath,
 // src/gpu/fused_reference.cpp:198-422), organised for a B200 and for books of many netting sets:
 //
-//   simulateKernel   one thread per path draws the counter-based normals, correlates them and steps
-//                    Hull-White, the lognormal assets and the CIR++ intensities once per date, writing
+//   simulateKernel   producer warps draw the counter-based normals and correlate them, ahead of the warps that
+//                    step Hull-White, the lognormal assets and the CIR++ intensities once per date, writing
 //                    the factor state (x, D, S, Q; lnS and y when probes read them) path-major to HBM.
 //                    Every netting set of the launch reuses it: the reference re-simulates per plan.
 //                    Only factors are stored, never the paths x dates x trades value cube.
@@ -18,6 +18,8 @@
 //                    warp reduce-scatter (9 shuffles) and one cross-warp pass per 128-path group into
 //                    per-group partials, which the reduce kernel sums in path order: the results are
 //                    deterministic and the same for every tile shape.
+#include <algorithm>
+
 #include "zk_device.cuh"
 #include "zk_kernels.h"
 
@@ -107,200 +109,66 @@ __device__ __forceinline__ R swapRate(R flt, R ann) {
   return ann != R(0) ? flt / ann : R(0);
 }
 
-constexpr int kSimThreads = 256;  // threads per CTA of the simulate kernel (one path each)
+constexpr int kSimWarps = 8, kSimThreads = 32 * kSimWarps;  // warps and threads per CTA of the simulate kernel
 
-// The normals of one date: every Box-Muller pair drawn up front (independent of one another, so they overlap),
-// or the injected normals, into this thread's column of shared memory, normal m at col[m * kSimThreads].
-template <typename R>
-__device__ __forceinline__ void drawDate(uint32_t stream, uint32_t j, R sign, const R* injected, uint32_t nStreams,
-                                         uint32_t injectedStream, uint32_t nNormals, R* col) {
-  if (injected) {
-    for (uint32_t m = 0; m < nNormals; ++m)
-      col[m * kSimThreads] = sign * injected[(static_cast<size_t>(j - 1) * nNormals + m) * nStreams + injectedStream];
-    return;
-  }
+// The simulate kernel's shared memory (values of R): a ring of two buffers of `dates` dates, each date `slots` values of the
+// CTA's streams, then, with `table`, the Brownian-bridge coefficients [nT][substeps - 1][2].  `need` normals are read
+// per date.
+struct SimLayout {
+  uint32_t need, slots, dates;
+  bool table;
+};
+
+// The drivers of one (stream, date) into its ring column, slot m at col[m * cols]: the correlated drivers w_0 .. w_{nCorr-1},
+// the independent normals of the integrated rates, and per credit the Brownian increments of its sub-steps (the last one
+// after all normals, slot need + c).  The Box-Muller pairs are independent of one another, so they overlap.
+template <typename R, uint32_t cols>
+__device__ __forceinline__ void drawDate(const ScenarioArgs<R>& sc, const SimLayout& L, uint32_t stream, uint32_t j, uint32_t injectedStream,
+                                         const R* bridge, R* col) {
+  const uint32_t nB = sc.substeps - 1;
+  if (sc.normals) {
+    for (uint32_t m = 0; m < L.need; ++m)
+      col[m * cols] = sc.normals[(static_cast<size_t>(j - 1) * sc.nNormals + m) * sc.nStreams + injectedStream];
+  } else {
 #pragma unroll 4
-  for (uint32_t q = 0; 2 * q < nNormals; ++q) {
-    R z0, z1;
-    gauss2(stream, j, q, z0, z1);
-    col[2 * q * kSimThreads] = sign * z0;
-    if (2 * q + 1 < nNormals) col[(2 * q + 1) * kSimThreads] = sign * z1;
+    for (uint32_t q = 0; 2 * q < L.need; ++q) {
+      R z0, z1;
+      gauss2(stream, j, q, z0, z1);
+      col[2 * q * cols] = z0;
+      if (2 * q + 1 < L.need) col[(2 * q + 1) * cols] = z1;
+    }
+  }
+  // Correlated drivers: each padded Cholesky row as two 4-term dot products (as the reference).
+  R z[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) z[k] = static_cast<uint32_t>(k) < sc.nCorr ? col[k * cols] : R(0);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (static_cast<uint32_t>(i) < sc.nCorr) {
+      const R* row = sc.chol + i * kChol;
+      const R d0 = fma(row[3], z[3], fma(row[2], z[2], fma(row[0], z[0], row[1] * z[1])));
+      const R d1 = fma(row[7], z[7], fma(row[6], z[6], fma(row[4], z[4], row[5] * z[5])));
+      col[i * cols] = d0 + d1;
+    }
+  if (sc.nC == 0) return;
+  const R dt = __ldg(sc.steps + static_cast<size_t>(j) * sc.stepStride + 6), h = dt / static_cast<R>(sc.substeps);
+  const R* bj = bridge + static_cast<size_t>(j) * nB * 2;
+  for (uint32_t c = 0; c < sc.nC; ++c) {
+    R* zc = col + (sc.nCorr + 1 + sc.nF + c * nB) * cols;
+    R rem = rsqrt_(dt) * col[(1 + sc.nA + c) * cols], remT = dt;
+    for (uint32_t s = 0; s < nB; ++s) {
+      const R a = L.table ? bj[2 * s] : h / remT;
+      const R b = L.table ? bj[2 * s + 1] : rsqrt_(fmax(h * (remT - h) / remT, R(0)));
+      const R dW = fma(a, rem, b * zc[s * cols]);
+      zc[s * cols] = dW;
+      rem -= dW;
+      remT -= h;
+    }
+    col[(L.need + c) * cols] = rem;
   }
 }
 
 }  // namespace
-
-// ---------------------------------------------------------------------------------------------
-// Risk factors of every path and date (the transitions of the reference's ScenarioGenerator:
-// hull_white.cpp:40-68, lognormal_asset.cpp:17-22, cir_intensity.cpp:49-66, in the statement order
-// of the reference kernel).
-template <typename R>
-__global__ void __launch_bounds__(kSimThreads) simulateKernel(const ScenarioArgs<R> sc, CubeArgs<R> cb, bool bridgeTable) {
-  extern __shared__ __align__(16) unsigned char simRaw[];
-  R* col = reinterpret_cast<R*>(simRaw) + threadIdx.x;  // this thread's normals of the current date
-  // The Brownian-bridge coefficients of the CIR sub-steps are the same for every path: with bridgeTable the
-  // CTA computes them once, [date][sub-step][a, b] after the normals, by the very operations of the loop below.
-  const uint32_t nB = sc.substeps - 1;
-  R* bridge = reinterpret_cast<R*>(simRaw) + static_cast<size_t>(sc.nNormals) * kSimThreads;
-  if (bridgeTable) {
-    for (uint32_t jj = threadIdx.x + 1; jj < sc.nT; jj += blockDim.x) {
-      const R dt = sc.steps[static_cast<size_t>(jj) * sc.stepStride + 6], h = dt / static_cast<R>(sc.substeps);
-      R remT = dt;
-      for (uint32_t q = 0; q < nB; ++q) {
-        bridge[(static_cast<size_t>(jj) * nB + q) * 2] = h / remT;
-        bridge[(static_cast<size_t>(jj) * nB + q) * 2 + 1] = rsqrt_(fmax(h * (remT - h) / remT, R(0)));
-        remT -= h;
-      }
-    }
-    __syncthreads();
-  }
-  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= sc.nP) return;
-  const uint32_t nP = sc.nP, nT = sc.nT;
-  const uint32_t po = sc.pathMap ? sc.pathMap[p] : p;  // the plan's path this thread simulates
-  R sign = R(1);
-  uint32_t pathStream = po;
-  if (sc.antithetic) {
-    pathStream = po >> 1u;
-    if (po & 1u) sign = R(-1);
-  }
-  const uint32_t injectedStream = sc.nStreams > 0 ? min(pathStream, sc.nStreams - 1) : 0u;
-  const uint32_t stream = pcg(pcg(sc.seed) ^ pcg(pathStream + 0x9E3779B9u));
-  auto normal = [&](uint32_t m) { return col[m * kSimThreads]; };
-  // The deflator's exponent -sum of the integrated short rate accumulates in double precision in both modes (the
-  // reference's kernel sums it in single precision, fused_kernels.cpp:250-253); D = exp(lnD) is then taken in R.
-  R x = R(0), D = R(1);
-  double lnD = 0.0;
-  R S[4], lnS[4] = {R(0), R(0), R(0), R(0)}, y[2], Y[2] = {R(0), R(0)};
-  R xf[2] = {R(0), R(0)};  // stochastic foreign short-rate states of assets 0 and 1
-#pragma unroll
-  for (int a = 0; a < 4; ++a) S[a] = sc.spots[a];
-#pragma unroll
-  for (int c = 0; c < 2; ++c) y[c] = sc.cir[4 * c + 3];
-  auto put = [&](uint32_t field, uint32_t j, R v) { cb.data[(static_cast<size_t>(field) * nT + j) * nP + p] = v; };
-
-  for (uint32_t j = 0; j < nT; ++j) {
-    R Qc[2] = {R(1), R(1)};
-    if (j > 0) {
-      const R* step = sc.steps + static_cast<size_t>(j) * sc.stepStride;
-      drawDate<R>(stream, j, sign, sc.normals, sc.nStreams, injectedStream, sc.nNormals, col);
-      // Correlated drivers: each padded Cholesky row as two 4-term dot products (as the reference).
-      R z[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) z[k] = static_cast<uint32_t>(k) < sc.nCorr ? normal(k) : R(0);
-      R w[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const R* row = sc.chol + i * kChol;
-        const R d0 = row[0] * z[0] + row[1] * z[1] + row[2] * z[2] + row[3] * z[3];
-        const R d1 = row[4] * z[4] + row[5] * z[5] + row[6] * z[6] + row[7] * z[7];
-        w[i] = d0 + d1;
-      }
-      const R zI = normal(sc.nCorr);
-      const R integratedRate = x * step[5] + step[2] * w[0] + step[3] * zI + step[4];
-      x = x * step[0] + step[1] * w[0];
-      lnD -= static_cast<double>(integratedRate);
-      D = rexp(static_cast<R>(lnD));
-      // Stochastic foreign rates: the exact Hull-White step of x_f (with its quanto drift) and of its integral, on
-      // driver 1 + nA + nC + f and the independent normal nCorr + 1 + f; the asset's carry is then the simulated
-      // integral of r_f instead of the deterministic one.
-      R carry[4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) carry[a] = step[8 + a];
-#pragma unroll
-      for (int f = 0; f < 2; ++f) {
-        if (static_cast<uint32_t>(f) < sc.nF) {
-          const R* fs = step + kStepStride + 8 * f;
-          const uint32_t wi = 1 + sc.nA + sc.nC + f;
-          R wf = w[7];
-#pragma unroll
-          for (int i = 6; i >= 0; --i)
-            if (wi == static_cast<uint32_t>(i)) wf = w[i];
-          const R zf = normal(sc.nCorr + 1 + f);
-          carry[f] = xf[f] * fs[5] + fs[2] * wf + fs[3] * zf + fs[4] + fs[7];
-          xf[f] = xf[f] * fs[0] + fs[1] * wf + fs[6];
-        }
-      }
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        if (static_cast<uint32_t>(a) < sc.nA) {
-          lnS[a] = lnS[a] + (integratedRate - carry[a] - step[16 + a] + step[12 + a] * w[1 + a]);
-          S[a] = sc.spots[a] * rexp(lnS[a]);
-        }
-      }
-      const R dt = step[6];
-      uint32_t off = sc.nCorr + 1 + sc.nF;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        if (static_cast<uint32_t>(c) < sc.nC) {
-          const R kappa = sc.cir[4 * c], theta = sc.cir[4 * c + 1], xi = sc.cir[4 * c + 2];
-          const R h = dt / static_cast<R>(sc.substeps);
-          const uint32_t wi = 1 + sc.nA + c;
-          R wc = w[7];
-#pragma unroll
-          for (int i = 6; i >= 0; --i)
-            if (wi == static_cast<uint32_t>(i)) wc = w[i];
-          R rem = rsqrt_(dt) * wc, remT = dt, yy = y[c], YY = Y[c];
-          const R* bj = bridge + static_cast<size_t>(j) * nB * 2;
-          for (uint32_t s = 0; s < sc.substeps; ++s) {
-            R dW = rem;
-            if (s + 1 < sc.substeps) {
-              const R a = bridgeTable ? bj[2 * s] : h / remT;
-              const R b = bridgeTable ? bj[2 * s + 1] : rsqrt_(fmax(h * (remT - h) / remT, R(0)));
-              dW = a * rem + b * normal(off + s);
-            }
-            rem -= dW;
-            remT -= h;
-            const R yp = fmax(yy, R(0));
-            const R yn = yy + kappa * (theta - yp) * h + xi * rsqrt_(yp) * dW;
-            YY += R(0.5) * (yp + fmax(yn, R(0))) * h;
-            yy = yn;
-          }
-          y[c] = yy;
-          Y[c] = YY;
-          off += sc.substeps - 1;
-          Qc[c] = rexp(-Y[c] - step[20 + c]);
-        }
-      }
-    }
-    put(0, j, x);
-    put(1, j, D);
-    for (uint32_t a = 0; a < sc.nA; ++a) put(cb.fS + a, j, sel4(S, a));
-    for (uint32_t c = 0; c < sc.nC; ++c) put(cb.fQ + c, j, c == 0 ? Qc[0] : Qc[1]);
-    for (uint32_t f = 0; f < sc.nF; ++f) put(cb.fXf + f, j, f == 0 ? xf[0] : xf[1]);
-    if (cb.probes) {
-      for (uint32_t a = 0; a < sc.nA; ++a) put(cb.fLnS + a, j, sel4(lnS, a));
-      for (uint32_t c = 0; c < sc.nC; ++c) put(cb.fY + c, j, c == 0 ? y[0] : y[1]);
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------------------------
-// The exponential of a lowered term: 2^(b x) with b = -B log2 e in single precision, e^(b x) with b = -B
-// in double (lowerTerms, capi.cu).
-__device__ __forceinline__ float termExp(float b, float x) { return ex2(b * x); }
-__device__ __forceinline__ double termExp(double b, double x) { return exp(b * x); }
-
-template <typename R> struct Vec4;
-template <> struct Vec4<float> { using T = float4; };
-template <> struct Vec4<double> { using T = double4; };
-__device__ __forceinline__ float4 ld4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
-__device__ __forceinline__ double4 ld4(const double* p) {
-  const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
-  return make_double4(a.x, a.y, b.x, b.y);
-}
-
-// Prefetches into L1 the 128-byte lines of one date's lowered terms, one line per thread of the CTA:
-// the next date's block arrives while the current date computes.
-__device__ __forceinline__ void prefetchL1(const void* p) {
-  asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(p)));
-}
-template <typename R>
-__device__ __forceinline__ void prefetchDate(uint32_t begin, uint32_t end, const R* table, uint32_t tid) {
-  const size_t b = static_cast<size_t>(begin) * 4 * sizeof(R), e = static_cast<size_t>(end) * 4 * sizeof(R);
-  const uint32_t lines = e > b ? static_cast<uint32_t>((e - 1) / 128 - b / 128 + 1) : 0u;
-  if (tid < lines) prefetchL1(reinterpret_cast<const char*>(table) + (b / 128 + tid) * 128);
-}
 
 // A thread's PPT adjacent paths in one 8- or 16-byte access (p aligned to PPT values).
 template <typename R, int PPT>
@@ -333,6 +201,234 @@ __device__ __forceinline__ void stPaths(R* p, const R (&v)[PPT]) {
 #pragma unroll
     for (int q = 0; q < PPT; q += 2) reinterpret_cast<double2*>(p)[q / 2] = make_double2(v[q], v[q + 1]);
   }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Risk factors of every path and date (the transitions of the reference's ScenarioGenerator:
+// hull_white.cpp:40-68, lognormal_asset.cpp:17-22, cir_intensity.cpp:49-66, in the statement order
+// of the reference kernel; the fused multiply-adds are written out so that every shape rounds alike).
+//
+// Only the states are serial in the dates; the normals and everything linear in them (correlation, Brownian bridge) are
+// not, and they are most of the work.  So a CTA takes `cols` normal streams with eight warps: one steps the rates and the
+// assets, one per credit steps its CIR++ intensity, and the others produce the drivers of several dates ahead into a
+// shared-memory ring.  An antithetic pair's drivers differ by their sign only (exactly, rounding being symmetric), so
+// they are produced once per pair: with 32 streams a lane steps both paths of its stream (PPL = 2: two independent
+// chains of the CIR++ sub-steps' square roots, which bind), with 16 streams adjacent lanes share one and a producer pass
+// covers two dates.  Without pairs a stream is a path.
+// Before (one thread drew and stepped a path): 389 us at 2,000 paths x 121 dates, 4 factors, 1,159 us at 100,000 x 169,
+// 6 factors, 4,800 us at 500,000.  16 streams: 80, 991 and 4,433 us; 32: 108, 735 and 3,475 us.
+template <typename R, int PPL, uint32_t cols>
+__global__ void __launch_bounds__(kSimThreads, sizeof(R) == 4 ? 4 : 2) simulateKernel(const ScenarioArgs<R> sc, const CubeArgs<R> cb,
+                                                                                     const SimLayout L) {
+  extern __shared__ __align__(16) unsigned char simRaw[];
+  R* ring = reinterpret_cast<R*>(simRaw);
+  const uint32_t bufLen = L.dates * L.slots * cols;
+  R* bridge = ring + 2 * static_cast<size_t>(bufLen);
+  // The Brownian-bridge coefficients of the CIR sub-steps are the same for every path: with L.table the CTA computes
+  // them once.
+  const uint32_t nB = sc.substeps - 1, nP = sc.nP, nT = sc.nT;
+  if (L.table) {
+    for (uint32_t jj = threadIdx.x + 1; jj < nT; jj += blockDim.x) {
+      const R dt = sc.steps[static_cast<size_t>(jj) * sc.stepStride + 6], h = dt / static_cast<R>(sc.substeps);
+      R remT = dt;
+      for (uint32_t q = 0; q < nB; ++q) {
+        bridge[(static_cast<size_t>(jj) * nB + q) * 2] = h / remT;
+        bridge[(static_cast<size_t>(jj) * nB + q) * 2 + 1] = rsqrt_(fmax(h * (remT - h) / remT, R(0)));
+        remT -= h;
+      }
+    }
+    __syncthreads();
+  }
+  // The roles rotate with the CTA over the warps, so that the resident CTAs load the four schedulers alike.
+  const uint32_t lane = threadIdx.x & 31u, role = ((threadIdx.x >> 5) + blockIdx.x) & (kSimWarps - 1u);
+  const uint32_t numProducers = kSimWarps - 1 - sc.nC;
+  const uint32_t blocks = nT > 1 ? (nT - 1 + L.dates - 1) / L.dates : 0u;  // ring buffers, dates 1 .. nT - 1
+  // This lane's first path p0 (with PPL = 2, p0 + 1 is the antithetic one) and its stream's column; lanes past the last
+  // path repeat it and write nothing.
+  const uint32_t p0 = (blockIdx.x * 32u + lane) * PPL, col = cols == 16u ? lane >> 1u : lane;
+  auto planPath = [&](uint32_t p) { return sc.pathMap ? sc.pathMap[min(p, nP - 1)] : min(p, nP - 1); };
+
+  if (role > sc.nC) {
+    // ================================ producers ================================
+    constexpr uint32_t perPass = 32u / cols;  // dates of a producer warp's pass
+    const uint32_t mine = lane & (cols - 1u), sub = lane / cols;
+    const uint32_t po = planPath(cols == 16u ? blockIdx.x * 32u + 2u * mine : p0);
+    const uint32_t pathStream = sc.antithetic ? po >> 1u : po;
+    const uint32_t injectedStream = sc.nStreams > 0 ? min(pathStream, sc.nStreams - 1) : 0u;
+    const uint32_t stream = pcg(pcg(sc.seed) ^ pcg(pathStream + 0x9E3779B9u));
+    for (uint32_t b = 0; b <= blocks; ++b) {
+      if (b < blocks)
+        for (uint32_t d = (role - 1 - sc.nC) * perPass + sub; d < L.dates; d += numProducers * perPass) {
+          const uint32_t j = 1 + b * L.dates + d;
+          if (j < nT) drawDate<R, cols>(sc, L, stream, j, injectedStream, bridge, ring + (b & 1u) * bufLen + d * L.slots * cols + mine);
+        }
+      __syncthreads();
+    }
+    return;
+  }
+
+  // ================================ the states ================================
+  const uint32_t po = planPath(p0);
+  R sign[PPL];
+#pragma unroll
+  for (int i = 0; i < PPL; ++i) sign[i] = PPL == 2 ? (i == 0 ? R(1) : R(-1)) : sc.antithetic && (po & 1u) ? R(-1) : R(1);
+  const bool vec = PPL == 2 && nP % 2u == 0u;  // a lane's pair of paths in one store
+  auto put = [&](uint32_t field, uint32_t j, const R (&v)[PPL]) {
+    R* dst = cb.data + (static_cast<size_t>(field) * nT + j) * nP + p0;
+    if (vec) {
+      if (p0 < nP) stPaths<R, PPL>(dst, v);
+    } else {
+#pragma unroll
+      for (int i = 0; i < PPL; ++i)
+        if (p0 + i < nP) dst[i] = v[i];
+    }
+  };
+  if (role == 0) {
+    // The deflator's exponent -sum of the integrated short rate accumulates in double precision in both modes (the
+    // reference's kernel sums it in single precision, fused_kernels.cpp:250-253); D = exp(lnD) is then taken in R.
+    R x[PPL], D[PPL], S[4][PPL], lnS[4][PPL], xf[2][PPL];  // xf: stochastic foreign short-rate states of assets 0 and 1
+    double lnD[PPL];
+#pragma unroll
+    for (int i = 0; i < PPL; ++i) {
+      x[i] = R(0), D[i] = R(1), lnD[i] = 0.0, xf[0][i] = xf[1][i] = R(0);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) S[a][i] = sc.spots[a], lnS[a][i] = R(0);
+    }
+    auto write = [&](uint32_t j) {
+      put(0, j, x);
+      put(1, j, D);
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+        if (static_cast<uint32_t>(a) < sc.nA) put(cb.fS + a, j, S[a]);
+#pragma unroll
+      for (int f = 0; f < 2; ++f)
+        if (static_cast<uint32_t>(f) < sc.nF) put(cb.fXf + f, j, xf[f]);
+      if (cb.probes)
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+          if (static_cast<uint32_t>(a) < sc.nA) put(cb.fLnS + a, j, lnS[a]);
+    };
+    write(0);
+    for (uint32_t b = 0; b <= blocks; ++b) {
+      if (b > 0) {
+        const uint32_t j0 = 1 + (b - 1) * L.dates, j1 = min(j0 + L.dates, nT);
+        const R* buf = ring + ((b - 1) & 1u) * bufLen + col;
+#pragma unroll 1
+        for (uint32_t j = j0; j < j1; ++j, buf += L.slots * cols) {
+          const R* step = sc.steps + static_cast<size_t>(j) * sc.stepStride;
+          const R s0 = __ldg(step), s1 = __ldg(step + 1), s2 = __ldg(step + 2), s3 = __ldg(step + 3), s4 = __ldg(step + 4),
+                  s5 = __ldg(step + 5);
+          const R w0 = buf[0], zI = buf[sc.nCorr * cols];
+          R integratedRate[PPL], carry[4][PPL];
+#pragma unroll
+          for (int i = 0; i < PPL; ++i) {
+            const R w = sign[i] * w0, z = sign[i] * zI;
+            integratedRate[i] = fma(s3, z, fma(x[i], s5, s2 * w)) + s4;
+            x[i] = fma(x[i], s0, s1 * w);
+            lnD[i] -= static_cast<double>(integratedRate[i]);
+            D[i] = rexp(static_cast<R>(lnD[i]));
+          }
+          // Stochastic foreign rates: the exact Hull-White step of x_f (with its quanto drift) and of its integral, on
+          // driver 1 + nA + nC + f and the independent normal nCorr + 1 + f; the asset's carry is then the simulated
+          // integral of r_f instead of the deterministic one.
+#pragma unroll
+          for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int i = 0; i < PPL; ++i) carry[a][i] = __ldg(step + 8 + a);
+#pragma unroll
+          for (int f = 0; f < 2; ++f) {
+            if (static_cast<uint32_t>(f) < sc.nF) {
+              const R* fs = step + kStepStride + 8 * f;
+              const R wf0 = buf[(1 + sc.nA + sc.nC + f) * cols], zf0 = buf[(sc.nCorr + 1 + f) * cols];
+#pragma unroll
+              for (int i = 0; i < PPL; ++i) {
+                const R wf = sign[i] * wf0, zf = sign[i] * zf0;
+                carry[f][i] = fma(__ldg(fs + 3), zf, fma(xf[f][i], __ldg(fs + 5), __ldg(fs + 2) * wf)) + __ldg(fs + 4) + __ldg(fs + 7);
+                xf[f][i] = fma(xf[f][i], __ldg(fs), __ldg(fs + 1) * wf) + __ldg(fs + 6);
+              }
+            }
+          }
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            if (static_cast<uint32_t>(a) < sc.nA) {
+              const R drift = __ldg(step + 16 + a), vol = __ldg(step + 12 + a), wa = buf[(1 + a) * cols];
+#pragma unroll
+              for (int i = 0; i < PPL; ++i) {
+                lnS[a][i] = lnS[a][i] + fma(vol, sign[i] * wa, integratedRate[i] - carry[a][i] - drift);
+                S[a][i] = sc.spots[a] * rexp(lnS[a][i]);
+              }
+            }
+          }
+          write(j);
+        }
+      }
+      __syncthreads();
+    }
+    return;
+  }
+  const uint32_t c = role - 1;  // this warp's credit
+  const R kappa = sc.cir[4 * c], theta = sc.cir[4 * c + 1], xi = sc.cir[4 * c + 2];
+  R y[PPL], Y[PPL], Q[PPL];
+#pragma unroll
+  for (int i = 0; i < PPL; ++i) y[i] = sc.cir[4 * c + 3], Y[i] = R(0), Q[i] = R(1);
+  put(cb.fQ + c, 0, Q);
+  if (cb.probes) put(cb.fY + c, 0, y);
+  const uint32_t at = (sc.nCorr + 1 + sc.nF + c * nB) * cols, last = (L.need + c) * cols;
+  for (uint32_t b = 0; b <= blocks; ++b) {
+    if (b > 0) {
+      const uint32_t j0 = 1 + (b - 1) * L.dates, j1 = min(j0 + L.dates, nT);
+      const R* buf = ring + ((b - 1) & 1u) * bufLen + col;
+#pragma unroll 1
+      for (uint32_t j = j0; j < j1; ++j, buf += L.slots * cols) {
+        const R* step = sc.steps + static_cast<size_t>(j) * sc.stepStride;
+        const R h = __ldg(step + 6) / static_cast<R>(sc.substeps), shift = __ldg(step + 20 + c);
+        auto subStep = [&](R dW0) {
+#pragma unroll
+          for (int i = 0; i < PPL; ++i) {
+            const R dW = sign[i] * dW0, yp = fmax(y[i], R(0));
+            const R yn = fma(xi * rsqrt_(yp), dW, fma(kappa * (theta - yp), h, y[i]));
+            Y[i] = fma(R(0.5) * (yp + fmax(yn, R(0))), h, Y[i]);
+            y[i] = yn;
+          }
+        };
+#pragma unroll 4
+        for (uint32_t s = 0; s < nB; ++s) subStep(buf[at + s * cols]);
+        subStep(buf[last]);
+#pragma unroll
+        for (int i = 0; i < PPL; ++i) Q[i] = rexp(-Y[i] - shift);
+        put(cb.fQ + c, j, Q);
+        if (cb.probes) put(cb.fY + c, j, y);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The exponential of a lowered term: 2^(b x) with b = -B log2 e in single precision, e^(b x) with b = -B
+// in double (lowerTerms, capi.cu).
+__device__ __forceinline__ float termExp(float b, float x) { return ex2(b * x); }
+__device__ __forceinline__ double termExp(double b, double x) { return exp(b * x); }
+
+template <typename R> struct Vec4;
+template <> struct Vec4<float> { using T = float4; };
+template <> struct Vec4<double> { using T = double4; };
+__device__ __forceinline__ float4 ld4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ double4 ld4(const double* p) {
+  const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
+  return make_double4(a.x, a.y, b.x, b.y);
+}
+
+// Prefetches into L1 the 128-byte lines of one date's lowered terms, one line per thread of the CTA:
+// the next date's block arrives while the current date computes.
+__device__ __forceinline__ void prefetchL1(const void* p) {
+  asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(p)));
+}
+template <typename R>
+__device__ __forceinline__ void prefetchDate(uint32_t begin, uint32_t end, const R* table, uint32_t tid) {
+  const size_t b = static_cast<size_t>(begin) * 4 * sizeof(R), e = static_cast<size_t>(end) * 4 * sizeof(R);
+  const uint32_t lines = e > b ? static_cast<uint32_t>((e - 1) / 128 - b / 128 + 1) : 0u;
+  if (tid < lines) prefetchL1(reinterpret_cast<const char*>(table) + (b / 128 + tid) * 128);
 }
 
 template <typename R, int PPT>
@@ -1067,17 +1163,32 @@ cudaError_t launchNestedIm(const ImArgs<R>& M, cudaStream_t stream) {
 // ---------------------------------------------------------------------------------------------
 template <typename R>
 cudaError_t launchSimulate(const ScenarioArgs<R>& sc, const CubeArgs<R>& cb, cudaStream_t stream) {
-  const uint32_t blocks = (sc.nP + kSimThreads - 1) / kSimThreads;
-  const size_t normals = static_cast<size_t>(sc.nNormals) * kSimThreads * sizeof(R);
+  SimLayout L{};
+  // Adjacent paths share a stream with opposite signs (a re-run of chosen paths does not keep pairs together).  16
+  // streams per CTA while they run in one wave (four CTAs per SM: 18,944 paths; 94 us against 120 at 10,000 paths, but
+  // 217 against 178 at 33,333), 32 beyond.
+  const bool paired = sc.antithetic && !sc.pathMap, small = paired && sc.nP <= 148u * 4u * 32u;
+  const uint32_t cols = small ? 16 : 32;
+  L.need = sc.nCorr + 1 + sc.nF + sc.nC * (sc.substeps - 1);
+  L.slots = (L.need + sc.nC) | 1u;  // odd: the two dates of a 16-stream pass fall on different banks
+  // A pass of each producer warp per buffer, two with short dates, as far as 96 KB hold two buffers.
+  const uint32_t perPass = 32 / cols, round = (kSimWarps - 1 - sc.nC) * perPass;
+  const size_t date = static_cast<size_t>(L.slots) * cols * sizeof(R);
+  L.dates = L.slots <= 8 ? 2 * round : round;
+  L.dates = std::min(L.dates, std::max(static_cast<uint32_t>(96 * 1024 / (2 * date)), 1u));
+  size_t smem = 2 * L.dates * date;
   const size_t table = static_cast<size_t>(sc.nT) * (sc.substeps - 1) * 2 * sizeof(R);
-  const bool bridgeTable = sc.nC > 0 && sc.substeps > 1 && normals + table <= 64 * 1024;
-  const size_t smem = normals + (bridgeTable ? table : 0);
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(simulateKernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-  }
-  simulateKernel<R><<<blocks, kSimThreads, smem, stream>>>(sc, cb, bridgeTable);
-  return cudaGetLastError();
+  L.table = sc.nC > 0 && sc.substeps > 1 && table <= 32 * 1024;
+  if (L.table) smem += table;
+  auto go = [&](auto kernel, uint32_t paths) {
+    if (smem > 48 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+      if (e != cudaSuccess) return e;
+    }
+    kernel<<<(sc.nP + paths - 1) / paths, kSimThreads, smem, stream>>>(sc, cb, L);
+    return cudaGetLastError();
+  };
+  return small ? go(simulateKernel<R, 1, 16>, 32) : paired ? go(simulateKernel<R, 2, 32>, 64) : go(simulateKernel<R, 1, 32>, 32);
 }
 
 size_t revalueSmemBytes(size_t stateWordsMax, bool perTrade, bool f64, int ppt) {
