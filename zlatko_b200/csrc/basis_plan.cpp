@@ -25,11 +25,14 @@ uint32_t bitsOf(float v) {
   return u;
 }
 
-double fromHalf(uint16_t h) {
-  const double s = (h & 0x8000u) ? -1.0 : 1.0;
-  const int E = (h >> 10) & 31, M = h & 1023;
-  if (E == 0) return s * std::ldexp(static_cast<double>(M), -24);
-  return s * std::ldexp(static_cast<double>(1024 + M), E - 25);
+double fromHalf(uint16_t h) {  // by its bits (a call of ldexp per coefficient was half of a book's lowering)
+  const uint64_t sign = static_cast<uint64_t>(h & 0x8000u) << 48;
+  const uint64_t E = (h >> 10) & 31, M = h & 1023;
+  double v;
+  if (E == 0) return (sign ? -1.0 : 1.0) * static_cast<double>(M) * (1.0 / 16777216.0);
+  const uint64_t bits = sign | (E - 15 + 1023) << 52 | M << 42;
+  std::memcpy(&v, &bits, 8);
+  return v;
 }
 
 float bOf(float B) { return static_cast<float>(-static_cast<double>(B) * kLog2e); }
@@ -236,10 +239,18 @@ void buildDate(const std::vector<BasisPlanIn>& plans, const std::vector<Fix>& fi
   const size_t numKg = D.kgs.size();
   // per netting set of the date: the largest |C / mult| lands in [2^14, 2^15)
   std::vector<double> inv(kBasisRows, 1.0);
+  std::vector<double> largest(kBasisRows, 0.0);  // column by column: a column's coefficients are contiguous
+  for (size_t q = 0; q < colOfSlot.size(); ++q) {
+    if (colOfSlot[q] < 0) continue;
+    const double* cq = &coef[static_cast<size_t>(colOfSlot[q]) * kBasisRows];
+    const double m = 1.0 / D.kgs[q / 8].mult;  // a power of two
+    for (size_t n = 0; n < plans.size(); ++n) {
+      const double v = std::fabs(cq[n]) * m;
+      if (v > largest[n]) largest[n] = v;
+    }
+  }
   for (size_t n = 0; n < plans.size(); ++n) {
-    double mx = 0.0;
-    for (size_t q = 0; q < colOfSlot.size(); ++q)
-      if (colOfSlot[q] >= 0) mx = std::max(mx, std::fabs(coef[static_cast<size_t>(colOfSlot[q]) * kBasisRows + n]) / D.kgs[q / 8].mult);
+    const double mx = largest[n];
     if (mx > 0.0) {
       if (!std::isfinite(mx)) {
         D.why = "a non-finite coefficient";
@@ -271,6 +282,7 @@ void buildDate(const std::vector<BasisPlanIn>& plans, const std::vector<Fix>& fi
         const double m = 1.0 / D.kgs[c0 + g].mult;
         for (size_t n = 0; n < plans.size(); ++n) {
           const double v = coef[static_cast<size_t>(kc) * kBasisRows + n] * m * inv[n];
+          if (v == 0.0) continue;  // most netting sets hold a few of the date's columns
           const uint16_t h = f2h(static_cast<float>(v));
           const uint16_t l = f2h(static_cast<float>(v - fromHalf(h)));
           const size_t off = g * 1024 + (n & 7) * 8 + (n >> 3) * 64 + e;

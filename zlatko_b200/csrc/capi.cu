@@ -114,6 +114,7 @@ struct zk_context {
   size_t stageInBytes = 0;
   unsigned char* stageOut = nullptr;
   size_t stageOutBytes = 0;
+  uint32_t* hErr = nullptr;  // page-locked copy of *dErr
   // A second stream for the large-state revalue launch of a split batch, beside the small-state launch on the
   // context's stream (fork and join events order the two); created by the first eager execute that splits.
   cudaStream_t side = nullptr;
@@ -613,6 +614,7 @@ uint32_t numTilesOf(uint32_t nP, int ppt) {
 template <typename R>
 struct Batch {
   zk_context* ctx = nullptr;
+  bool times = false;  // record the phase events (zk_batch_timings, the autotuner)
   std::vector<Plan<R>> plans;
   struct Launch {
     ScenarioArgs<R> sc;
@@ -703,8 +705,9 @@ HostPool* hostPool(zk_context* ctx, size_t plans) {
   return ctx->pool.get();
 }
 
+// first: plan 0 when it is parsed already.
 template <typename R>
-void parseAll(const std::vector<View<R>>& views, std::vector<Plan<R>>& plans, HostPool* pool) {
+void parseAll(const std::vector<View<R>>& views, std::vector<Plan<R>>& plans, HostPool* pool, Plan<R>* first = nullptr) {
   const size_t n = views.size();
   plans.assign(n, Plan<R>());
   const size_t workers = n >= 8 && pool ? std::min<size_t>(pool->workers(), n / 4) : 1;
@@ -712,7 +715,8 @@ void parseAll(const std::vector<View<R>>& views, std::vector<Plan<R>>& plans, Ho
   auto work = [&](size_t w) {
     for (size_t i = w; i < n; i += workers) {
       try {
-        plans[i] = parse(views[i], i);
+        if (i == 0 && first) plans[0] = std::move(*first);
+        else plans[i] = parse(views[i], i);
       } catch (...) {
         errs[i] = std::current_exception();
       }
@@ -836,17 +840,18 @@ struct BuildOpts {
   bool exact = false;
   const std::vector<std::vector<uint32_t>>* maps = nullptr;
   const Presim* presim = nullptr;  // the first plan's scenario already simulated (single precision, counter normals)
+  bool ctxArena = false;  // the batch goes into the context's arena
 };
 
 // parsed: the plans already validated and lowered (their views' tables stay the caller's), else parsed from views.
 template <typename R>
 std::unique_ptr<Batch<R>> build(zk_context* ctx, std::vector<View<R>> views, bool sink, const double* normals, size_t streams,
-                                const BuildOpts& opts = BuildOpts(), std::vector<Plan<R>>* parsed = nullptr) {
+                                const BuildOpts& opts = BuildOpts(), std::vector<Plan<R>>* parsed = nullptr, Plan<R>* first = nullptr) {
   auto B = std::make_unique<Batch<R>>();
   B->ctx = ctx;
   B->sink = sink;
   if (parsed) B->plans = std::move(*parsed);
-  else parseAll(views, B->plans, hostPool(ctx, views.size()));
+  else parseAll(views, B->plans, hostPool(ctx, views.size()), first);
   const size_t nPlans = B->plans.size();
   if (opts.maps) {
     for (size_t i = 0; i < nPlans; ++i) {
@@ -973,7 +978,16 @@ std::unique_ptr<Batch<R>> build(zk_context* ctx, std::vector<View<R>> views, boo
   bool anyIm = false;
   for (const auto& P : B->plans) allRows += rowsBytes(P), anyIm = anyIm || P.im;
   uint64_t budget = ctx ? ctx->rowBudget : 0;
-  if (ctx && budget == 0) {
+  // Asking the driver for the free memory takes 0.1 ms, and milliseconds when other processes keep it busy: only a batch
+  // that may run in waves asks, and not when the context's arena already holds it whole (no memory is taken then).
+  size_t whole = off + allRows;  // the arena of the batch in one wave
+  auto sized = [](size_t bytes) { return alignUp(std::max<size_t>(bytes, 16)); };
+  for (const auto& P : B->plans) {
+    whole += sized(static_cast<size_t>(P.nT) * P.nS * sizeof(R)) + sized(static_cast<size_t>(std::max<uint32_t>(P.v.num_outputs, 1)) * sizeof(R));
+    if (opts.exact && !P.guard.empty()) whole += sized(static_cast<size_t>((P.nP + 31) / 32) * 4);
+  }
+  const bool mayWave = !sink && !anyIm && !normals && !(opts.ctxArena && ctx && whole <= ctx->arenaBytes);
+  if (ctx && budget == 0 && mayWave) {
     size_t freeB = 0, totalB = 0;
     if (cudaMemGetInfo(&freeB, &totalB) == cudaSuccess && allRows > freeB / 10 * 7) budget = freeB / 10 * 6;
     else cudaGetLastError();
@@ -1218,7 +1232,8 @@ void growStage(unsigned char*& stage, size_t& bytes, size_t need) {
 
 // The arena: the context's (useCtxArena), a spare block of the context (spare: short-lived batches), or its own.
 template <typename R>
-void upload(Batch<R>& B, zk_context* ctx, bool useCtxArena, const double* normals, size_t streams, bool spare = false) {
+void upload(Batch<R>& B, zk_context* ctx, bool useCtxArena, const double* normals, size_t streams, bool spare = false,
+            bool idle = false) {
   if (!useCtxArena && spare) {
     size_t bytes = 0;
     B.base = takeBlock(ctx, B.totalBytes, bytes);
@@ -1241,9 +1256,10 @@ void upload(Batch<R>& B, zk_context* ctx, bool useCtxArena, const double* normal
   }
   if (useCtxArena) {
     // Calls on the context arena synchronise before they return, so the context's page-locked staging is free;
-    // the waits below cover a previous call that failed with its copy, or a forked launch, in flight.
-    ZK_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (ctx->side) ZK_CUDA(cudaStreamSynchronize(ctx->side));
+    // the waits below cover a previous call that failed with its copy, or a forked launch, in flight (idle: the
+    // caller has waited already).
+    if (!idle) ZK_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (!idle && ctx->side) ZK_CUDA(cudaStreamSynchronize(ctx->side));
     growStage(ctx->stageIn, ctx->stageInBytes, B.inputBytes);
     fillImage(B, normals, streams, ctx->stageIn);
     ZK_CUDA(cudaMemcpyAsync(B.base, ctx->stageIn, B.inputBytes, cudaMemcpyHostToDevice, ctx->stream));
@@ -1324,11 +1340,14 @@ template <typename R>
 void execute(Batch<R>& B, bool capturing = false) {
   zk_context* ctx = B.ctx;
   cudaStream_t s = ctx->stream;
-  if (!B.ev[0])
+  if (B.times && !B.ev[0])
     for (auto& e : B.ev) ZK_CUDA(cudaEventCreate(&e));
+  auto stamp = [&](int k) {
+    if (B.times) ZK_CUDA(recordEvent(B.ev[k], s, capturing));
+  };
   ZK_CUDA(cudaMemsetAsync(ctx->dErr, 0, 4, s));
   if (B.flagsBytes) ZK_CUDA(cudaMemsetAsync(B.base + B.flagsOff, 0, B.flagsBytes, s));
-  ZK_CUDA(recordEvent(B.ev[0], s, capturing));
+  stamp(0);
   const uintptr_t base = reinterpret_cast<uintptr_t>(B.base);
   // A re-run of chosen paths: every plan is a launch of a few paths; they run side by side on worker streams,
   // each its simulation then its revaluation, joined before the reduce.
@@ -1357,14 +1376,14 @@ void execute(Batch<R>& B, bool capturing = false) {
       ZK_CUDA(cudaEventRecord(ctx->workerJoin[q], ctx->workers[q]));
       ZK_CUDA(cudaStreamWaitEvent(s, ctx->workerJoin[q], 0));
     }
-    ZK_CUDA(recordEvent(B.ev[1], s, capturing));
+    stamp(1);
   } else {
     for (auto& L : B.launches) {
       if (L.presim) continue;  // simulated ahead of the host work
       injectPoint(ctx);
       ZK_CUDA(launchSimulate<R>(L.sc, L.cb, s));
     }
-    ZK_CUDA(recordEvent(B.ev[1], s, capturing));
+    stamp(1);
   }
   for (auto& L : B.launches) {
     if (fan) break;  // revalued on the worker streams above
@@ -1393,21 +1412,21 @@ void execute(Batch<R>& B, bool capturing = false) {
     injectPoint(ctx);
     ZK_CUDA(launchNestedIm<R>(M, s));
   }
-  ZK_CUDA(recordEvent(B.ev[2], s, capturing));
+  stamp(2);
   if (B.waved) {
-    ZK_CUDA(recordEvent(B.ev[3], s, capturing));
+    stamp(3);
   } else if (!B.sink) {
     injectPoint(ctx);
     ZK_CUDA(launchReduce<R>(reinterpret_cast<const ReduceJob<R>*>(base + B.reduceOff), static_cast<uint32_t>(B.plans.size()), B.maxReduceN,
                             B.ppt, s));
-    ZK_CUDA(recordEvent(B.ev[3], s, capturing));
+    stamp(3);
     injectPoint(ctx);
     ZK_CUDA(launchRowStats<R>(reinterpret_cast<const RowJob<R>*>(base + B.rowOff), B.numRowJobs, ctx->dErr, s, ctx->rowRounds));
   } else {
-    ZK_CUDA(recordEvent(B.ev[3], s, capturing));
+    stamp(3);
   }
-  ZK_CUDA(recordEvent(B.ev[4], s, capturing));
-  B.timed = true;
+  stamp(4);
+  B.timed = B.times;
 }
 
 // The status of a kernel's error word (DeviceError), the same for every entry point.
@@ -1423,30 +1442,33 @@ void throwDeviceError(uint32_t err) {
 template <typename R>
 void finish(Batch<R>& B) {
   zk_context* ctx = B.ctx;
-  uint32_t err = 0;
-  ZK_CUDA(cudaMemcpyAsync(&err, ctx->dErr, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  ZK_CUDA(cudaMemcpyAsync(ctx->hErr, ctx->dErr, 4, cudaMemcpyDeviceToHost, ctx->stream));
   ZK_CUDA(cudaStreamSynchronize(ctx->stream));
+  const uint32_t err = *ctx->hErr;
   if (B.timed) {
     for (int k = 0; k < 4; ++k) ZK_CUDA(cudaEventElapsedTime(&B.ms[k], B.ev[k], B.ev[k + 1]));
   }
   throwDeviceError(err);
 }
 
+// The outputs on their way into the context's page-locked staging.
+template <typename R>
+void startRead(Batch<R>& B) {
+  growStage(B.ctx->stageOut, B.ctx->stageOutBytes, B.outBytes);
+  ZK_CUDA(cudaMemcpyAsync(B.ctx->stageOut, B.base + B.outBegin, B.outBytes, cudaMemcpyDeviceToHost, B.ctx->stream));
+}
+
+// started: startRead has run since the last kernel that writes outputs.
 template <typename R, typename Out>
-void readOutputs(Batch<R>& B, Out* outs) {
-  zk_context* ctx = B.ctx;
-  growStage(ctx->stageOut, ctx->stageOutBytes, B.outBytes);
-  unsigned char* host = ctx->stageOut;
-  ZK_CUDA(cudaMemcpyAsync(host, B.base + B.outBegin, B.outBytes, cudaMemcpyDeviceToHost, ctx->stream));
+void readOutputs(Batch<R>& B, Out* outs, bool started = false) {
+  if (!started) startRead(B);
   finish(B);
+  const unsigned char* host = B.ctx->stageOut;
   for (size_t i = 0; i < B.plans.size(); ++i) {
     const auto& P = B.plans[i];
     const auto& D = B.dev[i];
-    const R* sums = reinterpret_cast<const R*>(host + (D.sums - B.outBegin));
-    const R* vals = reinterpret_cast<const R*>(host + (D.values - B.outBegin));
-    const size_t nS = static_cast<size_t>(P.nT) * P.nS, nV = std::max<uint32_t>(P.v.num_outputs, 1);
-    for (size_t k = 0; k < nS; ++k) outs[i].sums[k] = sums[k];
-    for (size_t k = 0; k < nV; ++k) outs[i].values[k] = vals[k];
+    std::memcpy(outs[i].sums, host + (D.sums - B.outBegin), static_cast<size_t>(P.nT) * P.nS * sizeof(R));
+    std::memcpy(outs[i].values, host + (D.values - B.outBegin), static_cast<size_t>(std::max<uint32_t>(P.v.num_outputs, 1)) * sizeof(R));
   }
 }
 
@@ -1640,6 +1662,7 @@ zk_status runInjected(zk_context* ctx, const ViewT* plan, const double* normals,
     if (!plan || !out) throw fail(ZK_ERR_INVALID_ARGUMENT, "null argument");
     BuildOpts bo;
     bo.exact = sizeof(R) == 4 && !normals && ctx->exactGuard > 0.0;
+    bo.ctxArena = true;
     auto B = build<R>(ctx, {viewOf(*plan)}, false, normals, streams, bo);
     checkOutputs(*B, out, sizeof(R) == 8);
     upload(*B, ctx, true, normals, streams);
@@ -1837,7 +1860,7 @@ namespace {
 bool captureExecute(zk_batch* b) {
   Batch<float>& B = *b->b;
   const cudaStream_t s = B.ctx->stream;
-  if (!B.ev[0])
+  if (B.times && !B.ev[0])
     for (auto& e : B.ev) ZK_CUDA(cudaEventCreate(&e));
   if (b->graph) cudaGraphExecDestroy(b->graph), b->graph = nullptr;
   if (cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
@@ -1881,6 +1904,7 @@ zk_status zk_context_create(int device, zk_context** out) {
     ZK_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     ctx->ownStream = true;
     ZK_CUDA(cudaMalloc(&ctx->dErr, 16));
+    ZK_CUDA(cudaMallocHost(reinterpret_cast<void**>(&ctx->hErr), 16));
   } catch (const Failure& f) {
     delete ctx;
     return f.status;
@@ -1897,6 +1921,7 @@ void zk_context_destroy(zk_context* ctx) {
   if (ctx->stageIn) cudaFreeHost(ctx->stageIn);
   if (ctx->stageOut) cudaFreeHost(ctx->stageOut);
   if (ctx->dErr) cudaFree(ctx->dErr);
+  if (ctx->hErr) cudaFreeHost(ctx->hErr);
   if (ctx->side) {
     cudaStreamSynchronize(ctx->side);
     cudaStreamDestroy(ctx->side);
@@ -1992,9 +2017,8 @@ namespace {
 // cube is being written while the host validates and lowers the plans; build() hands it to the launch that holds
 // plan 0 when that launch needs the same fields (else the launch simulates again).  The step table goes up first;
 // the buffers are reused by later calls, which synchronise before they return.
-Presim presimulate(zk_context* ctx, const zk_plan_view& v0) {
+Presim presimulate(zk_context* ctx, const Plan<float>& P0) {
   Presim pre;
-  const Plan<float> P0 = parse(viewOf(v0), 0);
   ScenarioArgs<float> sc;
   CubeArgs<float> cb;
   const uint32_t fields = scenarioOf(P0, P0.probes, 0, sc, cb);
@@ -2037,19 +2061,22 @@ zk_status zk_run_plans(zk_context* ctx, const zk_plan_view* plans, size_t n, zk_
     auto ms = [](Clock::time_point a, Clock::time_point b) { return std::chrono::duration<double, std::milli>(b - a).count(); };
     const auto t0 = Clock::now();
     ZK_CUDA(cudaStreamSynchronize(ctx->stream));  // a failed earlier call may have left work on the buffers
-    const Presim pre = presimulate(ctx, plans[0]);
-    bo.presim = &pre;
-    auto B = build<float>(ctx, views, false, nullptr, 0, bo);
+    if (ctx->side) ZK_CUDA(cudaStreamSynchronize(ctx->side));
+    Plan<float> first = parse(views[0], 0);
+    const Presim pre = presimulate(ctx, first);
+    bo.presim = &pre, bo.ctxArena = true;
+    auto B = build<float>(ctx, views, false, nullptr, 0, bo, nullptr, &first);
     checkOutputs(*B, outs, false);
     const auto t1 = Clock::now();
-    upload(*B, ctx, true, nullptr, 0);
+    upload(*B, ctx, true, nullptr, 0, false, true);
     const auto t2 = Clock::now();
     execute(*B);
+    if (!bo.exact) startRead(*B);  // the check patches the outputs first
     ZK_CUDA(cudaStreamSynchronize(ctx->stream));
     const auto t3 = Clock::now();
     const auto patches = exactCheck(*B);
     const auto t4 = Clock::now();
-    readOutputs(*B, outs);
+    readOutputs(*B, outs, !bo.exact);
     applyPatches(patches, outs);
     const auto t5 = Clock::now();
     ctx->callMs[0] = ms(t0, t1), ctx->callMs[1] = ms(t1, t2), ctx->callMs[2] = ms(t2, t3), ctx->callMs[3] = ms(t3, t4);
@@ -2144,30 +2171,47 @@ zk_status zk_gemm_bf16(zk_context* ctx, const uint16_t* A, const uint16_t* B, ui
 struct zk_surrogate {
   zk_context* ctx = nullptr;
   zk::SurrogateState S;
+  // Device memory for a call's rows (inputs, then targets or predictions), kept for the next call up to kKeepRows.
+  unsigned char* rows = nullptr;
+  size_t rowsBytes = 0;
 };
 
 namespace {
 zk_context* ctxOf(zk_surrogate* s) {
   if (!s || !s->ctx) throw fail(ZK_ERR_INVALID_ARGUMENT, "null surrogate");
   requireCtx(s->ctx);
+  s->S.stream = s->ctx->stream;  // the copies and the kernels of a call are ordered on the context's stream
   return s->ctx;
 }
-// A device copy of n host values; the caller frees it.
-template <typename T>
-T* toDevice(const T* h, size_t n, cudaStream_t st) {
-  void* d = nullptr;
-  ZK_CUDA(cudaMalloc(&d, std::max<size_t>(n, 1) * sizeof(T)));
-  const cudaError_t e = cudaMemcpyAsync(d, h, n * sizeof(T), cudaMemcpyHostToDevice, st);
-  if (e != cudaSuccess) {
-    cudaFree(d);
-    ZK_CUDA(e);
+// The surrogate's device rows for n inputs and n targets or predictions.  cudaMalloc and cudaFree on every call took
+// 0.7 ms of a 2 ms prediction, so up to kKeepRows bytes stay with the surrogate (rowsDone gives back more).
+constexpr size_t kKeepRows = 256u << 20;
+struct Rows {
+  float *x, *y;
+};
+Rows deviceRows(zk_surrogate* s, size_t n) {
+  const size_t xb = alignUp(std::max<size_t>(n, 1) * zk::kIn * 4), need = xb + alignUp(std::max<size_t>(n, 1) * 4);
+  if (s->rowsBytes < need) {
+    if (s->rows) cudaFree(s->rows);
+    s->rows = nullptr, s->rowsBytes = 0;
+    ZK_CUDA(cudaMalloc(reinterpret_cast<void**>(&s->rows), need));
+    s->rowsBytes = need;
   }
-  return static_cast<T*>(d);
+  return {reinterpret_cast<float*>(s->rows), reinterpret_cast<float*>(s->rows + xb)};
+}
+// After the call's work (waited for here if it failed half-way).
+void rowsDone(zk_surrogate* s, bool failed) {
+  if (!s || !s->ctx) return;
+  if (failed) cudaStreamSynchronize(s->ctx->stream);
+  if (s->rowsBytes > kKeepRows) {
+    cudaFree(s->rows);
+    s->rows = nullptr, s->rowsBytes = 0;
+  }
 }
 void checkErrWord(zk_context* ctx) {
-  uint32_t devErr = 0;
-  ZK_CUDA(cudaMemcpyAsync(&devErr, ctx->dErr, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  ZK_CUDA(cudaMemcpyAsync(ctx->hErr, ctx->dErr, 4, cudaMemcpyDeviceToHost, ctx->stream));
   ZK_CUDA(cudaStreamSynchronize(ctx->stream));
+  const uint32_t devErr = *ctx->hErr;
   if (devErr) throw fail(ZK_ERR_DEVICE_TIMEOUT, "a tensor-core wait gave up (error %u)", devErr);
 }
 void scaleFromHost(zk_surrogate* s, const float* x, const float* y, size_t n) {
@@ -2202,78 +2246,75 @@ void zk_surrogate_destroy(zk_surrogate* s) {
   if (!s) return;
   if (s->ctx) cudaSetDevice(s->ctx->device);
   zk::surrogateFree(s->S);
+  if (s->rows) cudaFree(s->rows);
   delete s;
 }
 
 zk_status zk_surrogate_train(zk_surrogate* s, const float* x, const float* y, size_t n, uint32_t epochs, uint32_t batch, float lr,
                              float weight_decay, float* loss_per_epoch) {
   zk_context* ctx = s ? s->ctx : nullptr;
-  float *dx = nullptr, *dy = nullptr;
   try {
     ctx = ctxOf(s);
     if (!x || !y || n == 0 || batch == 0) throw fail(ZK_ERR_INVALID_ARGUMENT, "empty training set or batch");
     if (!s->S.scaled) scaleFromHost(s, x, y, n);
-    dx = toDevice(x, n * zk::kIn, ctx->stream);
-    dy = toDevice(y, n, ctx->stream);
+    const Rows d = deviceRows(s, n);
+    ZK_CUDA(cudaMemcpyAsync(d.x, x, n * zk::kIn * 4, cudaMemcpyHostToDevice, ctx->stream));
+    ZK_CUDA(cudaMemcpyAsync(d.y, y, n * 4, cudaMemcpyHostToDevice, ctx->stream));
     ZK_CUDA(cudaMemsetAsync(ctx->dErr, 0, 4, ctx->stream));
     for (uint32_t e = 0; e < epochs; ++e) {
       double loss = 0.0;
-      ZK_CUDA(zk::surrogateEpoch(s->S, dx, dy, n, batch, lr, weight_decay, true, &loss));
+      ZK_CUDA(zk::surrogateEpoch(s->S, d.x, d.y, n, batch, lr, weight_decay, true, &loss));
       if (loss_per_epoch) loss_per_epoch[e] = static_cast<float>(loss);
     }
     checkErrWord(ctx);
-    cudaFree(dx), cudaFree(dy);
+    rowsDone(s, false);
     return ZK_OK;
   } catch (const Failure& f) {
-    if (dx) cudaFree(dx);
-    if (dy) cudaFree(dy);
+    rowsDone(s, true);
     return record(ctx, f);
   }
 }
 
 zk_status zk_surrogate_predict(zk_surrogate* s, const float* x, size_t n, float* y) {
   zk_context* ctx = s ? s->ctx : nullptr;
-  float *dx = nullptr, *dy = nullptr;
   try {
     ctx = ctxOf(s);
     if (!x || !y) throw fail(ZK_ERR_INVALID_ARGUMENT, "null argument");
     if (n == 0) return ZK_OK;
-    dx = toDevice(x, n * zk::kIn, ctx->stream);
-    ZK_CUDA(cudaMalloc(&dy, n * 4));
+    const Rows d = deviceRows(s, n);
+    ZK_CUDA(cudaMemcpyAsync(d.x, x, n * zk::kIn * 4, cudaMemcpyHostToDevice, ctx->stream));
     ZK_CUDA(cudaMemsetAsync(ctx->dErr, 0, 4, ctx->stream));
-    ZK_CUDA(zk::surrogatePredict(s->S, dx, n, dy));
-    ZK_CUDA(cudaMemcpyAsync(y, dy, n * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    ZK_CUDA(zk::surrogatePredict(s->S, d.x, n, d.y));
+    ZK_CUDA(cudaMemcpyAsync(y, d.y, n * 4, cudaMemcpyDeviceToHost, ctx->stream));
     checkErrWord(ctx);
-    cudaFree(dx), cudaFree(dy);
+    rowsDone(s, false);
     return ZK_OK;
   } catch (const Failure& f) {
-    if (dx) cudaFree(dx);
-    if (dy) cudaFree(dy);
+    rowsDone(s, true);
     return record(ctx, f);
   }
 }
 
 zk_status zk_surrogate_gradients(zk_surrogate* s, const float* x, const float* y, size_t n, float* loss, float* grads) {
   zk_context* ctx = s ? s->ctx : nullptr;
-  float *dx = nullptr, *dy = nullptr;
   try {
     ctx = ctxOf(s);
     if (!x || !y || !grads || n == 0) throw fail(ZK_ERR_INVALID_ARGUMENT, "null argument or empty set");
     if (n > (1u << 20)) throw fail(ZK_ERR_INVALID_ARGUMENT, "gradients of at most 2^20 rows (one batch)");
     if (!s->S.scaled) scaleFromHost(s, x, y, n);
-    dx = toDevice(x, n * zk::kIn, ctx->stream);
-    dy = toDevice(y, n, ctx->stream);
+    const Rows d = deviceRows(s, n);
+    ZK_CUDA(cudaMemcpyAsync(d.x, x, n * zk::kIn * 4, cudaMemcpyHostToDevice, ctx->stream));
+    ZK_CUDA(cudaMemcpyAsync(d.y, y, n * 4, cudaMemcpyHostToDevice, ctx->stream));
     ZK_CUDA(cudaMemsetAsync(ctx->dErr, 0, 4, ctx->stream));
     double l = 0.0;
-    ZK_CUDA(zk::surrogateEpoch(s->S, dx, dy, n, static_cast<uint32_t>(n), 0.0f, 0.0f, false, &l));
+    ZK_CUDA(zk::surrogateEpoch(s->S, d.x, d.y, n, static_cast<uint32_t>(n), 0.0f, 0.0f, false, &l));
     ZK_CUDA(cudaMemcpyAsync(grads, s->S.grad, zk::SurrogateState::kParams * 4, cudaMemcpyDeviceToHost, ctx->stream));
     checkErrWord(ctx);
     if (loss) *loss = static_cast<float>(l);
-    cudaFree(dx), cudaFree(dy);
+    rowsDone(s, false);
     return ZK_OK;
   } catch (const Failure& f) {
-    if (dx) cudaFree(dx);
-    if (dy) cudaFree(dy);
+    rowsDone(s, true);
     return record(ctx, f);
   }
 }
@@ -2456,6 +2497,7 @@ zk_status zk_batch_create(zk_context* ctx, const zk_plan_view* plans, size_t n, 
     for (size_t i = 0; i < n; ++i) views.push_back(viewOf(plans[i]));
     auto b = std::make_unique<zk_batch>();
     b->b = build<float>(ctx, views, false, nullptr, 0);
+    b->b->times = true;
     upload(*b->b, ctx, false, nullptr, 0);
     ZK_CUDA(cudaStreamSynchronize(ctx->stream));
     *out = b.release();
