@@ -457,7 +457,8 @@ Plan<R> parse(const View<R>& v, size_t index) {
 //   fixing (kSetFixing):             (A, b, 1 / c, slot)          fix[slot] = (A E(b x) - 1) / c
 // with b = -B log2 e and E = 2^ in single precision, b = -B and E = exp in double.  Fixings stay last, so a
 // running coupon still reads the previous fixing on its fixing date (the reference's merge order).  In
-// per-trade mode every term keeps its trade group in the generic run.  The date descriptor also carries
+// per-trade mode every term keeps its trade group in the generic run.  Slots, assets and a generic record's first two
+// words (code, slot) are integers by their bits (bitsOfUint).  The date descriptor also carries
 // the margin-call index and the reporting slot: the kernel reads one 32-byte record per date.
 template <typename R>
 void lowerTerms(Plan<R>& p) {
@@ -471,6 +472,7 @@ void lowerTerms(Plan<R>& p) {
     p.table.push_back(static_cast<R>(a)), p.table.push_back(static_cast<R>(b));
     p.table.push_back(static_cast<R>(c)), p.table.push_back(static_cast<R>(d));
   };
+  auto index = [&](size_t back, R v) { p.table[p.table.size() - back] = bitsOfUint<R>(static_cast<uint32_t>(v)); };
   for (uint32_t j = 0; j < p.nT; ++j) {
     uint32_t* d = &p.dates[static_cast<size_t>(j) * 8];
     const R* first = p.v.terms + static_cast<size_t>(I[j]) * kTermStride;
@@ -483,7 +485,8 @@ void lowerTerms(Plan<R>& p) {
     for (const R* r = first; r < last; r += kTermStride)
       if (isFloat(r)) {
         const double A = r[3];
-        push4(static_cast<double>(r[2]) * A, static_cast<double>(r[5]) * A, -static_cast<double>(r[4]) * bScale, r[1]);
+        push4(static_cast<double>(r[2]) * A, static_cast<double>(r[5]) * A, -static_cast<double>(r[4]) * bScale, 0.0);
+        index(1, r[1]);
       }
     d[1] = units();
     double pending[2] = {0, 0};
@@ -497,10 +500,10 @@ void lowerTerms(Plan<R>& p) {
     if (half) push4(pending[0], pending[1], 0.0, 0.0);  // the odd bond with a zero partner
     d[2] = units();
     for (const R* r = first; r < last; r += kTermStride)
-      if (isAsset(r)) push4(r[2], r[3], r[1], 0.0);
+      if (isAsset(r)) push4(r[2], r[3], 0.0, 0.0), index(2, r[1]);
     d[3] = units();
     // Generic records in plan order.  A run of two or more Bermudan bonds (kBermBond) of one Bermudan and trade group
-    // becomes a block: a header record (the run's code with extra 0, -count, the largest exercise index) and two
+    // becomes a block: a header record (the run's code with extra 0, kBlockMark + count, the largest exercise index) and two
     // bonds (c, A, B, exercise index) per record; the kernel skips the block in a warp none of whose paths has
     // exercised that Bermudan by then, and otherwise adds each bond as the record would.
     auto bermBond = [&](const R* r) { return (static_cast<uint32_t>(r[0]) & 15u) == static_cast<uint32_t>(kBermBond); };
@@ -516,12 +519,18 @@ void lowerTerms(Plan<R>& p) {
       const size_t n = static_cast<size_t>(e - r) / kTermStride;
       if (n < 2) {
         p.table.insert(p.table.end(), r, r + kTermStride);
+        index(kTermStride, r[0]);
+        // a foreign term's second word is its bond's coefficient, a continuation's the position, an extension's a value
+        const uint32_t kind = low & 15u;
+        if (kind == static_cast<uint32_t>(kBermBond)) index(kTermStride - 1, R(0));
+        else if (kind != kForeignForward && kind != kForeignOption && kind != kBermContinue && kind != kBermExt) index(kTermStride - 1, r[1]);
         r += kTermStride;
         continue;
       }
       double maxEx = 0.0;
       for (const R* q = r; q < e; q += kTermStride) maxEx = std::max(maxEx, static_cast<double>(static_cast<uint32_t>(q[0]) >> 12u));
-      push4(static_cast<double>(low), -static_cast<double>(n), maxEx, 0.0);
+      push4(0.0, 0.0, maxEx, 0.0);
+      p.table[p.table.size() - 4] = bitsOfUint<R>(low), p.table[p.table.size() - 3] = bitsOfUint<R>(kBlockMark + static_cast<uint32_t>(n));
       push4(0.0, 0.0, 0.0, 0.0);
       for (size_t q = 0; q < n; ++q) {
         const R* b = r + q * kTermStride;
@@ -533,7 +542,7 @@ void lowerTerms(Plan<R>& p) {
     }
     d[4] = units();
     for (const R* r = first; r < last; r += kTermStride)
-      if (isFixing(r)) push4(r[3], -static_cast<double>(r[4]) * bScale, 1.0 / static_cast<double>(r[2]), r[1]);
+      if (isFixing(r)) push4(r[3], -static_cast<double>(r[4]) * bScale, 1.0 / static_cast<double>(r[2]), 0.0), index(1, r[1]);
     d[5] = units();
     d[6] = I[p.offCall + j];
     d[7] = I[p.offRep + j];
@@ -646,6 +655,23 @@ struct Batch {
       BasisImage img;
       size_t dates = 0, kgs = 0, options = 0, fixings = 0, chunks = 0, blob = 0, scale = 0;
     };
+    // The netting sets after the basis groups run on the kernels split over the dates (planSplit) instead of
+    // revalueKernel: the host tables and their places in the arena.
+    struct Split {
+      bool on = false;
+      int ppt = 1;
+      uint32_t settlePaths = 32;
+      uint32_t slab = 0;                     // paths per slab
+      std::vector<ValueItem> items;          // those of AMC, probe or nested-margin plans first
+      uint32_t fullItems = 0;                // how many those are
+      std::vector<uint2> pre;
+      std::vector<uint8_t> exFirst;
+      std::vector<DecideJob> decides;
+      std::vector<R> table;
+      uint32_t slotsMax[2] = {0, 0}, bermsMax = 0;  // [0] the first fullItems, [1] the lean ones
+      size_t oItems = 0, oPre = 0, oFirst = 0, oDecides = 0, oTable = 0, oVals = 0, oIndex = 0;
+      size_t valsBytes = 0, indexBytes = 0;
+    } split;
     size_t basisCount = 0, groupArgs = 0;  // groupArgs: index of the first group's BasisArgs in the batch's array
     uint32_t descBytes = 0, fixSlots = 0;  // the basis kernel's shared memory: the largest over the groups
     std::vector<Group> groups;
@@ -806,6 +832,138 @@ void formGroups(Batch<R>& B, typename Batch<R>::Launch& L, uint32_t mode, HostPo
   }
 }
 
+// Sets up the split over the dates of a launch's netting sets [basisCount, n) (Launch::split), or leaves it off where
+// a plan needs revalueKernel: per-trade views, or Bermudans whose exercise indices do not follow their dates.
+template <typename R>
+void planSplit(Batch<R>& B, typename Batch<R>::Launch& L) {
+  const size_t nb = L.basisCount, n = L.planIdx.size() - nb;
+  if (n == 0 || n > 16384) return;
+  const uint32_t nP = L.sc.nP, nT = L.sc.nT;
+  auto& S = L.split;
+  auto full = [&](const Plan<R>& P) { return P.amcOrProbe || P.im; };
+  for (size_t k = 0; k < n; ++k)
+    if (B.plans[L.planIdx[nb + k]].nTr > 0) return;
+  // Bermudans: the exercises' dates, and their records date by date as decideKernel reads them.
+  std::vector<std::vector<std::vector<uint32_t>>> exDates(n);
+  for (size_t k = 0; k < n; ++k) {
+    const auto& P = B.plans[L.planIdx[nb + k]];
+    if (P.nBerm == 0) continue;
+    const uint32_t* I = P.v.indices;
+    exDates[k].resize(P.nBerm);
+    std::vector<std::vector<R>> prog(P.nBerm);
+    for (uint32_t j = 0; j < nT; ++j) {
+      std::vector<std::vector<const R*>> flows(P.manyBerm ? 1 : P.nBerm);
+      std::vector<const R*> swap;
+      for (uint32_t t = I[j]; t < I[j + 1]; ++t) {
+        const R* r = P.v.terms + static_cast<size_t>(t) * kTermStride;
+        const uint32_t code = static_cast<uint32_t>(r[0]), kind = code & 15u;
+        if (kind == kBermAnnuity || kind == kBermCoterm) swap.push_back(r);
+        if (kind == kBermContinue) swap.clear();
+        if (kind != kBermExercise && kind != kBermDecide) continue;
+        const uint32_t b = bermudanOf(code, P.manyBerm);
+        auto& mine = flows[P.manyBerm ? 0 : b];
+        if (kind == kBermExercise) {
+          mine.push_back(r);
+          continue;
+        }
+        const uint32_t e = code >> 12u;
+        if (e != exDates[k][b].size() || (e > 0 && exDates[k][b].back() >= j)) return;  // not the next exercise
+        exDates[k][b].push_back(j);
+        auto& out = prog[b];
+        auto put = [&](const R* q) {
+          out.insert(out.end(), q, q + kTermStride);
+          out[out.size() - kTermStride] = bitsOfUint<R>(static_cast<uint32_t>(q[0]));
+        };
+        const R mark[kTermStride] = {bitsOfUint<R>(kBond), bitsOfUint<R>(j), R(0), R(0), R(0), R(0), R(0), R(0)};
+        out.insert(out.end(), mark, mark + kTermStride);
+        for (const R* q : mine) put(q);
+        for (const R* q : swap) put(q);
+        put(r);
+        for (uint32_t u = t + 1; u < I[j + 1] && (static_cast<uint32_t>(r[(u - t) * kTermStride]) & 15u) == kBermExt; ++u) put(r + (u - t) * kTermStride);
+        swap.clear();
+        if (P.manyBerm) mine.clear();
+      }
+    }
+    for (uint32_t b = 0; b < P.nBerm; ++b) {
+      const uint32_t at = static_cast<uint32_t>(S.table.size() / 4);
+      S.table.insert(S.table.end(), prog[b].begin(), prog[b].end());
+      S.decides.push_back({static_cast<uint32_t>(k), b, at, static_cast<uint32_t>(S.table.size() / 4)});
+    }
+    S.indexBytes += alignUp(static_cast<size_t>(P.nBerm) * nP);
+    S.bermsMax = std::max(S.bermsMax, P.nBerm);
+  }
+  if (S.decides.size() > 65535) return;
+  // revalueKernel fills the GPU with a CTA per 128 to 512 paths of every netting set, and writes no values: without AMC
+  // terms it is the faster one from about a million paths x netting sets on (12 netting sets: 1,490 us against 1,026 here
+  // at 33,333 paths, 3.1 ms both at 100,000, 12.4 ms against 15.4 at 500,000).  With AMC terms it never is (24 + 24 netting
+  // sets, 800 trades, 65,536 paths: 66 ms against 28).
+  bool anyFull = false;
+  for (size_t k = 0; k < n; ++k) anyFull = anyFull || full(B.plans[L.planIdx[nb + k]]);
+  if (!anyFull && static_cast<uint64_t>(nP) * n > (1u << 20)) return;
+  // One slab's values take at most 1 GB (slabs of 64 MB, which would stay in the L2, cost 15% in their tails).
+  const size_t perPath = n * nT * sizeof(R), most = size_t(1) << 30;
+  S.slab = static_cast<uint32_t>(std::min<size_t>((nP + 255u) / 256u * 256u, std::max<size_t>(most / perPath / 256 * 256, 256)));
+  S.valsBytes = perPath * S.slab;
+  // Runs of dates of about equal work, enough of them for several CTAs per SM and slab: an item's cost counts its term
+  // records (a generic record as three) and a date's own work.
+  auto cost = [](const uint32_t* d) { return (d[2] - d[0]) + (d[3] - d[2]) + 3 * (d[4] - d[3]) / 2 + (d[5] - d[4]) + 6; };
+  uint64_t total = 0;
+  for (size_t k = 0; k < n; ++k) {
+    const auto& P = B.plans[L.planIdx[nb + k]];
+    for (uint32_t j = 0; j < nT; ++j) total += cost(&P.dates[8 * static_cast<size_t>(j)]);
+  }
+  S.ppt = static_cast<uint64_t>(S.slab) * total < (1ull << 25) ? 1 : 2;
+  // 32 paths per CTA of settleKernel while they run in one wave (11.5 us against 20 at 2,000 paths), 64 beyond (384 against
+  // 412 us at 12 x 33,333).
+  S.settlePaths = static_cast<uint64_t>((nP + 31) / 32) * n <= 148 * 6 ? 32 : 64;
+  const uint64_t tiles = (S.slab + kTile * S.ppt - 1) / (kTile * S.ppt), want = std::min<uint64_t>(std::max<uint64_t>((148ull * 64) / tiles, 1), 32768);
+  const uint64_t each = std::max<uint64_t>(total / want, 1);
+  std::vector<std::pair<uint64_t, ValueItem>> order;
+  for (size_t k = 0; k < n; ++k) {
+    const auto& P = B.plans[L.planIdx[nb + k]];
+    const int lean = full(P) ? 0 : 1;
+    S.slotsMax[lean] = std::max(S.slotsMax[lean], P.nSlots);
+    std::vector<uint2> set(P.nSlots, make_uint2(kNoRow, 0u));  // per slot: its last fixing's record and date
+    for (uint32_t j0 = 0; j0 < nT;) {
+      uint64_t c = 0;
+      uint32_t j1 = j0;
+      while (j1 < nT && (c < each || j1 < j0 + 2)) c += cost(&P.dates[8 * static_cast<size_t>(j1++)]);
+      ValueItem I{};
+      I.ns = static_cast<uint32_t>(k), I.j0 = j0, I.j1 = j1, I.preBegin = static_cast<uint32_t>(S.pre.size());
+      std::vector<uint2> now = set;
+      std::vector<uint8_t> read(P.nSlots, P.im ? 1 : 0), fresh(P.nSlots, 0);  // the margin's start reads every fixing
+      for (uint32_t j = j0; j < j1; ++j) {
+        const uint32_t* d = &P.dates[8 * static_cast<size_t>(j)];
+        for (uint32_t u = d[0]; u < d[1]; ++u) {
+          const uint32_t q = asUint(P.table[4 * static_cast<size_t>(u) + 3]);
+          if (!fresh[q]) read[q] = 1;
+        }
+        for (uint32_t t = P.v.indices[j]; t < P.v.indices[j + 1]; ++t) {
+          const R* r = P.v.terms + static_cast<size_t>(t) * kTermStride;
+          if ((static_cast<uint32_t>(r[0]) & 15u) == kBermFloat && !fresh[static_cast<uint32_t>(r[1])]) read[static_cast<uint32_t>(r[1])] = 1;
+        }
+        for (uint32_t u = d[4]; u < d[5]; ++u) {
+          const uint32_t q = asUint(P.table[4 * static_cast<size_t>(u) + 3]);
+          fresh[q] = 1, now[q] = make_uint2(u, j);
+        }
+      }
+      for (uint32_t q = 0; q < P.nSlots; ++q)
+        if (read[q] && set[q].x != kNoRow) S.pre.push_back(set[q]);
+      I.preEnd = static_cast<uint32_t>(S.pre.size());
+      I.exAt = static_cast<uint32_t>(S.exFirst.size());
+      for (uint32_t b = 0; b < P.nBerm; ++b)
+        S.exFirst.push_back(static_cast<uint8_t>(std::lower_bound(exDates[k][b].begin(), exDates[k][b].end(), j0) - exDates[k][b].begin()));
+      order.push_back({c + (lean ? 0 : total), I});
+      S.fullItems += lean ? 0u : 1u;
+      set = std::move(now), j0 = j1;
+    }
+  }
+  // AMC plans' runs first (one launch), then the lean ones; the heaviest first in each.
+  std::stable_sort(order.begin(), order.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+  for (const auto& o : order) S.items.push_back(o.second);
+  S.on = S.items.size() <= 65535;
+}
+
 // The simulation arguments of a launch whose first plan is P0 (probes: the launch's plans read ln S and the CIR
 // states); returns the cube's number of fields.
 template <typename R>
@@ -919,6 +1077,16 @@ std::unique_ptr<Batch<R>> build(zk_context* ctx, std::vector<View<R>> views, boo
     const size_t need = P0.anti ? (P0.nP + 1) / 2 : P0.nP;
     if (streams < need) throw fail(ZK_ERR_INVALID_ARGUMENT, "injected normals: %zu streams for %zu needed", streams, need);
   }
+  // Rows and warp partials of a plan in the arena.
+  auto rowsBytes = [&](const Plan<R>& P) {
+    const uint32_t warps = (P.nP + 31) / 32;  // the most revalue warps any tile shape uses: one partial each
+    return alignUp(static_cast<size_t>(std::max<uint32_t>(P.v.rows_total, 1)) * P.nP * sizeof(R)) +
+           alignUp(static_cast<size_t>(warps) * P.nT * P.nS * sizeof(R));
+  };
+  // Whether the batch may run split over the dates: with a context (the no-alloc entry has a fixed array), not the AMC
+  // state pass, not the re-run of chosen paths (its plans run side by side on worker streams).
+  if (ctx && !sink && !opts.maps)
+    for (auto& L : B->launches) planSplit(*B, L);
   // ---- arena layout: inputs first (one upload), then device-only scratch, outputs last ----
   size_t off = 0;
   auto take = [&](size_t bytes) { const size_t o = off; off = alignUp(off + std::max<size_t>(bytes, 16)); return o; };
@@ -952,6 +1120,12 @@ std::unique_ptr<Batch<R>> build(zk_context* ctx, std::vector<View<R>> views, boo
     }
   }
   B->basisArgsOff = take(B->numGroups * sizeof(BasisArgs));
+  for (auto& L : B->launches) {
+    auto& S = L.split;
+    if (!S.on) continue;
+    S.oItems = take(S.items.size() * sizeof(ValueItem)), S.oPre = take(S.pre.size() * sizeof(uint2)), S.oFirst = take(S.exFirst.size());
+    S.oDecides = take(S.decides.size() * sizeof(DecideJob)), S.oTable = take(S.table.size() * sizeof(R));
+  }
   B->reduceOff = take(nPlans * sizeof(ReduceJob<R>));
   for (const auto& P : B->plans) B->numRowJobs += static_cast<uint32_t>(P.nReq);
   B->rowOff = take(B->numRowJobs * sizeof(RowJob<R>));
@@ -969,18 +1143,16 @@ std::unique_ptr<Batch<R>> build(zk_context* ctx, std::vector<View<R>> views, boo
     if (!L.presim) L.cubeOff = take(static_cast<size_t>(L.numFields) * L.sc.nT * L.sc.nP * sizeof(R));
   // Rows and warp partials: one region per plan, or -- when they exceed the row budget -- waves of netting sets
   // (in each launch's order) that reuse one region, sized by the largest wave.
-  auto rowsBytes = [&](const Plan<R>& P) {
-    const uint32_t warps = (P.nP + 31) / 32;  // the most revalue warps any tile shape uses: one partial each
-    return alignUp(static_cast<size_t>(std::max<uint32_t>(P.v.rows_total, 1)) * P.nP * sizeof(R)) +
-           alignUp(static_cast<size_t>(warps) * P.nT * P.nS * sizeof(R));
-  };
   size_t allRows = 0;
   bool anyIm = false;
   for (const auto& P : B->plans) allRows += rowsBytes(P), anyIm = anyIm || P.im;
+  size_t splitBytes = 0;
+  for (const auto& L : B->launches)
+    if (L.split.on) splitBytes += alignUp(L.split.valsBytes) + alignUp(std::max<size_t>(L.split.indexBytes, 16));
   uint64_t budget = ctx ? ctx->rowBudget : 0;
   // Asking the driver for the free memory takes 0.1 ms, and milliseconds when other processes keep it busy: only a batch
   // that may run in waves asks, and not when the context's arena already holds it whole (no memory is taken then).
-  size_t whole = off + allRows;  // the arena of the batch in one wave
+  size_t whole = off + allRows + splitBytes;  // the arena of the batch in one wave
   auto sized = [](size_t bytes) { return alignUp(std::max<size_t>(bytes, 16)); };
   for (const auto& P : B->plans) {
     whole += sized(static_cast<size_t>(P.nT) * P.nS * sizeof(R)) + sized(static_cast<size_t>(std::max<uint32_t>(P.v.num_outputs, 1)) * sizeof(R));
@@ -989,8 +1161,13 @@ std::unique_ptr<Batch<R>> build(zk_context* ctx, std::vector<View<R>> views, boo
   const bool mayWave = !sink && !anyIm && !normals && !(opts.ctxArena && ctx && whole <= ctx->arenaBytes);
   if (ctx && budget == 0 && mayWave) {
     size_t freeB = 0, totalB = 0;
-    if (cudaMemGetInfo(&freeB, &totalB) == cudaSuccess && allRows > freeB / 10 * 7) budget = freeB / 10 * 6;
-    else cudaGetLastError();
+    if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess) {
+      cudaGetLastError();
+    } else {
+      if (allRows > freeB / 10 * 7) budget = freeB / 10 * 6;
+      if (whole > freeB / 10 * 9)  // no room for the split's values
+        for (auto& L : B->launches) L.split.on = false;
+    }
   }
   B->waved = budget > 0 && allRows > budget && !sink && !anyIm && !normals;
   auto placeRows = [&](size_t i, auto&& takeFn) {
@@ -999,6 +1176,10 @@ std::unique_ptr<Batch<R>> build(zk_context* ctx, std::vector<View<R>> views, boo
     B->dev[i].expo = takeFn(static_cast<size_t>(std::max<uint32_t>(P.v.rows_total, 1)) * P.nP * sizeof(R));
     B->dev[i].partials = takeFn(static_cast<size_t>(warps) * P.nT * P.nS * sizeof(R));
   };
+  if (B->waved)
+    for (auto& L : B->launches) L.split.on = false;
+  for (auto& L : B->launches)
+    if (L.split.on) L.split.oVals = take(L.split.valsBytes), L.split.oIndex = take(L.split.indexBytes);
   if (!B->waved) {
     for (size_t i = 0; i < nPlans; ++i) {
       const auto& P = B->plans[i];
@@ -1129,6 +1310,7 @@ void fillImage(Batch<R>& B, const double* normals, size_t streams, unsigned char
       A.usesAssets = P.usesAssets ? 1u : 0u;
       A.usesForeign = P.usesForeign ? 1u : 0u;
       A.stepStride = P.stepStride;
+      A.moreRows = P.rowDV != kNoRow || P.rowE != kNoRow || P.rowV != kNoRow || P.rowC != kNoRow || P.rowGross != kNoRow ? 1u : 0u;
       A.manyBerm = P.manyBerm ? 1u : 0u;
       if (!P.guard.empty()) {
         A.flags = static_cast<uint32_t*>(dptr(D.flags));
@@ -1153,6 +1335,22 @@ void fillImage(Batch<R>& B, const double* normals, size_t streams, unsigned char
         A.sinkEx = static_cast<R*>(dptr(B.sinkOff[2]));
         A.sinkRowOfBermudan = static_cast<const uint32_t*>(dptr(B.bermRowOff));
       }
+    }
+    if (L.split.on) {
+      const auto& S = L.split;
+      size_t at = S.oIndex;
+      for (size_t k = L.basisCount; k < L.planIdx.size(); ++k) {
+        const auto& P = B.plans[L.planIdx[k]];
+        args[k].vals = static_cast<R*>(dptr(S.oVals)) + (k - L.basisCount) * P.nT * static_cast<size_t>(S.slab);
+        if (P.nBerm == 0) continue;
+        args[k].exIndex = static_cast<signed char*>(dptr(at));
+        at += alignUp(static_cast<size_t>(P.nBerm) * P.nP);
+      }
+      std::memcpy(img + S.oItems, S.items.data(), S.items.size() * sizeof(ValueItem));
+      if (!S.pre.empty()) std::memcpy(img + S.oPre, S.pre.data(), S.pre.size() * sizeof(uint2));
+      if (!S.exFirst.empty()) std::memcpy(img + S.oFirst, S.exFirst.data(), S.exFirst.size());
+      if (!S.decides.empty()) std::memcpy(img + S.oDecides, S.decides.data(), S.decides.size() * sizeof(DecideJob));
+      if (!S.table.empty()) std::memcpy(img + S.oTable, S.table.data(), S.table.size() * sizeof(R));
     }
     std::memcpy(img + L.nsOff, args.data(), args.size() * sizeof(NsArgs<R>));
     if constexpr (sizeof(R) == 4) {
@@ -1189,6 +1387,9 @@ void fillImage(Batch<R>& B, const double* normals, size_t streams, unsigned char
     L.cb.data = L.presim ? L.presim : static_cast<R*>(dptr(L.cubeOff));
     (void)P0;
   }
+  std::vector<uint32_t> onSplit(B.plans.size(), 0);  // 32-path units of a partial
+  for (const auto& L : B.launches)
+    for (size_t k = L.basisCount; L.split.on && k < L.planIdx.size(); ++k) onSplit[L.planIdx[k]] = L.split.settlePaths / 32;
   std::vector<ReduceJob<R>> red(B.plans.size());
   std::vector<RowJob<R>> rows;
   rows.reserve(B.numRowJobs);
@@ -1197,9 +1398,9 @@ void fillImage(Batch<R>& B, const double* normals, size_t streams, unsigned char
     const size_t i = B.jobOrder[o];  // plan order, or wave by wave when the batch runs in waves
     const auto& P = B.plans[i];
     const auto& D = B.dev[i];
-    // pad: 2 for a basis plan (a partial per 64 paths), 0 for the batch's tile shape
+    // pad: 2 for a basis plan (a partial per 64 paths), 1 or 2 split over the dates (32 or 64 paths), 0 for the batch's tile shape
     red[o] = {static_cast<const R*>(dptr(D.partials)), static_cast<R*>(dptr(D.sums)), P.nT * P.nS, numTilesOf(P.nP, 1), P.nP,
-              B.onBasis[i] ? 2u : 0u};
+              B.onBasis[i] ? 2u : onSplit[i]};
     B.maxReduceN = std::max(B.maxReduceN, P.nT * P.nS);
     for (size_t q = 0; q < P.nReq; ++q)
       rows.push_back({static_cast<const R*>(dptr(D.expo)), static_cast<const R*>(dptr(D.req + q * kRequestStride * sizeof(R))),
@@ -1305,6 +1506,19 @@ void launchRevalues(const Batch<R>& B, const typename Batch<R>::Launch& L, uintp
   }
   if (count == 0) return;
   const auto* ns = reinterpret_cast<const NsArgs<R>*>(base + L.nsOff) + first;
+  if (L.split.on) {  // never in waves: [first, first + count) are the launch's netting sets after its basis groups
+    const auto& S = L.split;
+    SplitArgs<R> a{};
+    a.items = reinterpret_cast<const ValueItem*>(base + S.oItems), a.pre = reinterpret_cast<const uint2*>(base + S.oPre);
+    a.exFirst = reinterpret_cast<const uint8_t*>(base + S.oFirst), a.decides = reinterpret_cast<const DecideJob*>(base + S.oDecides);
+    a.decideTable = reinterpret_cast<const R*>(base + S.oTable);
+    a.numItems = static_cast<uint32_t>(S.items.size()), a.numFull = S.fullItems, a.numDecides = static_cast<uint32_t>(S.decides.size());
+    a.slabPaths = S.slab, a.slotsMax[0] = S.slotsMax[0], a.slotsMax[1] = S.slotsMax[1], a.bermsMax = S.bermsMax, a.ppt = S.ppt;
+    a.settlePaths = S.settlePaths;
+    injectPoint(B.ctx);
+    ZK_CUDA(launchSplit<R>(L.cb, ns, static_cast<uint32_t>(count), a, s));
+    return;
+  }
   const uint32_t n = static_cast<uint32_t>(count), tiles = numTilesOf(L.sc.nP, B.ppt);
   const size_t splitAt = std::min(count, L.splitAt > first ? L.splitAt - first : 0);
   const bool split = L.lean && !L.perTrade && !B.sink && sizeof(R) == 4 && B.ppt > 1 && splitAt < n;
@@ -1387,7 +1601,7 @@ void execute(Batch<R>& B, bool capturing = false) {
   }
   for (auto& L : B.launches) {
     if (fan) break;  // revalued on the worker streams above
-    const bool split = L.lean && !L.perTrade && !B.sink && sizeof(R) == 4 && B.ppt > 1 && L.splitAt < L.planIdx.size();
+    const bool split = !L.split.on && L.lean && !L.perTrade && !B.sink && sizeof(R) == 4 && B.ppt > 1 && L.splitAt < L.planIdx.size();
     if (split && L.splitAt > L.basisCount && !ctx->side && !capturing) {
       ZK_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
       ZK_CUDA(cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming));
@@ -2513,9 +2727,9 @@ zk_status zk_batch_execute(zk_batch* b) {
     ZK_CUDA(cudaSetDevice(b->b->ctx->device));
     if (!b->tuned) {
       // first execute: time the tile shapes on this batch, keep the fastest (they shape the term-by-term launches
-      // only: a batch entirely on the basis kernel keeps the default)
+      // of revalueKernel only: a batch entirely on the other kernels keeps the default)
       bool termByTerm = false;
-      for (const auto& L : b->b->launches) termByTerm = termByTerm || L.basisCount < L.planIdx.size();
+      for (const auto& L : b->b->launches) termByTerm = termByTerm || (L.basisCount < L.planIdx.size() && !L.split.on);
       if (termByTerm) autotune(*b->b);
       b->tuned = true;
     }
@@ -2598,6 +2812,11 @@ zk_status zk_batch_info_get(const zk_batch* b, zk_batch_info* info) {
       ++k, count -= last - first, first = last;
     }
     if (count == 0) return k;
+    if (L.split.on) {
+      const uint64_t slabs = (L.sc.nP + L.split.slab - 1) / L.split.slab;
+      const bool both = L.split.fullItems > 0 && L.split.fullItems < L.split.items.size();
+      return k + (L.split.decides.empty() ? 0 : 1) + slabs * (both ? 3 : 2);
+    }
     const size_t at = std::min(count, L.splitAt > first ? L.splitAt - first : 0);
     const bool split = L.lean && !L.perTrade && !B.sink && B.ppt > 1 && at < count;
     return k + (split && at > 0 ? 2 : 1);

@@ -97,7 +97,7 @@ __device__ __forceinline__ void loadTerm(const double* t, double (&r)[8]) {
 // the next record an extension (kBermExt); then its two extension records into e1, e2.
 template <typename R>
 __device__ __forceinline__ bool twoRegressors(const R* table, uint32_t u, uint32_t end, R (&e1)[8], R (&e2)[8]) {
-  if (u + 2 >= end || (static_cast<uint32_t>(table[4 * (u + 2)]) & 15u) != kBermExt) return false;
+  if (u + 2 >= end || (asUint(table[4 * (u + 2)]) & 15u) != kBermExt) return false;
   loadTerm(table + 4 * (u + 2), e1);
   loadTerm(table + 4 * (u + 4), e2);
   return true;
@@ -436,6 +436,265 @@ __device__ __forceinline__ R pick4(const R (&a)[4][PPT], uint32_t k, int i) {
   return k == 0 ? a[0][i] : k == 1 ? a[1][i] : k == 2 ? a[2][i] : a[3][i];
 }
 
+// A product never fused into an addition and an addition never fused with a product: what two kernels compute alike rounds
+// alike, however the compiler arranges each.
+__device__ __forceinline__ float mulRn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mulRn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float addRn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double addRn(double a, double b) { return __dadd_rn(a, b); }
+
+// The netting set's value on date j of a thread's PPT paths (value), from the date's lowered runs [d0, d1), and the
+// fixings and exercise states the date sets.  state: the fixings [slot][PPT][kTile]; the exercise index of Bermudan b
+// (-1: not exercised) in bytes exS[b][PPT][kTile] when exBytes, else in registers ex.  kGiven: the decisions are those
+// of decideKernel (A.exIndex), not taken here.
+template <typename R, int PPT, bool kPerTrade, bool kSink, bool kLean, bool kGiven>
+__device__ __forceinline__ void revalueDate(const NsArgs<R>& A, const CubeArgs<R>& cb, const R* const (&cubeP)[PPT], const uint4 d0,
+                                            const uint4 d1, const uint32_t j, const uint32_t tid, const uint32_t (&pth)[PPT],
+                                            const bool (&act)[PPT], const R (&x)[PPT], const R (&D)[PPT], const R (&S)[4][PPT],
+                                            const R (&xf)[2][PPT], const R guardJ, R* state, R* vtBuf, signed char* exS,
+                                            const bool exBytes, R (&ex)[4][PPT], R (&value)[PPT]) {
+  const R* __restrict__ table = A.table;
+  R* __restrict__ expo = A.expo;
+  const uint32_t nP = cb.nP;
+  const size_t fieldStride = static_cast<size_t>(cb.nT) * nP;
+  const bool manyBerm = !kLean && exBytes;
+  const uint32_t nTr = kPerTrade ? min(A.nTr, static_cast<uint32_t>(kMaxTradeGroups)) : 0u;
+  auto fix = [&](uint32_t slot, int i) -> R& { return state[(slot * PPT + i) * kTile + tid]; };
+  auto vt = [&](uint32_t g, int i) -> R& { return vtBuf[(g * PPT + i) * kTile + tid]; };
+  auto cube = [&](uint32_t field, uint32_t jj, int i) { return cubeP[i][field * fieldStride + static_cast<size_t>(jj) * nP]; };
+  auto xfOf = [&](uint32_t a, int i) { return kGiven ? (a == 0 ? xf[0][i] : xf[1][i]) : cube(cb.fXf + a, j, i); };
+  auto exOf = [&](uint32_t b, int i) -> R {
+    return manyBerm ? static_cast<R>(exS[(b * PPT + i) * kTile + tid]) : pick4<R, PPT>(ex, b, i);
+  };
+  R ev[4][PPT];
+  R annS[PPT], fltS[PPT];  // the co-terminal swap of the next two-regressor record: annuity, float leg
+#pragma unroll
+  for (int i = 0; i < PPT; ++i) {
+    value[i] = R(0), annS[i] = R(0), fltS[i] = R(0);
+#pragma unroll
+    for (int b = 0; b < 4; ++b) ev[b][i] = R(0);
+  }
+  using R4 = typename Vec4<R>::T;
+  for (uint32_t u = d0.x; u < d0.y; ++u) {  // running floating coupons
+    const R4 r = ld4(table + 4 * u);
+    const uint32_t slot = asUint(r.w);
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) value[i] = fma(fma(r.x, fix(slot, i), r.y), termExp(r.z, x[i]), value[i]);
+  }
+#pragma unroll 2
+  for (uint32_t u = d0.y; u < d0.z; ++u) {  // bonds, two per record
+    const R4 r = ld4(table + 4 * u);
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) value[i] += r.x * termExp(r.y, x[i]) + r.z * termExp(r.w, x[i]);
+  }
+  for (uint32_t u = d0.z; u < d0.w; ++u) {  // asset forwards: (c, A, asset)
+    const R4 r = ld4(table + 4 * u);
+    const uint32_t a = asUint(r.z) & 3u;
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) value[i] = fma(r.x * pick4<R, PPT>(S, a, i), r.y, value[i]);
+  }
+  if (kPerTrade && A.nTr > 0)
+    for (uint32_t g = 0; g < kMaxTradeGroups; ++g)
+#pragma unroll
+      for (int i = 0; i < PPT; ++i) vt(g, i) = R(0);
+  for (uint32_t u = d0.w; u < d1.x; u += 2) {  // generic terms: the reference's records
+    R rec[8];
+    loadTerm(table + 4 * u, rec);
+    const uint32_t code = asUint(rec[0]), slot = asUint(rec[1]);
+    const uint32_t kind = code & 15u, bm = bermudanOf(code, A.manyBerm != 0), extra = code >> 12u;
+    const uint32_t grp = min((code >> 4u) & 15u, 15u);
+    if (!kLean && kind == kBermBond && slot >= kBlockMark) {
+      // A block of nb bonds of Bermudan bm (the lowering's run of its kBermBond records): each counts on a path
+      // that exercised at or before the bond's exercise index; a warp with no such path skips the block.
+      const uint32_t nb = slot - kBlockMark;
+      R exi[PPT];
+      bool live = false;
+#pragma unroll
+      for (int i = 0; i < PPT; ++i) exi[i] = exOf(bm, i), live = live || (exi[i] >= R(0) && exi[i] <= rec[2]);
+      if (__any_sync(0xFFFFFFFFu, live))
+        for (uint32_t q = 0; q < nb; ++q) {
+          const R4 b = ld4(table + 4 * (u + 2 + q));
+          const R nBq = -b.z;
+#pragma unroll
+          for (int i = 0; i < PPT; ++i) {
+            R term = R(0);
+            if (exi[i] >= R(0) && exi[i] <= b.w) term = b.x * (b.y * fastExp(nBq * x[i]));
+            if (kPerTrade && A.nTr > 0) vt(grp, i) += term;
+            else value[i] = addRn(value[i], term);
+          }
+        }
+      u += 2 * ((nb + 1) / 2);
+      continue;
+    }
+    const R c = rec[2], nB = -rec[4];
+    R term[PPT];
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) term[i] = R(0);
+    switch (kind) {
+      case kBond:
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) term[i] = c * (rec[3] * fastExp(nB * x[i]));
+        break;
+      case kFixedFloat:
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) term[i] = (c * fix(slot, i) + rec[5]) * (rec[3] * fastExp(nB * x[i]));
+        break;
+      case kAsset:
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) term[i] = c * pick4<R, PPT>(S, slot & 3u, i) * rec[3];
+        break;
+      case kSetFixing:
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) fix(slot, i) = (rec[3] * fastExp(nB * x[i]) - R(1)) / c;
+        break;
+      case kOption: {
+        const R p3 = rec[7];
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) {
+          const R b0 = rec[3] * fastExp(nB * x[i]);
+          term[i] = c * black(pick4<R, PPT>(S, slot & 3u, i) * rec[5] / b0, rec[6], fabs(p3), b0, p3 > R(0));
+        }
+        break;
+      }
+      case kForeignForward: {  // c S P_f(t, T | x_f), P_f = A_f e^{-B_f x_f}: the foreign bond of the asset's currency
+        const uint32_t a = min(extra, 1u);
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) term[i] = c * pick4<R, PPT>(S, a, i) * (rec[3] * fastExp(-rec[1] * xfOf(a, i)));
+        break;
+      }
+      case kForeignOption: {  // Black on S P_f(t, T | x_f) / P(t, T | x)
+        const uint32_t a = min(extra, 1u);
+        const R p3 = rec[7];
+#pragma unroll
+        for (int i = 0; i < PPT; ++i) {
+          const R b0 = rec[3] * fastExp(nB * x[i]);
+          const R q = rec[5] * fastExp(-rec[1] * xfOf(a, i));
+          term[i] = c * black(pick4<R, PPT>(S, a, i) * q / b0, rec[6], fabs(p3), b0, p3 > R(0));
+        }
+        break;
+      }
+      default:
+        if constexpr (!kLean) switch (kind) {  // the AMC and probe terms (absent from lean launches)
+        case kBermExercise:
+          if constexpr (kGiven) break;
+#pragma unroll
+          for (int i = 0; i < PPT; ++i) {
+            const R v = c * (rec[3] * fastExp(nB * x[i]));
+            if (manyBerm || bm == 0) ev[0][i] += v;  // with many Bermudans, one running value: its policy follows
+            else if (bm == 1) ev[1][i] += v;
+            else if (bm == 2) ev[2][i] += v;
+            else ev[3][i] += v;
+          }
+          break;
+        case kBermAnnuity:
+#pragma unroll
+          for (int i = 0; i < PPT; ++i) annS[i] += c * (rec[3] * fastExp(nB * x[i]));
+          break;
+        case kBermCoterm:
+#pragma unroll
+          for (int i = 0; i < PPT; ++i) fltS[i] += c * (rec[3] * fastExp(nB * x[i]));
+          break;
+        case kBermExt:
+          break;  // read with its policy or continuation record
+        case kBermDecide: {
+          if constexpr (kGiven) {
+#pragma unroll
+            for (int i = 0; i < PPT; ++i) {
+              annS[i] = R(0), fltS[i] = R(0);
+              if (act[i] && A.exIndex[static_cast<size_t>(bm) * nP + pth[i]] == static_cast<int>(extra))
+                exS[(bm * PPT + i) * kTile + tid] = static_cast<signed char>(extra);
+            }
+            break;
+          }
+          R e1[8], e2[8];
+          const bool twoD = twoRegressors(table, u, d1.x, e1, e2);
+#pragma unroll
+          for (int i = 0; i < PPT; ++i) {
+            const R e = manyBerm ? ev[0][i] : pick4<R, PPT>(ev, bm, i);
+            if (manyBerm) ev[0][i] = R(0);
+            const R cont = twoD ? amcPoly2(rec, e1, e2, x[i], swapRate(fltS[i], annS[i])) : amcPoly(rec, x[i]);
+            annS[i] = R(0), fltS[i] = R(0);
+            if (kSink) {
+              if (act[i]) A.sinkEx[static_cast<size_t>(A.sinkRowOfBermudan[bm] + extra) * nP + pth[i]] = e;
+            } else if (exOf(bm, i) < R(0)) {
+              // the exact-decision check: the rule's margins are e (against 0) and e - cont
+              if (act[i] && (fabs(e) <= guardJ || fabs(e - cont) <= guardJ)) flagPath(A.flags, pth[i]);
+              if (e > R(0) && e > cont) {
+                const R v = static_cast<R>(extra);
+                if (manyBerm) exS[(bm * PPT + i) * kTile + tid] = static_cast<signed char>(extra);
+                else if (bm == 0) ex[0][i] = v;
+                else if (bm == 1) ex[1][i] = v;
+                else if (bm == 2) ex[2][i] = v;
+                else ex[3][i] = v;
+              }
+            }
+          }
+          break;
+        }
+        case kBermContinue: {
+          R e1[8], e2[8];
+          const bool twoD = twoRegressors(table, u, d1.x, e1, e2);
+#pragma unroll
+          for (int i = 0; i < PPT; ++i) {
+            const R cont = twoD ? amcPoly2(rec, e1, e2, x[i], swapRate(fltS[i], annS[i])) : amcPoly(rec, x[i]);
+            annS[i] = R(0), fltS[i] = R(0);
+            if (exOf(bm, i) < R(0)) term[i] = rec[1] * fmax(cont, R(0));
+          }
+          break;
+        }
+        case kBermBond:
+#pragma unroll
+          for (int i = 0; i < PPT; ++i) {
+            const R e = exOf(bm, i);
+            if (e >= R(0) && e <= static_cast<R>(extra)) term[i] = c * (rec[3] * fastExp(nB * x[i]));
+          }
+          break;
+        case kProbe: {
+          const uint32_t what = slot & 15u, ix = min(slot >> 4u, 3u), ic = min(ix, 1u);
+#pragma unroll
+          for (int i = 0; i < PPT; ++i) {
+            R q;
+            switch (what) {
+              case 0: q = x[i]; break;
+              case 1: q = D[i]; break;
+              case 2: q = pick4<R, PPT>(S, ix, i); break;
+              case 3: q = ix < cb.nA ? cube(cb.fLnS + ix, j, i) : R(0); break;
+              case 4: q = ic < cb.nC ? cube(cb.fY + ic, j, i) : R(0); break;
+              case 5: q = ic < cb.nC ? cube(cb.fQ + ic, j, i) : R(1); break;
+              case 6: q = D[i] * pick4<R, PPT>(S, ix, i); break;
+              default: q = D[i] * (rec[3] * fastExp(nB * x[i]));
+            }
+            if (!kSink && act[i]) expo[static_cast<size_t>(static_cast<uint32_t>(rec[5])) * nP + pth[i]] = q + c;
+          }
+          break;
+        }
+        default:  // kBermFloat
+#pragma unroll
+          for (int i = 0; i < PPT; ++i) {
+            const R e = exOf(bm, i);
+            if (e >= R(0) && e <= static_cast<R>(extra)) term[i] = (c * fix(slot, i) + rec[5]) * (rec[3] * fastExp(nB * x[i]));
+          }
+        }
+    }
+    if (kPerTrade && A.nTr > 0) {
+#pragma unroll
+      for (int i = 0; i < PPT; ++i) vt(grp, i) += term[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < PPT; ++i) value[i] = kLean ? value[i] + term[i] : addRn(value[i], term[i]);
+    }
+  }
+  for (uint32_t u = d1.x; u < d1.y; ++u) {  // fixings, after every use of the previous fixing
+    const R4 r = ld4(table + 4 * u);
+    const uint32_t slot = asUint(r.w);
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) fix(slot, i) = (r.x * termExp(r.y, x[i]) - R(1)) * r.z;
+  }
+  for (uint32_t g = 0; g < nTr; ++g)
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) value[i] += vt(g, i);
+}
+
 // Resident CTAs per SM the lean variants are compiled for (register budget 65536 / (128 x blocks)).  The
 // shared-memory state of a netting set with many swap slots allows 6 CTAs of 2-path threads; netting sets
 // with little state (kSmallState: at most kSmallStateWords words per path) fit 8, and their variant is
@@ -507,7 +766,9 @@ __global__ void __launch_bounds__(kTile, (revalueMinBlocks<PPT, kLean, kSmallSta
   for (int i = 0; i < PPT; ++i) cubeP[i] = cb.data + pp[i];
   auto cube = [&](uint32_t field, uint32_t j, int i) { return cubeP[i][field * fieldStride + static_cast<size_t>(j) * nP]; };
 
-  R held[PPT], prevDE[PPT], prevQ[PPT], prevRV[PPT], ex[4][PPT];
+  R held[PPT], prevDE[PPT], prevQ[PPT], prevRV[PPT], ex[4][PPT], noXf[2][PPT];  // noXf: the terms read x_f from the cube
+#pragma unroll
+  for (int i = 0; i < PPT; ++i) noXf[0][i] = noXf[1][i] = R(0);
   // The exercise index (-1: not exercised) of Bermudan b on the thread's path i.
   auto exOf = [&](uint32_t b, int i) -> R {
     return manyBerm ? static_cast<R>(exS[(b * PPT + i) * kTile + tid]) : pick4<R, PPT>(ex, b, i);
@@ -596,224 +857,9 @@ __global__ void __launch_bounds__(kTile, (revalueMinBlocks<PPT, kLean, kSmallSta
           A.sinkD[static_cast<size_t>(j) * nP + pth[i]] = D[i];
         }
 
-    R value[PPT], ev[4][PPT];
-    R annS[PPT], fltS[PPT];  // the co-terminal swap of the next two-regressor record: annuity, float leg
-#pragma unroll
-    for (int i = 0; i < PPT; ++i) {
-      value[i] = R(0), annS[i] = R(0), fltS[i] = R(0);
-#pragma unroll
-      for (int b = 0; b < 4; ++b) ev[b][i] = R(0);
-    }
-    using R4 = typename Vec4<R>::T;
-    for (uint32_t u = d0.x; u < d0.y; ++u) {  // running floating coupons
-      const R4 r = ld4(table + 4 * u);
-      const uint32_t slot = static_cast<uint32_t>(r.w);
-#pragma unroll
-      for (int i = 0; i < PPT; ++i) value[i] += (r.x * fix(slot, i) + r.y) * termExp(r.z, x[i]);
-    }
-#pragma unroll 2
-    for (uint32_t u = d0.y; u < d0.z; ++u) {  // bonds, two per record
-      const R4 r = ld4(table + 4 * u);
-#pragma unroll
-      for (int i = 0; i < PPT; ++i) value[i] += r.x * termExp(r.y, x[i]) + r.z * termExp(r.w, x[i]);
-    }
-    for (uint32_t u = d0.z; u < d0.w; ++u) {  // asset forwards: (c, A, asset)
-      const R4 r = ld4(table + 4 * u);
-      const uint32_t a = static_cast<uint32_t>(r.z) & 3u;
-#pragma unroll
-      for (int i = 0; i < PPT; ++i) value[i] += r.x * pick4<R, PPT>(S, a, i) * r.y;
-    }
-    if (kPerTrade && A.nTr > 0)
-      for (uint32_t g = 0; g < kMaxTradeGroups; ++g)
-#pragma unroll
-        for (int i = 0; i < PPT; ++i) vt(g, i) = R(0);
-    for (uint32_t u = d0.w; u < d1.x; u += 2) {  // generic terms: the reference's records
-      R rec[8];
-      loadTerm(table + 4 * u, rec);
-      const uint32_t code = static_cast<uint32_t>(rec[0]);
-      const uint32_t kind = code & 15u, bm = bermudanOf(code, manyBerm), extra = code >> 12u;
-      const uint32_t grp = min((code >> 4u) & 15u, 15u);
-      if (!kLean && kind == kBermBond && rec[1] < R(0)) {
-        // A block of nb bonds of Bermudan bm (the lowering's run of its kBermBond records): each counts on a path
-        // that exercised at or before the bond's exercise index; a warp with no such path skips the block.
-        const uint32_t nb = static_cast<uint32_t>(-rec[1]);
-        R exi[PPT];
-        bool live = false;
-#pragma unroll
-        for (int i = 0; i < PPT; ++i) exi[i] = exOf(bm, i), live = live || (exi[i] >= R(0) && exi[i] <= rec[2]);
-        if (__any_sync(0xFFFFFFFFu, live))
-          for (uint32_t q = 0; q < nb; ++q) {
-            const R4 b = ld4(table + 4 * (u + 2 + q));
-            const R nBq = -b.z;
-#pragma unroll
-            for (int i = 0; i < PPT; ++i) {
-              R term = R(0);
-              if (exi[i] >= R(0) && exi[i] <= b.w) term = b.x * (b.y * fastExp(nBq * x[i]));
-              if (kPerTrade && A.nTr > 0) vt(grp, i) += term;
-              else value[i] += term;
-            }
-          }
-        u += 2 * ((nb + 1) / 2);
-        continue;
-      }
-      const uint32_t slot = static_cast<uint32_t>(rec[1]);
-      const R c = rec[2], nB = -rec[4];
-      R term[PPT];
-#pragma unroll
-      for (int i = 0; i < PPT; ++i) term[i] = R(0);
-      switch (kind) {
-        case kBond:
-#pragma unroll
-          for (int i = 0; i < PPT; ++i) term[i] = c * (rec[3] * fastExp(nB * x[i]));
-          break;
-        case kFixedFloat:
-#pragma unroll
-          for (int i = 0; i < PPT; ++i) term[i] = (c * fix(slot, i) + rec[5]) * (rec[3] * fastExp(nB * x[i]));
-          break;
-        case kAsset:
-#pragma unroll
-          for (int i = 0; i < PPT; ++i) term[i] = c * pick4<R, PPT>(S, slot & 3u, i) * rec[3];
-          break;
-        case kSetFixing:
-#pragma unroll
-          for (int i = 0; i < PPT; ++i) fix(slot, i) = (rec[3] * fastExp(nB * x[i]) - R(1)) / c;
-          break;
-        case kOption: {
-          const R p3 = rec[7];
-#pragma unroll
-          for (int i = 0; i < PPT; ++i) {
-            const R b0 = rec[3] * fastExp(nB * x[i]);
-            term[i] = c * black(pick4<R, PPT>(S, slot & 3u, i) * rec[5] / b0, rec[6], fabs(p3), b0, p3 > R(0));
-          }
-          break;
-        }
-        case kForeignForward: {  // c S P_f(t, T | x_f), P_f = A_f e^{-B_f x_f}: the foreign bond of the asset's currency
-          const uint32_t a = min(extra, 1u);
-#pragma unroll
-          for (int i = 0; i < PPT; ++i) term[i] = c * pick4<R, PPT>(S, a, i) * (rec[3] * fastExp(-rec[1] * cube(cb.fXf + a, j, i)));
-          break;
-        }
-        case kForeignOption: {  // Black on S P_f(t, T | x_f) / P(t, T | x)
-          const uint32_t a = min(extra, 1u);
-          const R p3 = rec[7];
-#pragma unroll
-          for (int i = 0; i < PPT; ++i) {
-            const R b0 = rec[3] * fastExp(nB * x[i]);
-            const R q = rec[5] * fastExp(-rec[1] * cube(cb.fXf + a, j, i));
-            term[i] = c * black(pick4<R, PPT>(S, a, i) * q / b0, rec[6], fabs(p3), b0, p3 > R(0));
-          }
-          break;
-        }
-        default:
-          if constexpr (!kLean) switch (kind) {  // the AMC and probe terms (absent from lean launches)
-          case kBermExercise:
-  #pragma unroll
-            for (int i = 0; i < PPT; ++i) {
-              const R v = c * (rec[3] * fastExp(nB * x[i]));
-              if (manyBerm || bm == 0) ev[0][i] += v;  // with many Bermudans, one running value: its policy follows
-              else if (bm == 1) ev[1][i] += v;
-              else if (bm == 2) ev[2][i] += v;
-              else ev[3][i] += v;
-            }
-            break;
-          case kBermAnnuity:
-  #pragma unroll
-            for (int i = 0; i < PPT; ++i) annS[i] += c * (rec[3] * fastExp(nB * x[i]));
-            break;
-          case kBermCoterm:
-  #pragma unroll
-            for (int i = 0; i < PPT; ++i) fltS[i] += c * (rec[3] * fastExp(nB * x[i]));
-            break;
-          case kBermExt:
-            break;  // read with its policy or continuation record
-          case kBermDecide: {
-            R e1[8], e2[8];
-            const bool twoD = twoRegressors(table, u, d1.x, e1, e2);
-  #pragma unroll
-            for (int i = 0; i < PPT; ++i) {
-              const R e = manyBerm ? ev[0][i] : pick4<R, PPT>(ev, bm, i);
-              if (manyBerm) ev[0][i] = R(0);
-              const R cont = twoD ? amcPoly2(rec, e1, e2, x[i], swapRate(fltS[i], annS[i])) : amcPoly(rec, x[i]);
-              annS[i] = R(0), fltS[i] = R(0);
-              if (kSink) {
-                if (act[i]) A.sinkEx[static_cast<size_t>(A.sinkRowOfBermudan[bm] + extra) * nP + pth[i]] = e;
-              } else if (exOf(bm, i) < R(0)) {
-                // the exact-decision check: the rule's margins are e (against 0) and e - cont
-                if (act[i] && (fabs(e) <= guardJ || fabs(e - cont) <= guardJ)) flagPath(A.flags, pth[i]);
-                if (e > R(0) && e > cont) {
-                  const R v = static_cast<R>(extra);
-                  if (manyBerm) exS[(bm * PPT + i) * kTile + tid] = static_cast<signed char>(extra);
-                  else if (bm == 0) ex[0][i] = v;
-                  else if (bm == 1) ex[1][i] = v;
-                  else if (bm == 2) ex[2][i] = v;
-                  else ex[3][i] = v;
-                }
-              }
-            }
-            break;
-          }
-          case kBermContinue: {
-            R e1[8], e2[8];
-            const bool twoD = twoRegressors(table, u, d1.x, e1, e2);
-  #pragma unroll
-            for (int i = 0; i < PPT; ++i) {
-              const R cont = twoD ? amcPoly2(rec, e1, e2, x[i], swapRate(fltS[i], annS[i])) : amcPoly(rec, x[i]);
-              annS[i] = R(0), fltS[i] = R(0);
-              if (exOf(bm, i) < R(0)) term[i] = rec[1] * fmax(cont, R(0));
-            }
-            break;
-          }
-          case kBermBond:
-  #pragma unroll
-            for (int i = 0; i < PPT; ++i) {
-              const R e = exOf(bm, i);
-              if (e >= R(0) && e <= static_cast<R>(extra)) term[i] = c * (rec[3] * fastExp(nB * x[i]));
-            }
-            break;
-          case kProbe: {
-            const uint32_t what = slot & 15u, ix = min(slot >> 4u, 3u), ic = min(ix, 1u);
-  #pragma unroll
-            for (int i = 0; i < PPT; ++i) {
-              R q;
-              switch (what) {
-                case 0: q = x[i]; break;
-                case 1: q = D[i]; break;
-                case 2: q = pick4<R, PPT>(S, ix, i); break;
-                case 3: q = ix < cb.nA ? cube(cb.fLnS + ix, j, i) : R(0); break;
-                case 4: q = ic < cb.nC ? cube(cb.fY + ic, j, i) : R(0); break;
-                case 5: q = ic < cb.nC ? cube(cb.fQ + ic, j, i) : R(1); break;
-                case 6: q = D[i] * pick4<R, PPT>(S, ix, i); break;
-                default: q = D[i] * (rec[3] * fastExp(nB * x[i]));
-              }
-              if (!kSink && act[i]) expo[static_cast<size_t>(static_cast<uint32_t>(rec[5])) * nP + pth[i]] = q + c;
-            }
-            break;
-          }
-          default:  // kBermFloat
-  #pragma unroll
-            for (int i = 0; i < PPT; ++i) {
-              const R e = exOf(bm, i);
-              if (e >= R(0) && e <= static_cast<R>(extra)) term[i] = (c * fix(slot, i) + rec[5]) * (rec[3] * fastExp(nB * x[i]));
-            }
-          }
-      }
-      if (kPerTrade && A.nTr > 0) {
-#pragma unroll
-        for (int i = 0; i < PPT; ++i) vt(grp, i) += term[i];
-      } else {
-#pragma unroll
-        for (int i = 0; i < PPT; ++i) value[i] += term[i];
-      }
-    }
-    for (uint32_t u = d1.x; u < d1.y; ++u) {  // fixings, after every use of the previous fixing
-      const R4 r = ld4(table + 4 * u);
-      const uint32_t slot = static_cast<uint32_t>(r.w);
-#pragma unroll
-      for (int i = 0; i < PPT; ++i) fix(slot, i) = (r.x * termExp(r.y, x[i]) - R(1)) * r.z;
-    }
-    for (uint32_t g = 0; g < nTr; ++g)
-#pragma unroll
-      for (int i = 0; i < PPT; ++i) value[i] += vt(g, i);
+    R value[PPT];
+    revalueDate<R, PPT, kPerTrade, kSink, kLean, false>(A, cb, cubeP, d0, d1, j, tid, pth, act, x, D, S, noXf, guardJ, state, vtBuf, exS,
+                                                        manyBerm, ex, value);
     if (kSink) continue;
 
     // ---- CSA: collateral called on the value at t - MPR (collateral.cpp:10-47) ----
@@ -944,6 +990,378 @@ __global__ void __launch_bounds__(kTile, (revalueMinBlocks<PPT, kLean, kSmallSta
 }
 
 // ---------------------------------------------------------------------------------------------
+// The same revaluation split over the dates.  revalueKernel walks every date of a (path tile, netting set) in one CTA: a
+// launch of few paths, or of netting sets of very different sizes, leaves most of the GPU idle or waiting for the
+// largest.  What is serial in the dates is little: a fixing needs its own date's short rate only, an exercise decision
+// its own date's state and whether an earlier one was taken, the collateral one comparison per date.  So
+//   decideKernel  per (paths, Bermudan): the exercise date chosen, from the exercise dates' records alone;
+//   valueKernel   per (path tile, netting set, run of dates): the netted values, into A.vals [date][path];
+//   settleKernel  per (32 paths, netting set): the collateral walk over the dates by one warp, then rows and statistics of
+//                 the dates by all eight.
+// Same arithmetic per date as revalueKernel (revalueDate), same statistics tree: the same results.
+// Revaluation before and after (us): 2,000 paths x 121 dates of 3 trades 146 and 20, 10,000 x 61 of 20 swaps 203 and 31, 12
+// netting sets of 119 trades at 33,333 paths x 169 dates 1,497 and 1,077, 24 + 24 netting sets with 40
+// Bermudans among 800 trades at 65,536 x 241 66,061 and 28,457.
+template <typename R>
+__global__ void __launch_bounds__(kTile) decideKernel(const CubeArgs<R> cb, const NsArgs<R>* __restrict__ nsArgs,
+                                                      const DecideJob* __restrict__ jobs, const R* __restrict__ table) {
+  const DecideJob J = jobs[blockIdx.y];
+  const NsArgs<R>& A = nsArgs[J.ns];
+  const uint32_t nP = cb.nP, p = blockIdx.x * kTile + threadIdx.x;
+  if (p >= nP) return;
+  const bool many = A.manyBerm != 0;
+  R x = R(0), ev = R(0), ann = R(0), flt = R(0), guardJ = R(-1), ex = R(-1);
+  for (uint32_t u = J.begin; u < J.end; u += 2) {
+    R rec[8];
+    loadTerm(table + 4 * u, rec);
+    const uint32_t code = asUint(rec[0]), kind = code & 15u;
+    if (kind == kBond) {  // the records of date rec[1] follow
+      const uint32_t j = asUint(rec[1]);
+      x = __ldg(cb.data + static_cast<size_t>(j) * nP + p);
+      ev = ann = flt = R(0);
+      guardJ = A.flags ? A.guard[j] : R(-1);
+      continue;
+    }
+    if (kind == kBermDecide) {
+      R e1[8], e2[8];
+      const bool twoD = twoRegressors(table, u, J.end, e1, e2);
+      const R cont = twoD ? amcPoly2(rec, e1, e2, x, swapRate(flt, ann)) : amcPoly(rec, x);
+      ann = flt = R(0);
+      if (ex < R(0)) {
+        if (fabs(ev) <= guardJ || fabs(ev - cont) <= guardJ) flagPath(A.flags, p);
+        if (ev > R(0) && ev > cont) ex = static_cast<R>(code >> 12u);
+      }
+      if (many) ev = R(0);
+    } else if (kind != kBermExt) {
+      const R v = rec[2] * (rec[3] * fastExp(-rec[4] * x));
+      if (kind == kBermExercise) ev += v;
+      else if (kind == kBermAnnuity) ann += v;
+      else flt += v;
+    }
+  }
+  A.exIndex[static_cast<size_t>(J.berm) * nP + p] = static_cast<signed char>(ex);
+  if (A.rowEx != kNoRow && (many || J.berm < 4u)) A.expo[(A.rowEx + J.berm) * static_cast<size_t>(nP) + p] = ex;
+}
+
+template <typename R, int PPT, bool kLean>
+__global__ void __launch_bounds__(kTile, (sizeof(R) == 8 ? 4 : kLean ? 8 : 6)) valueKernel(
+    const CubeArgs<R> cb, const NsArgs<R>* __restrict__ nsArgs, const ValueItem* __restrict__ items, const uint2* __restrict__ pre,
+    const uint8_t* __restrict__ exFirst, uint32_t pathBegin, uint32_t slabPaths) {
+  extern __shared__ __align__(16) unsigned char smemRaw[];
+  __shared__ NsArgs<R> sA;
+  R* state = reinterpret_cast<R*>(smemRaw);
+  const ValueItem I = items[blockIdx.y];
+  const uint32_t tid = threadIdx.x;
+  if (tid < sizeof(NsArgs<R>) / 4) reinterpret_cast<uint32_t*>(&sA)[tid] = reinterpret_cast<const uint32_t*>(nsArgs + I.ns)[tid];
+  __syncthreads();
+  const NsArgs<R>& A = sA;
+  const uint32_t nP = cb.nP, nT = cb.nT, nSlots = A.nSlots, last = min(pathBegin + slabPaths, nP);
+  uint32_t pth[PPT], pp[PPT];
+  bool act[PPT];
+#pragma unroll
+  for (int i = 0; i < PPT; ++i) {
+    pth[i] = pathBegin + (blockIdx.x * kTile + tid) * PPT + i;
+    act[i] = pth[i] < last;
+    pp[i] = act[i] ? pth[i] : nP % PPT == 0 ? nP - PPT + i : nP - 1;
+  }
+  const size_t fieldStride = static_cast<size_t>(nT) * nP;
+  const R* cubeP[PPT];
+#pragma unroll
+  for (int i = 0; i < PPT; ++i) cubeP[i] = cb.data + pp[i];
+  const bool vecPaths = PPT > 1 && nP % PPT == 0;
+  auto load = [&](size_t at, R (&v)[PPT]) {
+    if (vecPaths) {
+      ldPaths<R, PPT>(cubeP[0] + at, v);
+    } else {
+#pragma unroll
+      for (int i = 0; i < PPT; ++i) v[i] = __ldg(cubeP[i] + at);
+    }
+  };
+  // The fixings that the run's first dates read, each from its own date's short rate; fixings never set are zero.
+  for (uint32_t q = 0; q < nSlots; ++q)
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) state[(q * PPT + i) * kTile + tid] = R(0);
+  for (uint32_t q = I.preBegin; q < I.preEnd; ++q) {
+    const uint2 f = __ldg(pre + q);  // fixing record, date
+    const auto r = ld4(A.table + 4 * static_cast<size_t>(f.x));
+    R x[PPT];
+    load(static_cast<size_t>(f.y) * nP, x);
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) state[(asUint(r.w) * PPT + i) * kTile + tid] = (r.x * termExp(r.y, x[i]) - R(1)) * r.z;
+  }
+  signed char* exS = reinterpret_cast<signed char*>(state + static_cast<size_t>(nSlots) * PPT * kTile);
+  if constexpr (!kLean)
+    for (uint32_t b = 0; b < A.nBerm; ++b) {
+      const int e0 = exFirst[I.exAt + b];  // exercises decided before the run
+#pragma unroll
+      for (int i = 0; i < PPT; ++i) {
+        const int e = A.exIndex[static_cast<size_t>(b) * nP + pp[i]];
+        exS[(b * PPT + i) * kTile + tid] = static_cast<signed char>(e < e0 ? e : -1);
+      }
+    }
+  const uint4* __restrict__ dates = reinterpret_cast<const uint4*>(A.dates);
+  const size_t sOff = static_cast<size_t>(cb.fS) * fieldStride, fOff = static_cast<size_t>(cb.fXf) * fieldStride;
+  R nx[PPT], nD[PPT], nS4[4][PPT], nXf[2][PPT];
+  auto loadFactors = [&](uint32_t j) {
+    const size_t off = static_cast<size_t>(j) * nP;
+    load(off, nx);
+    if constexpr (!kLean) load(off + fieldStride, nD);  // probes
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+      if (A.usesAssets && static_cast<uint32_t>(a) < cb.nA) load(off + sOff + a * fieldStride, nS4[a]);
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+      if (A.usesForeign && static_cast<uint32_t>(a) < cb.nF) load(off + fOff + a * fieldStride, nXf[a]);
+  };
+#pragma unroll
+  for (int i = 0; i < PPT; ++i) {
+    nD[i] = R(0);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) nS4[a][i] = R(0);
+    nXf[0][i] = nXf[1][i] = R(0);
+  }
+  loadFactors(I.j0);
+  uint4 nd0 = __ldg(dates + 2 * I.j0), nd1 = __ldg(dates + 2 * I.j0 + 1);
+  for (uint32_t j = I.j0; j < I.j1; ++j) {
+    R x[PPT], D[PPT], S[4][PPT], xf[2][PPT], ex[4][PPT], value[PPT];
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) {
+      x[i] = nx[i], D[i] = nD[i], xf[0][i] = nXf[0][i], xf[1][i] = nXf[1][i];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) S[a][i] = nS4[a][i], ex[a][i] = R(-1);
+    }
+    const uint4 d0 = nd0, d1 = nd1;
+    if (j + 1 < I.j1) {
+      loadFactors(j + 1);
+      nd0 = __ldg(dates + 2 * (j + 1)), nd1 = __ldg(dates + 2 * (j + 1) + 1);
+      prefetchDate<R>(nd0.x, nd1.y, A.table, tid);
+    }
+    revalueDate<R, PPT, false, false, kLean, true>(A, cb, cubeP, d0, d1, j, tid, pth, act, x, D, S, xf, R(-1), state, nullptr, exS, true, ex,
+                                                   value);
+    R* dst = A.vals + static_cast<size_t>(j) * slabPaths + (pth[0] - pathBegin);
+    if (vecPaths && slabPaths % PPT == 0) {
+      if (act[0]) stPaths<R, PPT>(dst, value);
+    } else {
+#pragma unroll
+      for (int i = 0; i < PPT; ++i)
+        if (act[i]) dst[i] = value[i];
+    }
+    if (!kLean && A.imState && d1.w > 0) {  // the start of the paths' inner paths
+#pragma unroll
+      for (int i = 0; i < PPT; ++i)
+        if (act[i]) {
+          R* st = A.imState + static_cast<size_t>(d1.w - 1) * A.imWords * nP + pth[i];
+          st[0] = value[i];
+#pragma unroll
+          for (uint32_t b = 0; b < 4; ++b)
+            st[static_cast<size_t>(1 + b) * nP] = b < A.nBerm ? static_cast<R>(exS[(b * PPT + i) * kTile + tid]) : R(-1);
+          for (uint32_t q = 0; q < nSlots; ++q) st[static_cast<size_t>(5 + q) * nP] = state[(q * PPT + i) * kTile + tid];
+        }
+    }
+  }
+}
+
+constexpr uint32_t kSettleThreads = 256, kSettleWarps = kSettleThreads / 32;
+
+// What a CTA of settleKernel holds of kDates dates and its 32 V paths; rows padded so that a column's walk over the paths
+// by one thread per date meets no bank conflict.
+template <typename R, int V>
+struct SettleSmem {
+  static constexpr uint32_t kDates = sizeof(R) * V == 4 ? 64 : 32, kRow = 32 * V + 1;
+  R v[kDates][kRow];  // values, then exposures e
+  R c[kDates][kRow];  // required collateral, then collateral, then D max(e, 0); the sums' parts with d
+  R d[kDates][kRow];  // deflators
+  R q[kDates][kRow];  // the counterparty's survival
+  R lastDE[32 * V], lastQ[32 * V];  // D max(e, 0) and Q of the last reporting date before them
+  uint32_t call[kDates], slot[kDates], prev[kDates];  // margin-call date, reporting slot, previous reporting date (kNoRow: none)
+};
+
+// V: paths per lane, 32 apart (a row's address and loop are shared by them).
+template <typename R, int V>
+__global__ void __launch_bounds__(kSettleThreads) settleKernel(const CubeArgs<R> cb, const NsArgs<R>* __restrict__ nsArgs, uint32_t pathBegin,
+                                                               uint32_t slabPaths) {
+  extern __shared__ __align__(16) unsigned char smemRaw[];
+  __shared__ NsArgs<R> sA;
+  SettleSmem<R, V>& s = *reinterpret_cast<SettleSmem<R, V>*>(smemRaw);
+  constexpr uint32_t kDates = SettleSmem<R, V>::kDates, kGroups = kSettleThreads / kDates, kPer = 32 * V / kGroups;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  if (tid < sizeof(NsArgs<R>) / 4) reinterpret_cast<uint32_t*>(&sA)[tid] = reinterpret_cast<const uint32_t*>(nsArgs + blockIdx.y)[tid];
+  if (tid < 32 * V) s.lastDE[tid] = R(0), s.lastQ[tid] = R(1);
+  __syncthreads();
+  const NsArgs<R>& A = sA;
+  const uint32_t nP = cb.nP, nT = cb.nT, first = pathBegin + blockIdx.x * 32u * V;
+  const uint32_t live = min(32u * V, min(pathBegin + slabPaths, nP) - first);  // the CTA's paths
+  const bool hasCsa = A.hasCsa != 0, hasQ = A.cpty < cb.nC;
+  const uint32_t unit = first / (32u * V);
+  uint32_t at[V];  // the lane's paths from `first`; past the last path they repeat it and write nothing
+#pragma unroll
+  for (int i = 0; i < V; ++i) at[i] = min(lane + 32u * i, live - 1);
+  const R* __restrict__ vals = A.vals + (first - pathBegin);
+  const size_t fieldStride = static_cast<size_t>(nT) * nP;
+  const R* __restrict__ cube = cb.data + first;
+  const size_t qOff = hasQ ? (cb.fQ + A.cpty) * fieldStride : 0;
+  R held[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) held[i] = R(0);
+  uint32_t lastRep = kNoRow;
+  for (uint32_t j0 = 0; j0 < nT; j0 += kDates) {
+    const uint32_t n = min(kDates, nT - j0);
+#pragma unroll 4
+    for (uint32_t k = warp; k < n; k += kSettleWarps) {
+      const R* pv = vals + static_cast<size_t>(j0 + k) * slabPaths;
+      const R* pd = cube + fieldStride + static_cast<size_t>(j0 + k) * nP;
+      const R* pq = cube + qOff + static_cast<size_t>(j0 + k) * nP;
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        s.v[k][lane + 32 * i] = __ldg(pv + at[i]);
+        s.d[k][lane + 32 * i] = __ldg(pd + at[i]);
+        s.q[k][lane + 32 * i] = hasQ ? __ldg(pq + at[i]) : R(1);
+      }
+    }
+    if (tid < n) {
+      const uint2 w = __ldg(reinterpret_cast<const uint2*>(A.dates + 8 * static_cast<size_t>(j0 + tid) + 6));
+      s.call[tid] = w.x, s.slot[tid] = w.y;
+    }
+    __syncthreads();
+    if (tid < n) {
+      uint32_t k = tid;
+      while (k > 0 && s.slot[k - 1] == 0) --k;
+      s.prev[tid] = k > 0 ? j0 + k - 1 : lastRep;
+    }
+    // ---- CSA: collateral called on the value at t - MPR (collateral.cpp:10-47) ----
+    if (hasCsa) {
+      for (uint32_t k = warp; k < n; k += kSettleWarps) {
+        const uint32_t callJ = s.call[k];
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          const R vc = callJ >= j0 ? s.v[callJ - j0][lane + 32 * i] : __ldg(vals + static_cast<size_t>(callJ) * slabPaths + at[i]);
+          R required = R(0);
+          if (vc > A.hc) required += vc - A.hc;
+          if (A.hb >= R(0) && -vc > A.hb) required -= -vc - A.hb;
+          s.c[k][lane + 32 * i] = required;
+        }
+      }
+      __syncthreads();
+      if (warp == 0) {  // the one serial step: the collateral held, date by date
+        if (A.ctype == 0 && !A.flags) {  // cash: one unit is worth one, no division
+          const R mta = A.mta, ia = A.ia;
+#pragma unroll 8
+          for (uint32_t k = 0; k < n; ++k)
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+              const R required = s.c[k][lane + 32 * i];
+              if (j0 + k == 0 || fabs(required - held[i]) >= mta) held[i] = required;
+              s.c[k][lane + 32 * i] = held[i] + ia;
+            }
+        } else {
+          auto price = [&](uint32_t j, uint32_t p) -> R {
+            if (A.ctype == 1) {
+              const R* st = A.steps + static_cast<size_t>(j) * A.stepStride;
+              return st[22] * rexp(-st[23] * __ldg(cube + static_cast<size_t>(j) * nP + p));
+            }
+            return A.ctype == 2 ? __ldg(cube + (cb.fS + min(A.casset, 3u)) * fieldStride + static_cast<size_t>(j) * nP + p) : R(1);
+          };
+          for (uint32_t k = 0; k < n; ++k)
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+              const uint32_t j = j0 + k, callJ = s.call[k];
+              const R guardJ = A.flags ? A.guard[j] : R(-1);  // < 0: no check
+              const R required = s.c[k][lane + 32 * i], pj = price(j, at[i]), pCall = callJ != j ? price(callJ, at[i]) : pj;
+              const R gap = A.ctype == 0 ? fabs(required - held[i]) : fabs(required - held[i] * A.keepHaircut * pCall);
+              if (j > 0 && lane + 32 * i < live && fabs(gap - A.mta) <= guardJ) flagPath(A.flags, first + lane + 32 * i);
+              if (j == 0 || gap >= A.mta) held[i] = A.ctype == 0 ? required : required / (A.keepHaircut * pCall);
+              s.c[k][lane + 32 * i] = held[i] * pj + A.ia;
+            }
+        }
+      }
+    }
+    __syncthreads();
+    // ---- exposures and the reporting dates' rows ----
+    for (uint32_t k = warp; k < n; k += kSettleWarps) {
+      const uint32_t rs = s.slot[k];
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        const uint32_t col = lane + 32 * i;
+        const R value = s.v[k][col], collateral = hasCsa ? s.c[k][col] : R(0), e = value - collateral, ep = fmax(e, R(0));
+        s.v[k][col] = e;
+        s.c[k][col] = mulRn(s.d[k][col], ep);
+        if (rs > 0 && col < live) {
+          const size_t row = static_cast<size_t>(rs - 1) * nP + first + col;
+          A.expo[static_cast<size_t>(A.rowEP) * nP + row] = ep;
+          if (A.moreRows) {
+            if (A.rowDV != kNoRow) {
+              const R before = s.prev[k] != kNoRow ? __ldg(vals + static_cast<size_t>(s.prev[k]) * slabPaths + col) : R(0);
+              A.expo[static_cast<size_t>(A.rowDV) * nP + row] = rs == 1 ? R(0) : fabs(value - before);
+            }
+            if (A.rowE != kNoRow) A.expo[static_cast<size_t>(A.rowE) * nP + row] = e;
+            if (A.rowV != kNoRow) A.expo[static_cast<size_t>(A.rowV) * nP + row] = value;
+            if (A.rowC != kNoRow) A.expo[static_cast<size_t>(A.rowC) * nP + row] = collateral;
+            if (A.rowGross != kNoRow) A.expo[static_cast<size_t>(A.rowGross) * nP + row] = R(0);  // no trade groups here
+          }
+        }
+      }
+    }
+    __syncthreads();
+    // ---- the 8 statistics of each date: a thread sums kPer adjacent paths of one date as a binary tree, then the groups
+    // are added as one: revalueKernel's tree over the paths, and its roundings ----
+    const uint32_t k = tid % kDates, g = tid / kDates;
+    R sum[8];
+    if (k < n) {
+      const bool rep = s.slot[k] > 0 && j0 + k > 0;
+      const uint32_t pk = s.prev[k];
+      const bool inside = pk != kNoRow && pk >= j0;  // else the last reporting date before these, or none (DE 0, Q 1)
+      const R* prevDE = inside ? s.c[pk - j0] : s.lastDE;
+      const R* prevQ = inside ? s.q[pk - j0] : s.lastQ;
+      R level[4][8];  // the sums of 1, 2, 4 paths that wait for their neighbour
+#pragma unroll
+      for (uint32_t u = 0; u < kPer; ++u) {
+        const uint32_t i = g * kPer + u;
+        R t[8] = {R(0), R(0), R(0), R(0), R(0), R(0), R(0), R(0)};
+        if (i < live) {
+          const R e = s.v[k][i], D = s.d[k][i], Q = s.q[k][i], ep = fmax(e, R(0)), en = fmin(e, R(0));
+          t[0] = e, t[1] = ep, t[2] = en, t[3] = s.c[k][i], t[4] = mulRn(D, en), t[6] = Q, t[7] = D;
+          if (rep) t[5] = mulRn(R(0.5) * (prevDE[i] + t[3]), prevQ[i] - Q);
+        }
+        uint32_t l = 0;
+#pragma unroll
+        for (uint32_t w = u; w & 1u; w >>= 1, ++l)
+#pragma unroll
+          for (int c = 0; c < 8; ++c) t[c] = level[l][c] + t[c];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) level[l][c] = t[c];
+        if (u + 1 == kPer)
+#pragma unroll
+          for (int c = 0; c < 8; ++c) sum[c] = t[c];
+      }
+    }
+    // The last reporting date so far, for the next dates.
+    uint32_t rep = n;
+    while (rep > 0 && s.slot[rep - 1] == 0) --rep;
+    const R de = rep > 0 && tid < 32 * V ? s.c[rep - 1][tid] : R(0), q = rep > 0 && tid < 32 * V ? s.q[rep - 1][tid] : R(0);
+    __syncthreads();
+    if (rep > 0 && tid < 32 * V) s.lastDE[tid] = de, s.lastQ[tid] = q;
+    if (rep > 0) lastRep = j0 + rep - 1;
+    R* part = &s.c[0][0];  // [kGroups][8][kDates + 1], over c and d
+    static_assert(sizeof(R) * kGroups * 8 * (kDates + 1) <= sizeof(s.c) + sizeof(s.d), "the parts fit");
+    if (k < n)
+#pragma unroll
+      for (int c = 0; c < 8; ++c) part[(g * 8 + c) * (kDates + 1) + k] = sum[c];
+    __syncthreads();
+    for (uint32_t o = tid; o < n * 8; o += kSettleThreads) {
+      const R* mine = part + (o % 8) * (kDates + 1) + o / 8;
+      auto of = [&](uint32_t h) { return mine[h * 8 * (kDates + 1)]; };
+      R t = (of(0) + of(1)) + (of(2) + of(3));
+      if constexpr (kGroups == 8) t = t + ((of(4) + of(5)) + (of(6) + of(7)));
+      A.partials[(static_cast<size_t>(unit) * nT + j0 + o / 8) * A.nS + o % 8] = t;
+    }
+    if (A.nS > 8)
+      for (uint32_t o = tid; o < n * (A.nS - 8); o += kSettleThreads)
+        A.partials[(static_cast<size_t>(unit) * nT + j0 + o / (A.nS - 8)) * A.nS + 8 + o % (A.nS - 8)] = R(0);
+    __syncthreads();  // before the next dates overwrite the shared memory
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
 // Nested Monte Carlo for the conditional initial margin (the reference's innerStep / innerValue and the
 // inner loop of simulatePath: fused_reference.cpp:108-196, 356-393).  The reference runs the nInner inner
 // paths of an outer path one after the other inside the path's thread; here one warp takes one
@@ -1002,7 +1420,7 @@ __device__ R innerDateValue(const ImArgs<R>& M, uint32_t jj, R x, const R (&S)[4
   R value = R(0), ev[4] = {R(0), R(0), R(0), R(0)};
   for (uint32_t u = d0.x; u < d0.y; ++u) {
     const R4 r = ld4(table + 4 * u);
-    value += (r.x * fix[static_cast<uint32_t>(r.w) * 32u] + r.y) * termExp(r.z, x);
+    value += (r.x * fix[asUint(r.w) * 32u] + r.y) * termExp(r.z, x);
   }
   for (uint32_t u = d0.y; u < d0.z; ++u) {
     const R4 r = ld4(table + 4 * u);
@@ -1010,15 +1428,15 @@ __device__ R innerDateValue(const ImArgs<R>& M, uint32_t jj, R x, const R (&S)[4
   }
   for (uint32_t u = d0.z; u < d0.w; ++u) {
     const R4 r = ld4(table + 4 * u);
-    value += r.x * sel4(S, static_cast<uint32_t>(r.z) & 3u) * r.y;
+    value += r.x * sel4(S, asUint(r.z) & 3u) * r.y;
   }
   for (uint32_t u = d0.w; u < d1.x; u += 2) {
     R rec[8];
     loadTerm(table + 4 * u, rec);
-    const uint32_t code = static_cast<uint32_t>(rec[0]);
+    const uint32_t code = asUint(rec[0]), slot = asUint(rec[1]);
     const uint32_t kind = code & 15u, bm = min((code >> 8u) & 15u, 3u), extra = code >> 12u;
-    if (kind == kBermBond && rec[1] < R(0)) {  // a block of the Bermudan's bonds (see the outer kernel)
-      const uint32_t nb = static_cast<uint32_t>(-rec[1]);
+    if (kind == kBermBond && slot >= kBlockMark) {  // a block of the Bermudan's bonds (see the outer kernel)
+      const uint32_t nb = slot - kBlockMark;
       const R e = sel4(ex, bm);
       if (e >= R(0) && e <= rec[2])
         for (uint32_t q = 0; q < nb; ++q) {
@@ -1028,7 +1446,6 @@ __device__ R innerDateValue(const ImArgs<R>& M, uint32_t jj, R x, const R (&S)[4
       u += 2 * ((nb + 1) / 2);
       continue;
     }
-    const uint32_t slot = static_cast<uint32_t>(rec[1]);
     const R c = rec[2];
     switch (kind) {
       case kBond: value += c * (rec[3] * fastExp(-rec[4] * x)); break;
@@ -1062,7 +1479,7 @@ __device__ R innerDateValue(const ImArgs<R>& M, uint32_t jj, R x, const R (&S)[4
   }
   for (uint32_t u = d1.x; u < d1.y; ++u) {
     const R4 r = ld4(table + 4 * u);
-    fix[static_cast<uint32_t>(r.w) * 32u] = (r.x * termExp(r.y, x) - R(1)) * r.z;
+    fix[asUint(r.w) * 32u] = (r.x * termExp(r.y, x) - R(1)) * r.z;
   }
   return value;
 }
@@ -1232,6 +1649,43 @@ cudaError_t launchRevalue(const CubeArgs<R>& cb, const NsArgs<R>* nsArgs, uint32
   }
 }
 
+template <typename R>
+cudaError_t launchSplit(const CubeArgs<R>& cb, const NsArgs<R>* nsArgs, uint32_t numNs, const SplitArgs<R>& sp, cudaStream_t stream) {
+  if (numNs == 0 || sp.numItems == 0) return cudaSuccess;
+  if (numNs > 65535u || sp.numItems > 65535u || sp.numDecides > 65535u) return cudaErrorInvalidConfiguration;
+  if (sp.numDecides > 0) {
+    decideKernel<R><<<dim3((cb.nP + kTile - 1) / kTile, sp.numDecides), kTile, 0, stream>>>(cb, nsArgs, sp.decides, sp.decideTable);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  auto value = [&](auto kernel, bool lean, uint32_t at, uint32_t n) {
+    const uint32_t items = lean ? sp.numItems - sp.numFull : sp.numFull, tile = static_cast<uint32_t>(kTile * sp.ppt);
+    if (items == 0) return cudaSuccess;
+    const size_t smem = (sp.slotsMax[lean] * sizeof(R) + (lean ? 0u : sp.bermsMax)) * tile;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    kernel<<<dim3((n + tile - 1) / tile, items), kTile, smem, stream>>>(cb, nsArgs, sp.items + (lean ? sp.numFull : 0u), sp.pre, sp.exFirst, at,
+                                                                        sp.slabPaths);
+    return cudaGetLastError();
+  };
+  auto settle = [&](auto kernel, size_t smem, uint32_t paths, uint32_t at, uint32_t n) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    kernel<<<dim3((n + paths - 1) / paths, numNs), kSettleThreads, smem, stream>>>(cb, nsArgs, at, sp.slabPaths);
+    return cudaGetLastError();
+  };
+  for (uint32_t at = 0; at < cb.nP; at += sp.slabPaths) {
+    const uint32_t n = std::min(sp.slabPaths, cb.nP - at);
+    cudaError_t e = sp.ppt == 1 ? value(valueKernel<R, 1, false>, false, at, n) : value(valueKernel<R, 2, false>, false, at, n);
+    if (e == cudaSuccess) e = sp.ppt == 1 ? value(valueKernel<R, 1, true>, true, at, n) : value(valueKernel<R, 2, true>, true, at, n);
+    if (e == cudaSuccess) e = sp.settlePaths == 32 ? settle(settleKernel<R, 1>, sizeof(SettleSmem<R, 1>), 32u, at, n)
+                                                   : settle(settleKernel<R, 2>, sizeof(SettleSmem<R, 2>), 64u, at, n);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+template cudaError_t launchSplit<float>(const CubeArgs<float>&, const NsArgs<float>*, uint32_t, const SplitArgs<float>&, cudaStream_t);
+template cudaError_t launchSplit<double>(const CubeArgs<double>&, const NsArgs<double>*, uint32_t, const SplitArgs<double>&, cudaStream_t);
 template cudaError_t launchNestedIm<float>(const ImArgs<float>&, cudaStream_t);
 template cudaError_t launchNestedIm<double>(const ImArgs<double>&, cudaStream_t);
 template cudaError_t launchSimulate<float>(const ScenarioArgs<float>&, const CubeArgs<float>&, cudaStream_t);

@@ -5,6 +5,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cstring>
 #include <cuda_runtime.h>
 
 namespace zk {
@@ -53,6 +54,40 @@ enum HeaderWord : int {
   hTr = 18, hRowDV = 19, hRowE = 20, hRowV = 21, hRowC = 22, hRowGross = 23, hRowTrades = 24, hRowEx = 25,
   hReq = 26, hBerm = 27, hRowEP = 28, hRowIm = 29, hInner = 30, hImLevel = 31,
 };
+
+// In the lowered term tables (lowerTerms) the codes, slots and assets are integers by their bits, not converted values:
+// a conversion per record would run on the special-function unit beside the exponentials.  A block of Bermudan bonds has
+// kBlockMark + its length as its slot.
+__host__ __device__ __forceinline__ uint32_t asUint(float v) {
+#ifdef __CUDA_ARCH__
+  return __float_as_uint(v);
+#else
+  uint32_t u;
+  memcpy(&u, &v, 4);
+  return u;
+#endif
+}
+__host__ __device__ __forceinline__ uint32_t asUint(double v) {
+#ifdef __CUDA_ARCH__
+  return static_cast<uint32_t>(__double_as_longlong(v));
+#else
+  uint64_t u;
+  memcpy(&u, &v, 8);
+  return static_cast<uint32_t>(u);
+#endif
+}
+template <typename R>
+R bitsOfUint(uint32_t v) {
+  R r;
+  if constexpr (sizeof(R) == 4) {
+    memcpy(&r, &v, 4);
+  } else {
+    const uint64_t w = v;
+    memcpy(&r, &w, 8);
+  }
+  return r;
+}
+constexpr uint32_t kBlockMark = 0x80000000u;
 
 // Error word written by kernels (checked by the host after each launch sequence).
 enum DeviceError : uint32_t { kDevOk = 0, kDevTimeout = 1, kDevBadTerm = 2 };
@@ -104,7 +139,7 @@ struct NsArgs {
   uint32_t usesForeign;    // some term reads a foreign short-rate state
   uint32_t manyBerm;       // more than 4 Bermudans: exercise indices in shared memory, bytes [nBerm][PPT][kTile]
   uint32_t stepStride;     // values per row of `steps`
-  uint32_t pad0;
+  uint32_t moreRows;       // some row besides the exposure rows and the exercise rows
   // AMC state pass (zk_amc_states, zk_fit_amc): x / deflator [date][path] and exercise values [row][path].
   R* sinkX;
   R* sinkD;
@@ -120,6 +155,10 @@ struct NsArgs {
   // double precision.  flags null: off.
   uint32_t* flags;
   const R* guard;
+  // The split revaluation (valueKernel): the netted values [date][path of the slab] and the exercise chosen by each
+  // path [Bermudan][path] (-1: none).
+  R* vals;
+  signed char* exIndex;
 };
 
 // Marks path p for the double-precision re-check (a rare event: one atomic per flagged decision).
@@ -196,9 +235,9 @@ __device__ __forceinline__ double ncdf(double x) { return 0.5 * erfc(-x / 1.4142
 __device__ __forceinline__ float black(float F, float K, float sd, float df, bool isCall) {
   const float s = isCall ? 1.0f : -1.0f;
   if (sd <= 1e-7f || F <= 0.0f) return df * fmaxf(s * (F - K), 0.0f);
-  const float d1 = __fdividef(__logf(__fdividef(F, K)), sd) + 0.5f * sd;
+  const float d1 = fmaf(0.5f, sd, __fdividef(__logf(__fdividef(F, K)), sd));
   const float d2 = d1 - sd;
-  return df * s * (F * ncdf(s * d1) - K * ncdf(s * d2));
+  return df * s * fmaf(F, ncdf(s * d1), -__fmul_rn(K, ncdf(s * d2)));
 }
 __device__ __forceinline__ double black(double F, double K, double sd, double df, bool isCall) {
   const double s = isCall ? 1.0 : -1.0;

@@ -28,6 +28,32 @@ cudaError_t launchRevalue(const CubeArgs<R>& cb, const NsArgs<R>* nsArgs, uint32
                           bool cash = false);
 size_t revalueSmemBytes(size_t stateWordsMax, bool perTrade, bool f64, int ppt);
 
+// The revaluation split over the dates (valueKernel and the kernels beside it): a run of dates [j0, j1) of netting set ns,
+// the fixings set before it that it reads -- (record of the lowered table, date) pairs pre[preBegin, preEnd) -- and per
+// Bermudan the number of exercises decided before it, exFirst[exAt + b]; and per Bermudan the records of its exercise
+// dates in `decideTable` [begin, end), in units of 4 values: a record (kBond, date) before each date's; codes by their bits.
+struct ValueItem {
+  uint32_t ns, j0, j1, preBegin, preEnd, exAt, pad[2];
+};
+struct DecideJob {
+  uint32_t ns, berm, begin, end;
+};
+template <typename R>
+struct SplitArgs {
+  const ValueItem* items;
+  const uint2* pre;
+  const uint8_t* exFirst;
+  const DecideJob* decides;
+  const R* decideTable;
+  uint32_t numItems, numFull;      // the first numFull items: netting sets with AMC or probe terms or the nested margin
+  uint32_t numDecides, slabPaths;  // paths per slab: A.vals holds one slab's values
+  uint32_t slotsMax[2], bermsMax;  // the most fixing slots of the first numFull items' netting sets, of the others'; Bermudans
+  int ppt;                         // paths per thread of valueKernel (1 or 2)
+  uint32_t settlePaths;            // paths per CTA of settleKernel and per partial (32 or 64)
+};
+template <typename R>
+cudaError_t launchSplit(const CubeArgs<R>& cb, const NsArgs<R>* nsArgs, uint32_t numNs, const SplitArgs<R>& sp, cudaStream_t stream);
+
 // The nested initial margin of one plan (fused_reference.cpp:356-393), after its revalue launch: one warp
 // per (reporting slot, outer path), the lanes running the inner paths; the margin into rows rowIm + r.
 template <typename R>
