@@ -698,6 +698,7 @@ struct Batch {
   unsigned char* base = nullptr;     // device arena
   bool ownsArena = false;
   bool sink = false;
+  bool sinkPrograms = false;         // the state pass runs on the exercises' records (else on revalueKernel)
   bool exact = false;                // the exact-decision check: guard bands and flags (Dev::guard, Dev::flags)
   size_t flagsOff = 0, flagsBytes = 0;
   uint32_t exerciseRows = 0;
@@ -832,6 +833,55 @@ void formGroups(Batch<R>& B, typename Batch<R>::Launch& L, uint32_t mode, HostPo
   }
 }
 
+// The exercise dates of each Bermudan of netting set ns and, appended to jobs and table, its exercises' records date by
+// date as decideKernel reads them; false where the exercise indices do not follow the dates.
+template <typename R>
+bool exercisePrograms(const Plan<R>& P, uint32_t ns, std::vector<std::vector<uint32_t>>& exDates, std::vector<DecideJob>& jobs,
+                      std::vector<R>& table) {
+  const uint32_t* I = P.v.indices;
+  exDates.assign(P.nBerm, {});
+  std::vector<std::vector<R>> prog(P.nBerm);
+  for (uint32_t j = 0; j < P.nT; ++j) {
+    std::vector<std::vector<const R*>> flows(P.manyBerm ? 1 : P.nBerm);
+    std::vector<const R*> swap;
+    for (uint32_t t = I[j]; t < I[j + 1]; ++t) {
+      const R* r = P.v.terms + static_cast<size_t>(t) * kTermStride;
+      const uint32_t code = static_cast<uint32_t>(r[0]), kind = code & 15u;
+      if (kind == kBermAnnuity || kind == kBermCoterm) swap.push_back(r);
+      if (kind == kBermContinue) swap.clear();
+      if (kind != kBermExercise && kind != kBermDecide) continue;
+      const uint32_t b = bermudanOf(code, P.manyBerm);
+      auto& mine = flows[P.manyBerm ? 0 : b];
+      if (kind == kBermExercise) {
+        mine.push_back(r);
+        continue;
+      }
+      const uint32_t e = code >> 12u;
+      if (e != exDates[b].size() || (e > 0 && exDates[b].back() >= j)) return false;  // not the next exercise
+      exDates[b].push_back(j);
+      auto& out = prog[b];
+      auto put = [&](const R* q) {
+        out.insert(out.end(), q, q + kTermStride);
+        out[out.size() - kTermStride] = bitsOfUint<R>(static_cast<uint32_t>(q[0]));
+      };
+      const R mark[kTermStride] = {bitsOfUint<R>(kBond), bitsOfUint<R>(j), R(0), R(0), R(0), R(0), R(0), R(0)};
+      out.insert(out.end(), mark, mark + kTermStride);
+      for (const R* q : mine) put(q);
+      for (const R* q : swap) put(q);
+      put(r);
+      for (uint32_t u = t + 1; u < I[j + 1] && (static_cast<uint32_t>(r[(u - t) * kTermStride]) & 15u) == kBermExt; ++u) put(r + (u - t) * kTermStride);
+      swap.clear();
+      if (P.manyBerm) mine.clear();
+    }
+  }
+  for (uint32_t b = 0; b < P.nBerm; ++b) {
+    const uint32_t at = static_cast<uint32_t>(table.size() / 4);
+    table.insert(table.end(), prog[b].begin(), prog[b].end());
+    jobs.push_back({ns, b, at, static_cast<uint32_t>(table.size() / 4)});
+  }
+  return true;
+}
+
 // Sets up the split over the dates of a launch's netting sets [basisCount, n) (Launch::split), or leaves it off where
 // a plan needs revalueKernel: per-trade views, or Bermudans whose exercise indices do not follow their dates.
 template <typename R>
@@ -843,52 +893,11 @@ void planSplit(Batch<R>& B, typename Batch<R>::Launch& L) {
   auto full = [&](const Plan<R>& P) { return P.amcOrProbe || P.im; };
   for (size_t k = 0; k < n; ++k)
     if (B.plans[L.planIdx[nb + k]].nTr > 0) return;
-  // Bermudans: the exercises' dates, and their records date by date as decideKernel reads them.
   std::vector<std::vector<std::vector<uint32_t>>> exDates(n);
   for (size_t k = 0; k < n; ++k) {
     const auto& P = B.plans[L.planIdx[nb + k]];
     if (P.nBerm == 0) continue;
-    const uint32_t* I = P.v.indices;
-    exDates[k].resize(P.nBerm);
-    std::vector<std::vector<R>> prog(P.nBerm);
-    for (uint32_t j = 0; j < nT; ++j) {
-      std::vector<std::vector<const R*>> flows(P.manyBerm ? 1 : P.nBerm);
-      std::vector<const R*> swap;
-      for (uint32_t t = I[j]; t < I[j + 1]; ++t) {
-        const R* r = P.v.terms + static_cast<size_t>(t) * kTermStride;
-        const uint32_t code = static_cast<uint32_t>(r[0]), kind = code & 15u;
-        if (kind == kBermAnnuity || kind == kBermCoterm) swap.push_back(r);
-        if (kind == kBermContinue) swap.clear();
-        if (kind != kBermExercise && kind != kBermDecide) continue;
-        const uint32_t b = bermudanOf(code, P.manyBerm);
-        auto& mine = flows[P.manyBerm ? 0 : b];
-        if (kind == kBermExercise) {
-          mine.push_back(r);
-          continue;
-        }
-        const uint32_t e = code >> 12u;
-        if (e != exDates[k][b].size() || (e > 0 && exDates[k][b].back() >= j)) return;  // not the next exercise
-        exDates[k][b].push_back(j);
-        auto& out = prog[b];
-        auto put = [&](const R* q) {
-          out.insert(out.end(), q, q + kTermStride);
-          out[out.size() - kTermStride] = bitsOfUint<R>(static_cast<uint32_t>(q[0]));
-        };
-        const R mark[kTermStride] = {bitsOfUint<R>(kBond), bitsOfUint<R>(j), R(0), R(0), R(0), R(0), R(0), R(0)};
-        out.insert(out.end(), mark, mark + kTermStride);
-        for (const R* q : mine) put(q);
-        for (const R* q : swap) put(q);
-        put(r);
-        for (uint32_t u = t + 1; u < I[j + 1] && (static_cast<uint32_t>(r[(u - t) * kTermStride]) & 15u) == kBermExt; ++u) put(r + (u - t) * kTermStride);
-        swap.clear();
-        if (P.manyBerm) mine.clear();
-      }
-    }
-    for (uint32_t b = 0; b < P.nBerm; ++b) {
-      const uint32_t at = static_cast<uint32_t>(S.table.size() / 4);
-      S.table.insert(S.table.end(), prog[b].begin(), prog[b].end());
-      S.decides.push_back({static_cast<uint32_t>(k), b, at, static_cast<uint32_t>(S.table.size() / 4)});
-    }
+    if (!exercisePrograms(P, static_cast<uint32_t>(k), exDates[k], S.decides, S.table)) return;
     S.indexBytes += alignUp(static_cast<size_t>(P.nBerm) * nP);
     S.bermsMax = std::max(S.bermsMax, P.nBerm);
   }
@@ -1087,6 +1096,12 @@ std::unique_ptr<Batch<R>> build(zk_context* ctx, std::vector<View<R>> views, boo
   // state pass, not the re-run of chosen paths (its plans run side by side on worker streams).
   if (ctx && !sink && !opts.maps)
     for (auto& L : B->launches) planSplit(*B, L);
+  // The AMC state pass reads the exercises' records alone; x and the deflator stay in the factor cube.
+  if (sink) {
+    auto& S = B->launches[0].split;
+    std::vector<std::vector<uint32_t>> dates;
+    B->sinkPrograms = exercisePrograms(B->plans[0], 0u, dates, S.decides, S.table) && S.decides.size() <= 65535;
+  }
   // ---- arena layout: inputs first (one upload), then device-only scratch, outputs last ----
   size_t off = 0;
   auto take = [&](size_t bytes) { const size_t o = off; off = alignUp(off + std::max<size_t>(bytes, 16)); return o; };
@@ -1122,6 +1137,7 @@ std::unique_ptr<Batch<R>> build(zk_context* ctx, std::vector<View<R>> views, boo
   B->basisArgsOff = take(B->numGroups * sizeof(BasisArgs));
   for (auto& L : B->launches) {
     auto& S = L.split;
+    if (sink && B->sinkPrograms) S.oDecides = take(S.decides.size() * sizeof(DecideJob)), S.oTable = take(S.table.size() * sizeof(R));
     if (!S.on) continue;
     S.oItems = take(S.items.size() * sizeof(ValueItem)), S.oPre = take(S.pre.size() * sizeof(uint2)), S.oFirst = take(S.exFirst.size());
     S.oDecides = take(S.decides.size() * sizeof(DecideJob)), S.oTable = take(S.table.size() * sizeof(R));
@@ -1223,8 +1239,9 @@ std::unique_ptr<Batch<R>> build(zk_context* ctx, std::vector<View<R>> views, boo
   }
   if (sink) {
     const auto& P = B->plans[0];
-    B->sinkOff[0] = take(static_cast<size_t>(P.nT) * P.nP * sizeof(R));
-    B->sinkOff[1] = take(static_cast<size_t>(P.nT) * P.nP * sizeof(R));
+    const size_t field = static_cast<size_t>(P.nT) * P.nP * sizeof(R);
+    if (B->sinkPrograms) B->sinkOff[0] = B->launches[0].cubeOff, B->sinkOff[1] = B->launches[0].cubeOff + field;  // fields 0 and 1
+    else B->sinkOff[0] = take(field), B->sinkOff[1] = take(field);
     B->sinkOff[2] = take(static_cast<size_t>(std::max<uint32_t>(P.exerciseRows, 1)) * P.nP * sizeof(R));
   }
   // The exact-decision check's flags: a bit per path of every checked plan, cleared by each execute.
@@ -1349,6 +1366,9 @@ void fillImage(Batch<R>& B, const double* normals, size_t streams, unsigned char
       std::memcpy(img + S.oItems, S.items.data(), S.items.size() * sizeof(ValueItem));
       if (!S.pre.empty()) std::memcpy(img + S.oPre, S.pre.data(), S.pre.size() * sizeof(uint2));
       if (!S.exFirst.empty()) std::memcpy(img + S.oFirst, S.exFirst.data(), S.exFirst.size());
+    }
+    if (L.split.on || B.sinkPrograms) {
+      const auto& S = L.split;
       if (!S.decides.empty()) std::memcpy(img + S.oDecides, S.decides.data(), S.decides.size() * sizeof(DecideJob));
       if (!S.table.empty()) std::memcpy(img + S.oTable, S.table.data(), S.table.size() * sizeof(R));
     }
@@ -1506,6 +1526,12 @@ void launchRevalues(const Batch<R>& B, const typename Batch<R>::Launch& L, uintp
   }
   if (count == 0) return;
   const auto* ns = reinterpret_cast<const NsArgs<R>*>(base + L.nsOff) + first;
+  if (B.sinkPrograms) {
+    injectPoint(B.ctx);
+    ZK_CUDA(launchExerciseValues<R>(L.cb, ns, reinterpret_cast<const DecideJob*>(base + L.split.oDecides),
+                                    static_cast<uint32_t>(L.split.decides.size()), reinterpret_cast<const R*>(base + L.split.oTable), s));
+    return;
+  }
   if (L.split.on) {  // never in waves: [first, first + count) are the launch's netting sets after its basis groups
     const auto& S = L.split;
     SplitArgs<R> a{};
@@ -1896,10 +1922,15 @@ zk_status runInjected(zk_context* ctx, const ViewT* plan, const double* normals,
   }
 }
 
+// The regressions among items [first, first + count): a step of the chain lists the Bermudans that only update last.
+uint32_t fitsOf(const std::vector<FitItem>& items, uint32_t first, uint32_t count) {
+  while (count > 0 && items[first + count - 1].slot == kNoRow) --count;
+  return count;
+}
+
 // The Longstaff-Schwartz fit of a plan's Bermudans (fitAmc, src/gpu/fused_exposure.cpp:103-156): the AMC
-// state pass of the fused kernel (x, deflator, exercise values on the device), then one thread-block
-// cluster per Bermudan fits the policy of every exercise and the continuation of every date, and the
-// fitted records are written into a copy of the plan's term table.
+// state pass (x, deflator, exercise values on the device), then the regressions of the policy of every exercise and the
+// continuation of every date (amc_fit.cu), and the fitted records are written into a copy of the plan's term table.
 template <typename R, typename ViewT>
 zk_status fitAmc(zk_context* ctx, const ViewT* plan, const double* normals, size_t streams, const uint32_t* degrees,
                  size_t numBermudans, R* termsOut, size_t termsLen) {
@@ -1953,85 +1984,165 @@ zk_status fitAmc(zk_context* ctx, const ViewT* plan, const double* normals, size
           cont[b].push_back({j, t});
         }
       }
-    std::vector<AmcFitJob> jobs(numBermudans);
-    std::vector<uint32_t> contDates;
-    uint32_t slots = 0, eRow = 0;
+    // Slots of the fitted records (exercise k of Bermudan b at slotBase[b] + k, its continuation i at slotBase[b] + nE + i) and
+    // the first exercise row of each Bermudan.
+    std::vector<uint32_t> slotBase(numBermudans), eRow(numBermudans);
+    uint32_t slots = 0, rows = 0, maxE = 1;
+    bool any2 = false;
     for (size_t b = 0; b < numBermudans; ++b) {
       if (degrees[b] > 3) throw fail(ZK_ERR_INVALID_ARGUMENT, "AMC regression degree %u above 3", degrees[b]);
-      AmcFitJob& J = jobs[b];
-      J = AmcFitJob{};
-      J.nP = P.nP, J.nT = P.nT, J.nE = static_cast<uint32_t>(decide[b].size()), J.degree = degrees[b];
-      J.twoD = twoD[b] > 0 ? 1u : 0u;
-      if (J.nE != P.bermRows[b]) throw fail(ZK_ERR_INVALID_PLAN, "Bermudan %zu: inconsistent exercise terms", b);
-      J.eRow = eRow, eRow += J.nE;
-      J.slotBase = slots, slots += J.nE + static_cast<uint32_t>(cont[b].size());
-      for (uint32_t e = 0; e < J.nE; ++e) {
+      const uint32_t nE = static_cast<uint32_t>(decide[b].size());
+      if (nE != P.bermRows[b]) throw fail(ZK_ERR_INVALID_PLAN, "Bermudan %zu: inconsistent exercise terms", b);
+      for (uint32_t e = 0; e < nE; ++e)
         if (decide[b][e].first == 0xFFFFFFFFu || (e > 0 && decide[b][e].second <= decide[b][e - 1].second))
           throw fail(ZK_ERR_INVALID_PLAN, "Bermudan %zu: exercise %u missing or out of order", b, e);
-        J.exDate[e] = decide[b][e].second;
-      }
-      J.contBegin = static_cast<uint32_t>(contDates.size()), J.contCount = static_cast<uint32_t>(cont[b].size());
-      for (const auto& c : cont[b]) contDates.push_back(c.first);
-    }
-    // Per fit slot, the range of its co-terminal bonds (two-regressor Bermudans only).
-    std::vector<uint2> bondRange(std::max<uint32_t>(slots, 1), make_uint2(0, 0));
-    for (size_t b = 0; b < numBermudans; ++b) {
-      const AmcFitJob& J = jobs[b];
-      if (!J.twoD) continue;
-      for (uint32_t e = 0; e < J.nE; ++e) bondRange[J.slotBase + e] = coterm.at(decide[b][e].first);
-      for (uint32_t i = 0; i < J.contCount; ++i) bondRange[J.slotBase + J.nE + i] = coterm.at(cont[b][i].second);
+      eRow[b] = rows, rows += nE;
+      slotBase[b] = slots, slots += nE + static_cast<uint32_t>(cont[b].size());
+      maxE = std::max(maxE, nE);
+      any2 = any2 || twoD[b] > 0;
     }
     std::copy(v.terms, v.terms + termsLen, termsOut);
     if (numBermudans == 0) return ZK_OK;
     upload(*B, ctx, true, normals, streams);
     execute(*B);
-    // Device scratch: jobs, continuation dates, realised values per Bermudan, fitted records, co-terminal bonds and
-    // their ranges.
-    const size_t jobsBytes = jobs.size() * sizeof(AmcFitJob), datesBytes = std::max<size_t>(contDates.size(), 1) * 4;
-    const size_t realisedBytes = numBermudans * static_cast<size_t>(P.nP) * 8, outBytes = static_cast<size_t>(slots) * kFitOut * 8;
-    const size_t bondsBytes = std::max<size_t>(bonds.size(), 1) * sizeof(double4), rangeBytes = bondRange.size() * sizeof(uint2);
-    const size_t o1 = alignUp(jobsBytes), o2 = o1 + alignUp(datesBytes), o3 = o2 + alignUp(realisedBytes);
-    const size_t scratchBytes = bonds.empty() ? 0 : realisedBytes;  // the two-regressor fits' swap rates per path
-    const size_t o4 = o3 + alignUp(outBytes), o5 = o4 + alignUp(bondsBytes), o6 = o5 + alignUp(rangeBytes), total = o6 + scratchBytes;
-    dmem = takeBlock(ctx, total, dmemBytes);
-    if (!dmem) throw fail(ZK_ERR_OUT_OF_MEMORY, "AMC fit: %zu bytes of device memory", total);
-    unsigned char* d = static_cast<unsigned char*>(dmem);
-    ZK_CUDA(cudaMemcpyAsync(d, jobs.data(), jobsBytes, cudaMemcpyHostToDevice, ctx->stream));
-    if (!contDates.empty()) ZK_CUDA(cudaMemcpyAsync(d + o1, contDates.data(), contDates.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-    if (!bonds.empty()) {
-      ZK_CUDA(cudaMemcpyAsync(d + o4, bonds.data(), bonds.size() * sizeof(double4), cudaMemcpyHostToDevice, ctx->stream));
-      ZK_CUDA(cudaMemcpyAsync(d + o5, bondRange.data(), rangeBytes, cudaMemcpyHostToDevice, ctx->stream));
+    // Bermudans in groups whose realised values after each exercise (nE rows each) take at most 2 GB; the continuations'
+    // swap rates (two regressors) at most 512 MB of rows at a time.
+    const size_t rowBytes = static_cast<size_t>(P.nP) * 8;
+    const size_t group = std::max<size_t>(1, std::min<size_t>(numBermudans, (size_t(2) << 30) / (rowBytes * maxE)));
+    const uint32_t contAtOnce = static_cast<uint32_t>(std::max<size_t>(1, std::min<size_t>(any2 ? (size_t(512) << 20) / rowBytes : 65535, 65535)));
+    struct FitLaunch {
+      uint32_t first, count;
+      bool gram, dates;  // dates: items of `shared`
+    };
+    std::vector<FitItem> items;
+    std::vector<FitDate> shared;
+    std::vector<FitLaunch> launches;
+    for (size_t b0 = 0; b0 < numBermudans; b0 += group) {
+      const size_t b1 = std::min(numBermudans, b0 + group);
+      auto realisedRow = [&](size_t b, uint32_t s) { return s == 0 ? kNoRow : static_cast<uint32_t>((b - b0) * maxE + s - 1); };
+      auto swapRow = [&](size_t b, uint32_t s) { return static_cast<uint32_t>((b - b0) * 2 + (s & 1u)); };
+      // The chain, all Bermudans of the group in step: step s fits the policy of exercise nE - 1 - s on the realised values
+      // after the s later ones; one more step leaves those after the first exercise.
+      for (uint32_t s = 0; s <= maxE; ++s) {
+        const uint32_t first = static_cast<uint32_t>(items.size());
+        bool fits = false;
+        for (size_t b = b0; b < b1; ++b) {
+          const uint32_t nE = static_cast<uint32_t>(decide[b].size());
+          if (nE == 0 || s > nE) continue;
+          FitItem I{};
+          const uint32_t k = nE - 1 - s;  // s == nE: only the update
+          const bool fit = s < nE;
+          I.date = fit ? decide[b][k].second : 0u, I.eRow = fit ? eRow[b] + k : kNoRow, I.slot = fit ? slotBase[b] + k : kNoRow;
+          I.degree = degrees[b], I.twoD = twoD[b] > 0 ? 1u : 0u;
+          I.prevSlot = s > 0 ? slotBase[b] + k + 1 : kNoRow, I.prevDate = s > 0 ? decide[b][k + 1].second : 0u;
+          I.prevERow = s > 0 ? eRow[b] + k + 1 : 0u;
+          I.realisedIn = s > 0 ? realisedRow(b, s - 1) : kNoRow, I.realisedOut = realisedRow(b, s);
+          I.swapRow = swapRow(b, s), I.prevSwapRow = swapRow(b, s + 1);
+          if (fit && I.twoD) I.bonds = coterm.at(decide[b][k].first);
+          items.push_back(I);
+          fits = fits || fit;
+        }
+        std::stable_partition(items.begin() + first, items.end(), [](const FitItem& I) { return I.slot != kNoRow; });
+        if (items.size() > first) launches.push_back({first, static_cast<uint32_t>(items.size()) - first, fits, false});
+      }
+      // The continuations: on a date whose next exercise is k the realised values after exercise k's policy.
+      uint32_t first = static_cast<uint32_t>(items.size());
+      const size_t firstDate = shared.size();
+      std::map<std::pair<uint32_t, uint32_t>, size_t> open;  // (date, degree): its item with room
+      for (size_t b = b0; b < b1; ++b) {
+        const uint32_t nE = static_cast<uint32_t>(decide[b].size());
+        for (uint32_t i = 0; i < cont[b].size(); ++i) {
+          const uint32_t jc = cont[b][i].first;
+          uint32_t k = 0;
+          while (k < nE && decide[b][k].second <= jc) ++k;
+          if (k == nE) continue;  // no exercise ahead
+          if (twoD[b] <= 0) {
+            auto [at, fresh] = open.try_emplace({jc, degrees[b]}, shared.size());
+            if (fresh || shared[at->second].count == static_cast<uint32_t>(kFitShared)) {
+              at->second = shared.size();
+              shared.push_back({jc, 0u, degrees[b], 0u, {}, {}});
+            }
+            FitDate& T = shared[at->second];
+            T.slot[T.count] = slotBase[b] + nE + i, T.realisedIn[T.count++] = realisedRow(b, nE - k);
+            continue;
+          }
+          FitItem I{};
+          I.date = jc, I.eRow = kNoRow, I.slot = slotBase[b] + nE + i, I.degree = degrees[b], I.twoD = twoD[b] > 0 ? 1u : 0u;
+          I.realisedIn = realisedRow(b, nE - k), I.realisedOut = kNoRow, I.prevSlot = kNoRow;
+          I.swapRow = static_cast<uint32_t>(2 * group + (items.size() - first));
+          if (I.twoD) I.bonds = coterm.at(cont[b][i].second);
+          items.push_back(I);
+          if (items.size() - first == contAtOnce) {
+            launches.push_back({first, contAtOnce, true, false});
+            first = static_cast<uint32_t>(items.size());
+          }
+        }
+      }
+      if (items.size() > first) launches.push_back({first, static_cast<uint32_t>(items.size()) - first, true, false});
+      for (size_t at = firstDate; at < shared.size(); at += 65535)
+        launches.push_back({static_cast<uint32_t>(at), static_cast<uint32_t>(std::min<size_t>(shared.size() - at, 65535)), true, true});
     }
-    const uint32_t cluster = P.nP >= 65536 ? 8u : P.nP >= 16384 ? 4u : P.nP >= 4096 ? 2u : 1u;
-    const R* sx = reinterpret_cast<const R*>(B->base + B->sinkOff[0]);
-    const R* sd = reinterpret_cast<const R*>(B->base + B->sinkOff[1]);
-    const R* se = reinterpret_cast<const R*>(B->base + B->sinkOff[2]);
-    ZK_CUDA(launchAmcFit<R>(reinterpret_cast<const AmcFitJob*>(d), static_cast<uint32_t>(numBermudans), sx, sd, se,
-                            reinterpret_cast<const uint32_t*>(d + o1),
-                            bonds.empty() ? nullptr : reinterpret_cast<const double4*>(d + o4),
-                            reinterpret_cast<const uint2*>(d + o5), reinterpret_cast<double*>(d + o2),
-                            bonds.empty() ? nullptr : reinterpret_cast<double*>(d + o6), reinterpret_cast<double*>(d + o3),
-                            ctx->dErr, cluster, ctx->stream));
+    // CTAs per regression, at least a path per thread: a step of the chain in about one wave (its CTAs are few and short),
+    // the continuations in two.
+    auto chunksOf = [&](uint32_t count, bool dates) {
+      return std::max(1u, std::min({(P.nP + 255u) / 256u, (148u * (dates ? 8u : 4u) + count - 1) / count, 296u}));
+    };
+    uint32_t maxItems = 1;
+    size_t parts = 1;
+    for (const auto& l : launches) maxItems = std::max(maxItems, l.count), parts = std::max<size_t>(parts, static_cast<size_t>(l.count) * chunksOf(l.count, l.dates));
+    // Device scratch: one image of the items and bonds, then the records, counters, partials, realised values and swap rates.
+    size_t off = 0;
+    auto take = [&](size_t bytes) { const size_t o = off; off = alignUp(off + std::max<size_t>(bytes, 16)); return o; };
+    const size_t oItems = take(items.size() * sizeof(FitItem)), oBonds = take(bonds.size() * sizeof(double4)), oShared = take(shared.size() * sizeof(FitDate));
+    const size_t imageBytes = off;
+    const size_t oFit = take(static_cast<size_t>(slots) * kFitOut * 8), oCount = take(maxItems * 4), zeroEnd = off;
+    const size_t oPart = take(parts * kFitSums * 8), oRealised = take(group * maxE * rowBytes);
+    const size_t oSwap = take(any2 ? (2 * group + std::min<size_t>(contAtOnce, items.size())) * rowBytes : 0);
+    dmem = takeBlock(ctx, off, dmemBytes);
+    if (!dmem) throw fail(ZK_ERR_OUT_OF_MEMORY, "AMC fit: %zu bytes of device memory", off);
+    unsigned char* d = static_cast<unsigned char*>(dmem);
+    std::vector<unsigned char> image(imageBytes, 0);
+    std::memcpy(image.data() + oItems, items.data(), items.size() * sizeof(FitItem));
+    if (!shared.empty()) std::memcpy(image.data() + oShared, shared.data(), shared.size() * sizeof(FitDate));
+    if (!bonds.empty()) std::memcpy(image.data() + oBonds, bonds.data(), bonds.size() * sizeof(double4));
+    ZK_CUDA(cudaMemcpyAsync(d, image.data(), imageBytes, cudaMemcpyHostToDevice, ctx->stream));
+    ZK_CUDA(cudaMemsetAsync(d + oFit, 0, zeroEnd - oFit, ctx->stream));
+    FitData<R> F{};
+    F.x = reinterpret_cast<const R*>(B->base + B->sinkOff[0]), F.D = reinterpret_cast<const R*>(B->base + B->sinkOff[1]);
+    F.E = reinterpret_cast<const R*>(B->base + B->sinkOff[2]);
+    F.bonds = reinterpret_cast<const double4*>(d + oBonds), F.realised = reinterpret_cast<double*>(d + oRealised);
+    F.swap = reinterpret_cast<double*>(d + oSwap), F.fit = reinterpret_cast<double*>(d + oFit);
+    F.part = reinterpret_cast<double*>(d + oPart), F.counter = reinterpret_cast<uint32_t*>(d + oCount), F.err = ctx->dErr, F.nP = P.nP;
+    for (const auto& l : launches) {
+      if (l.dates) {
+        ZK_CUDA(launchFitDates<R>(reinterpret_cast<const FitDate*>(d + oShared) + l.first, l.count, chunksOf(l.count, true), F, ctx->stream));
+        continue;
+      }
+      const FitItem* at = reinterpret_cast<const FitItem*>(d + oItems) + l.first;
+      ZK_CUDA(launchFit<R>(at, l.count, chunksOf(l.count, false), false, any2, F, ctx->stream));
+      if (l.gram) ZK_CUDA(launchFit<R>(at, fitsOf(items, l.first, l.count), chunksOf(l.count, false), true, any2, F, ctx->stream));
+    }
     std::vector<double> fitted(static_cast<size_t>(slots) * kFitOut);
-    uint32_t devErr = 0;
-    ZK_CUDA(cudaMemcpyAsync(fitted.data(), d + o3, outBytes, cudaMemcpyDeviceToHost, ctx->stream));
-    ZK_CUDA(cudaMemcpyAsync(&devErr, ctx->dErr, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    ZK_CUDA(cudaMemcpyAsync(fitted.data(), d + oFit, fitted.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    ZK_CUDA(cudaMemcpyAsync(ctx->hErr, ctx->dErr, 4, cudaMemcpyDeviceToHost, ctx->stream));
     ZK_CUDA(cudaStreamSynchronize(ctx->stream));
+    const uint32_t devErr = *ctx->hErr;
     giveBlock(ctx, static_cast<unsigned char*>(dmem), dmemBytes);
     dmem = nullptr;
     if (devErr != 0) throw fail(ZK_ERR_CUDA, "the AMC fit reported error %u (normal equations not positive definite)", devErr);
     // The records as the reference writes them: center, 1 / scale, c0..c3 (fused_exposure.cpp:118-123).
     // Two-regressor records: cx, 1 / sx, cs, 1 / ss, c0, c1 in the record, c2..c8 in the first extension record's
     // fields 1..7 and c9 in the second's field 1 (the kernel's amcPoly2 reads them so).
+    auto inverse = [](double scale) { return scale != 0.0 ? 1.0 / scale : 1.0; };  // 0: a record with no exercise ahead, not fitted
     auto write = [&](uint32_t term, const double* f, bool two) {
       R* r = termsOut + static_cast<size_t>(term) * kTermStride;
       if (!two) {
         r[2] = static_cast<R>(f[0]);
-        r[3] = static_cast<R>(1.0 / f[1]);
+        r[3] = static_cast<R>(inverse(f[1]));
         for (int i = 0; i < 4; ++i) r[4 + i] = static_cast<R>(f[2 + i]);
         return;
       }
-      r[2] = static_cast<R>(f[0]), r[3] = static_cast<R>(1.0 / f[1]), r[4] = static_cast<R>(f[2]), r[5] = static_cast<R>(1.0 / f[3]);
+      r[2] = static_cast<R>(f[0]), r[3] = static_cast<R>(inverse(f[1])), r[4] = static_cast<R>(f[2]), r[5] = static_cast<R>(inverse(f[3]));
       r[6] = static_cast<R>(f[4]), r[7] = static_cast<R>(f[5]);
       R* e1 = r + kTermStride;
       R* e2 = r + 2 * kTermStride;
@@ -2039,9 +2150,9 @@ zk_status fitAmc(zk_context* ctx, const ViewT* plan, const double* normals, size
       e2[1] = static_cast<R>(f[13]);
     };
     for (size_t b = 0; b < numBermudans; ++b) {
-      const AmcFitJob& J = jobs[b];
-      for (uint32_t e = 0; e < J.nE; ++e) write(decide[b][e].first, &fitted[(J.slotBase + e) * kFitOut], J.twoD != 0);
-      for (uint32_t i = 0; i < J.contCount; ++i) write(cont[b][i].second, &fitted[(J.slotBase + J.nE + i) * kFitOut], J.twoD != 0);
+      const size_t nE = decide[b].size();
+      for (size_t e = 0; e < nE; ++e) write(decide[b][e].first, &fitted[(slotBase[b] + e) * kFitOut], twoD[b] > 0);
+      for (size_t i = 0; i < cont[b].size(); ++i) write(cont[b][i].second, &fitted[(slotBase[b] + nE + i) * kFitOut], twoD[b] > 0);
     }
     return ZK_OK;
   } catch (const Failure& f) {

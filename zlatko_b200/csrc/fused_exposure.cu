@@ -1002,7 +1002,8 @@ __global__ void __launch_bounds__(kTile, (revalueMinBlocks<PPT, kLean, kSmallSta
 // Revaluation before and after (us): 2,000 paths x 121 dates of 3 trades 146 and 20, 10,000 x 61 of 20 swaps 203 and 31, 12
 // netting sets of 119 trades at 33,333 paths x 169 dates 1,497 and 1,077, 24 + 24 netting sets with 40
 // Bermudans among 800 trades at 65,536 x 241 66,061 and 28,457.
-template <typename R>
+// kSink: the AMC state pass, which keeps the exercise values (A.sinkEx) instead of deciding on them.
+template <typename R, bool kSink>
 __global__ void __launch_bounds__(kTile) decideKernel(const CubeArgs<R> cb, const NsArgs<R>* __restrict__ nsArgs,
                                                       const DecideJob* __restrict__ jobs, const R* __restrict__ table) {
   const DecideJob J = jobs[blockIdx.y];
@@ -1023,6 +1024,11 @@ __global__ void __launch_bounds__(kTile) decideKernel(const CubeArgs<R> cb, cons
       continue;
     }
     if (kind == kBermDecide) {
+      if constexpr (kSink) {
+        A.sinkEx[static_cast<size_t>(A.sinkRowOfBermudan[J.berm] + (code >> 12u)) * nP + p] = ev;
+        if (many) ev = R(0);
+        continue;
+      }
       R e1[8], e2[8];
       const bool twoD = twoRegressors(table, u, J.end, e1, e2);
       const R cont = twoD ? amcPoly2(rec, e1, e2, x, swapRate(flt, ann)) : amcPoly(rec, x);
@@ -1039,6 +1045,7 @@ __global__ void __launch_bounds__(kTile) decideKernel(const CubeArgs<R> cb, cons
       else flt += v;
     }
   }
+  if constexpr (kSink) return;
   A.exIndex[static_cast<size_t>(J.berm) * nP + p] = static_cast<signed char>(ex);
   if (A.rowEx != kNoRow && (many || J.berm < 4u)) A.expo[(A.rowEx + J.berm) * static_cast<size_t>(nP) + p] = ex;
 }
@@ -1654,7 +1661,7 @@ cudaError_t launchSplit(const CubeArgs<R>& cb, const NsArgs<R>* nsArgs, uint32_t
   if (numNs == 0 || sp.numItems == 0) return cudaSuccess;
   if (numNs > 65535u || sp.numItems > 65535u || sp.numDecides > 65535u) return cudaErrorInvalidConfiguration;
   if (sp.numDecides > 0) {
-    decideKernel<R><<<dim3((cb.nP + kTile - 1) / kTile, sp.numDecides), kTile, 0, stream>>>(cb, nsArgs, sp.decides, sp.decideTable);
+    decideKernel<R, false><<<dim3((cb.nP + kTile - 1) / kTile, sp.numDecides), kTile, 0, stream>>>(cb, nsArgs, sp.decides, sp.decideTable);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -1684,6 +1691,18 @@ cudaError_t launchSplit(const CubeArgs<R>& cb, const NsArgs<R>* nsArgs, uint32_t
   }
   return cudaSuccess;
 }
+template <typename R>
+cudaError_t launchExerciseValues(const CubeArgs<R>& cb, const NsArgs<R>* nsArgs, const DecideJob* jobs, uint32_t numJobs, const R* table,
+                                 cudaStream_t stream) {
+  if (numJobs == 0) return cudaSuccess;
+  if (numJobs > 65535u) return cudaErrorInvalidConfiguration;
+  decideKernel<R, true><<<dim3((cb.nP + kTile - 1) / kTile, numJobs), kTile, 0, stream>>>(cb, nsArgs, jobs, table);
+  return cudaGetLastError();
+}
+template cudaError_t launchExerciseValues<float>(const CubeArgs<float>&, const NsArgs<float>*, const DecideJob*, uint32_t, const float*,
+                                                 cudaStream_t);
+template cudaError_t launchExerciseValues<double>(const CubeArgs<double>&, const NsArgs<double>*, const DecideJob*, uint32_t, const double*,
+                                                  cudaStream_t);
 template cudaError_t launchSplit<float>(const CubeArgs<float>&, const NsArgs<float>*, uint32_t, const SplitArgs<float>&, cudaStream_t);
 template cudaError_t launchSplit<double>(const CubeArgs<double>&, const NsArgs<double>*, uint32_t, const SplitArgs<double>&, cudaStream_t);
 template cudaError_t launchNestedIm<float>(const ImArgs<float>&, cudaStream_t);

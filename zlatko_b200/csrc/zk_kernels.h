@@ -124,25 +124,52 @@ cudaError_t launchRowStats(const RowJob<R>* jobs, uint32_t numJobs, uint32_t* er
 cudaError_t launchScatterRows(const double* src, uint32_t m, const uint32_t* map, uint32_t rows, float* dst, uint32_t nP,
                               cudaStream_t stream);
 
-// One Bermudan of the AMC fit (zk_fit_amc): its exercise dates (grid indices, ascending), its first row of
-// exercise values in the AMC pass, the slots of its fitted records (slotBase + k: policy of exercise k;
-// slotBase + nE + i: continuation on date contDates[contBegin + i]) and its regression degree.
+// One regression of the AMC fit (zk_fit_amc).  Rows of `realised` and `swap` are nP doubles.
 constexpr int kMaxExercises = 64;
-struct AmcFitJob {
-  uint32_t nP, nT, nE, degree, eRow, slotBase, contBegin, contCount;
-  uint32_t twoD, pad;  // twoD: the Bermudan's records use the two-regressor basis
-  uint32_t exDate[kMaxExercises];
+constexpr int kFitOut = 16;   // doubles per fitted slot: 1D center, scale, c0..c3; 2D cx, sx, cs, ss, c0..c9; last the degree
+constexpr int kFitSums = 38;  // doubles of a CTA's partial
+struct FitItem {
+  uint32_t date, eRow;       // its date; the row of exercise values whose positive entries it includes (kNoRow: every path)
+  uint32_t slot, degree;     // its record (kNoRow: only the update below)
+  uint32_t realisedIn;       // row of realised values read (kNoRow: zeros)
+  uint32_t realisedOut;      // with prevSlot: the row of the realised values after that policy
+  uint32_t prevSlot, prevDate, prevERow;  // the policy applied first (kNoRow: none), its date and exercise row
+  uint32_t twoD, swapRow, prevSwapRow;    // the two-regressor basis: its row of swap rates and the previous policy's
+  uint2 bonds;               // two regressors: the range of its co-terminal swap's bonds
+  uint32_t pad[2];
 };
-// The two-regressor basis: per fit slot (exercise k at slotBase + k, continuation i at slotBase + nE + i) the range
-// [bondRange.x, + bondRange.y) of its co-terminal swap's bonds {kind (annuity 13 / float leg 14), c, A, B}; the
-// regressor s = sum_float c A e^{-B x} / sum_annuity c A e^{-B x}, as the fused kernel forms it.
-constexpr int kFitOut = 16;  // doubles per fitted slot: 1D center, scale, c0..c3; 2D cx, sx, cs, ss, c0..c9
-// One thread-block cluster of clusterSize CTAs per job; out[slot][kFitOut]; realised and, with bonds, swapScratch:
-// [numJobs][nP] doubles of scratch.
+// The continuation regressions of one date and degree for up to kFitShared Bermudans of the one-regressor basis.
+constexpr int kFitShared = 4;
+struct FitDate {
+  uint32_t date, count, degree, pad;
+  uint32_t slot[kFitShared], realisedIn[kFitShared];
+};
+// What the regressions read.  bonds {kind (annuity 13 / float leg 14), c, A, B}: the regressor s = sum_float c A e^{-B x} /
+// sum_annuity c A e^{-B x}, as the fused kernel forms it.  part: [items][chunks][kFitSums]; counter: [items], zero.
 template <typename R>
-cudaError_t launchAmcFit(const AmcFitJob* jobs, uint32_t numJobs, const R* x, const R* D, const R* E, const uint32_t* contDates,
-                         const double4* bonds, const uint2* bondRange, double* realised, double* swapScratch, double* out,
-                         uint32_t* err, uint32_t clusterSize, cudaStream_t stream);
+struct FitData {
+  const R* x;  // [date][nP]
+  const R* D;
+  const R* E;  // [exercise row][nP]
+  const double4* bonds;
+  double* realised;
+  double* swap;
+  double* fit;  // [slot][kFitOut]
+  double* part;
+  uint32_t* counter;
+  uint32_t* err;
+  uint32_t nP;
+};
+// The first pass (gram = false) or the second of numItems regressions, each over `chunks` CTAs.
+template <typename R>
+cudaError_t launchFit(const FitItem* items, uint32_t numItems, uint32_t chunks, bool gram, bool twoD, const FitData<R>& F, cudaStream_t stream);
+// Both passes of the dates' regressions.
+template <typename R>
+cudaError_t launchFitDates(const FitDate* items, uint32_t numItems, uint32_t chunks, const FitData<R>& F, cudaStream_t stream);
+// The exercise values of every Bermudan exercise [row][path] (the AMC state pass; A.sinkEx) from the decide programs.
+template <typename R>
+cudaError_t launchExerciseValues(const CubeArgs<R>& cb, const NsArgs<R>* nsArgs, const DecideJob* jobs, uint32_t numJobs, const R* table,
+                                 cudaStream_t stream);
 
 // C = A B^T with A [M][K], B [N][K] bf16 row-major (K contiguous) and FP32 accumulation on the tensor cores
 // (mlp.cu); M % 128 == 0, N % 16 == 0, K % 16 == 0.  Epilogue: z = acc + bias[n], times silu'(gradOf[m][n])
