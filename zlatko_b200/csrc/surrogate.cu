@@ -18,16 +18,36 @@ namespace zk {
 
 namespace {
 
+// Parts of a batch in the weight gradients (three layers: 144 CTAs), up to kGradRows rows.  The tensor core's FP32 accumulation
+// over one chain and over parts differ by about 1e-9 of the gradient's norm per row (9e-6 at 8,192 rows, 1.5e-5 at 12,288); larger batches keep the
+// one chain, and with it their results (131,072 rows: 29.3 ms before, 4.4 now).
+constexpr uint32_t kGradParts = 48, kGradRows = 9216;
+
+// A row of 128 bf16 as 16-byte loads, f(j, value) in order.
+template <typename F>
+__device__ __forceinline__ void forRow(const bf16* h, F&& f) {
+#pragma unroll 4
+  for (uint32_t q = 0; q < kHid / 8; ++q) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(h) + q);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e)
+      f(8 * q + 2 * e, __uint_as_float(w[e] << 16)), f(8 * q + 2 * e + 1, __uint_as_float(w[e] & 0xFFFF0000u));
+  }
+}
+
 // Row pass of the head: pred = h3 . w4 + b4 (standardised units); with targets, dOut = 2 (pred - y) / n and the
 // block's sum of squared errors.  Rows >= n are padding and contribute nothing.
 __global__ void headKernel(const bf16* __restrict__ H3, const float* __restrict__ w4, const float* __restrict__ b4,
                            const float* __restrict__ y, uint32_t n, float* __restrict__ pred, float* __restrict__ dOut,
                            float* __restrict__ lossPart) {
   __shared__ float red[128];
+  __shared__ float w[kHid];
+  w[threadIdx.x] = w4[threadIdx.x];
+  __syncthreads();
   const uint32_t r = blockIdx.x * 128 + threadIdx.x;
-  const bf16* h = H3 + static_cast<size_t>(r) * kHid;
   float p = 0.0f, l = 0.0f;
-  for (uint32_t j = 0; j < kHid; ++j) p += __bfloat162float(h[j]) * w4[j];
+  forRow(H3 + static_cast<size_t>(r) * kHid, [&](uint32_t j, float h) { p += h * w[j]; });
   p += b4[0];
   if (pred) pred[r] = p;
   if (dOut) {
@@ -47,42 +67,63 @@ __global__ void headKernel(const bf16* __restrict__ H3, const float* __restrict_
 }
 
 // Column pass of the head on a block of 128 rows: the block's partial dw4 and db4, and
-// dZ3 = dOut w4 silu'(Z3) row-major and transposed.
-__global__ void headBackKernel(const bf16* __restrict__ H3, const bf16* __restrict__ Z3, const float* __restrict__ w4,
-                               const float* __restrict__ dOut, uint32_t rows, float* __restrict__ part,
-                               bf16* __restrict__ dZ3, bf16* __restrict__ dZ3T) {
+// dZ3 = dOut w4 silu'(Z3) row-major and transposed.  Thread (j, half) takes column j of 64 rows, the transposed copy
+// leaving 8 rows (16 bytes) at a time.
+__global__ void __launch_bounds__(256) headBackKernel(const bf16* __restrict__ H3, const bf16* __restrict__ Z3, const float* __restrict__ w4,
+                                                      const float* __restrict__ dOut, uint32_t rows, float* __restrict__ part,
+                                                      bf16* __restrict__ dZ3, bf16* __restrict__ dZ3T) {
   __shared__ float d[128];
-  const uint32_t r0 = blockIdx.x * 128, j = threadIdx.x;
-  d[j] = dOut[r0 + j];
+  __shared__ float half[kHid + 1];
+  const uint32_t r0 = blockIdx.x * 128, j = threadIdx.x & 127u, up = threadIdx.x >> 7;
+  if (up == 0) d[j] = dOut[r0 + j];
   __syncthreads();
   float gw = 0.0f, gb = 0.0f;
-  for (uint32_t i = 0; i < 128; ++i) {
-    const size_t at = static_cast<size_t>(r0 + i) * kHid + j;
-    gw += d[i] * __bfloat162float(H3[at]);
-    gb += d[i];
-    const bf16 v = __float2bfloat16_rn(d[i] * w4[j] * umma::siluGrad(__bfloat162float(Z3[at])));
-    dZ3[at] = v;
-    dZ3T[static_cast<size_t>(j) * rows + r0 + i] = v;
+  const float w = w4[j];
+  for (uint32_t i0 = 64 * up; i0 < 64 * up + 64; i0 += 8) {
+    bf16 h[8], z[8];
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q) {
+      const size_t at = static_cast<size_t>(r0 + i0 + q) * kHid + j;
+      h[q] = H3[at], z[q] = Z3[at];
+    }
+    __align__(16) bf16 out[8];
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q) {
+      gw += d[i0 + q] * __bfloat162float(h[q]);
+      gb += d[i0 + q];
+      out[q] = __float2bfloat16_rn(d[i0 + q] * w * umma::siluGrad(__bfloat162float(z[q])));
+      dZ3[static_cast<size_t>(r0 + i0 + q) * kHid + j] = out[q];
+    }
+    *reinterpret_cast<uint4*>(dZ3T + static_cast<size_t>(j) * rows + r0 + i0) = *reinterpret_cast<const uint4*>(out);
   }
-  part[static_cast<size_t>(blockIdx.x) * (kHid + 1) + j] = gw;
-  if (j == 0) part[static_cast<size_t>(blockIdx.x) * (kHid + 1) + kHid] = gb;
+  if (up == 1) {
+    half[j] = gw;
+    if (j == 0) half[kHid] = gb;
+  }
+  __syncthreads();
+  if (up == 1) return;
+  part[static_cast<size_t>(blockIdx.x) * (kHid + 1) + j] = gw + half[j];
+  if (j == 0) part[static_cast<size_t>(blockIdx.x) * (kHid + 1) + kHid] = gb + half[kHid];
 }
 
-// out[c] = sum over blocks b of part[b][c], in block order (deterministic).
-__global__ void sumRowsKernel(const float* __restrict__ part, uint32_t blocks, uint32_t w, float* __restrict__ out) {
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= w) return;
-  float s = 0.0f;
-  for (uint32_t b = 0; b < blocks; ++b) s += part[static_cast<size_t>(b) * w + c];
-  out[c] = s;
-}
-
-// Column sums of a bf16 [rows][128] matrix (the bias gradients), in row order.
-__global__ void colSumKernel(const bf16* __restrict__ M, uint32_t rows, float* __restrict__ out) {
-  const uint32_t j = threadIdx.x;
-  float s = 0.0f;
-  for (uint32_t r = 0; r < rows; ++r) s += __bfloat162float(M[static_cast<size_t>(r) * kHid + j]);
-  out[j] = s;
+// The head's gradient out[c] = sum over blocks b of part[b][c] (w columns) and the batch's squared errors added to *loss.  One
+// CTA per 8 columns, 32 lanes over the blocks, then a fixed tree (deterministic).
+__global__ void __launch_bounds__(256) sumRowsKernel(const float* __restrict__ part, uint32_t blocks, uint32_t w, float* __restrict__ out,
+                                                     const float* __restrict__ lossPart, double* __restrict__ loss) {
+  const uint32_t lane = threadIdx.x & 31u, c = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (c < w) {
+    float s = 0.0f;
+    for (uint32_t b = lane; b < blocks; b += 32) s += __ldg(part + static_cast<size_t>(b) * w + c);
+#pragma unroll
+    for (uint32_t o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+    if (lane == 0) out[c] = s;
+  } else if (c == w) {
+    double s = 0.0;
+    for (uint32_t b = lane; b < blocks; b += 32) s += static_cast<double>(__ldg(lossPart + b));
+#pragma unroll
+    for (uint32_t o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+    if (lane == 0) *loss += s;
+  }
 }
 
 // Adam on one parameter block [outDim][inDim] (or a vector); refreshes the bf16 copies of matrices.
@@ -155,15 +196,17 @@ cudaError_t ensureWorkspace(SurrogateState& S, uint32_t rows) {
   S.cap = 0;
   const size_t r = rows, bh = r * kHid * 2, bi = r * kIn * 2;
   const size_t sizes[] = {bi, bi, bh, bh, bh, bh, bh, bh, bh, bh, bh, bh, bh, bh, bh, bh,
-                          r * 4, r * 4, r * 4, (r / 128 + 1) * (kHid + 1) * 4, (r / 128 + 1) * 4};
+                          r * 4, r * 4, r * 4, (r / 128 + 1) * (kHid + 1) * 4, (r / 128 + 1) * 4,
+                          kGradParts * (SurrogateState::kParams + 3) * size_t(4), 8};
   constexpr size_t nb = sizeof(sizes) / sizeof(sizes[0]);
   size_t off[nb], total = 0;
   for (size_t i = 0; i < nb; ++i) off[i] = total, total += (sizes[i] + 255) / 256 * 256;
   SG_CUDA(cudaMalloc(&S.ws, total));
   bf16** bp[] = {&S.X, &S.XT, &S.Z1, &S.H1, &S.H1T, &S.Z2, &S.H2, &S.H2T, &S.Z3, &S.H3, &S.dZ3, &S.dZ3T, &S.dZ2, &S.dZ2T, &S.dZ1, &S.dZ1T};
   for (size_t i = 0; i < 16; ++i) *bp[i] = reinterpret_cast<bf16*>(S.ws + off[i]);
-  float** fp[] = {&S.ys, &S.pred, &S.dOut, &S.part, &S.lossPart};
-  for (size_t i = 0; i < 5; ++i) *fp[i] = reinterpret_cast<float*>(S.ws + off[16 + i]);
+  float** fp[] = {&S.ys, &S.pred, &S.dOut, &S.part, &S.lossPart, &S.gradPart};
+  S.loss = reinterpret_cast<double*>(S.ws + off[22]);
+  for (size_t i = 0; i < 6; ++i) *fp[i] = reinterpret_cast<float*>(S.ws + off[16 + i]);
   S.cap = rows;
   return cudaSuccess;
 }
@@ -175,19 +218,17 @@ GemmArgs gemm(const bf16* A, const bf16* B, uint32_t M, uint32_t N, uint32_t K, 
 }
 
 // Forward pass of `rows` (a multiple of 128) standardised rows in S.X: Z and H of the three hidden layers
-// (and the transposed H1, H2 that the weight gradients read, when training).
-// headOut (inference): the last layer's epilogue evaluates the linear head into it and H3 is not written.
-cudaError_t forward(SurrogateState& S, uint32_t rows, bool training, float* headOut = nullptr) {
+// (and the transposed H1, H2 that the weight gradients read).
+cudaError_t forward(SurrogateState& S, uint32_t rows) {
   const cudaStream_t s = S.stream;
   GemmArgs g = gemm(S.X, S.wb, rows, kHid, kIn, S.err);
-  g.bias = S.b1(), g.act = 1, g.Z = training ? S.Z1 : nullptr, g.H = S.H1, g.HT = training ? S.H1T : nullptr;  // Z: backward only
+  g.bias = S.b1(), g.act = 1, g.Z = S.Z1, g.H = S.H1, g.HT = S.H1T;
   SG_CUDA(launchGemm(g, s));
   g = gemm(S.H1, S.wb + SurrogateState::kW1, rows, kHid, kHid, S.err);
-  g.bias = S.b2(), g.act = 1, g.Z = training ? S.Z2 : nullptr, g.H = S.H2, g.HT = training ? S.H2T : nullptr;
+  g.bias = S.b2(), g.act = 1, g.Z = S.Z2, g.H = S.H2, g.HT = S.H2T;
   SG_CUDA(launchGemm(g, s));
   g = gemm(S.H2, S.wb + SurrogateState::kW1 + SurrogateState::kW2, rows, kHid, kHid, S.err);
-  g.bias = S.b3(), g.act = 1, g.Z = training ? S.Z3 : nullptr, g.H = headOut ? nullptr : S.H3;
-  if (headOut) g.headW = S.w4(), g.headB = S.b4(), g.headOut = headOut;
+  g.bias = S.b3(), g.act = 1, g.Z = S.Z3, g.H = S.H3;
   SG_CUDA(launchGemm(g, s));
   return cudaSuccess;
 }
@@ -197,30 +238,23 @@ cudaError_t backward(SurrogateState& S, uint32_t n, uint32_t rows) {
   const cudaStream_t s = S.stream;
   const uint32_t blocks = rows / 128;
   headKernel<<<blocks, 128, 0, s>>>(S.H3, S.w4(), S.b4(), S.ys, n, S.pred, S.dOut, S.lossPart);
-  headBackKernel<<<blocks, 128, 0, s>>>(S.H3, S.Z3, S.w4(), S.dOut, rows, S.part, S.dZ3, S.dZ3T);
-  sumRowsKernel<<<2, 128, 0, s>>>(S.part, blocks, kHid + 1, S.grad + S.offOf(S.w4()));
-  // dW3 = dZ3^T H2, db3, dZ2 = (dZ3 W3) silu'(Z2)
-  GemmArgs g = gemm(S.dZ3T, S.H2T, kHid, kHid, rows, S.err);
-  g.C = S.grad + S.offOf(S.W3());
-  SG_CUDA(launchGemm(g, s));
-  colSumKernel<<<1, kHid, 0, s>>>(S.dZ3, rows, S.grad + S.offOf(S.b3()));
-  g = gemm(S.dZ3, S.wbT + SurrogateState::kW1 + SurrogateState::kW2, rows, kHid, kHid, S.err);
+  headBackKernel<<<blocks, 256, 0, s>>>(S.H3, S.Z3, S.w4(), S.dOut, rows, S.part, S.dZ3, S.dZ3T);
+  sumRowsKernel<<<(kHid + 2 + 7) / 8, 256, 0, s>>>(S.part, blocks, kHid + 1, S.grad + S.offOf(S.w4()), S.lossPart, S.loss);
+  // dZ2 = (dZ3 W3) silu'(Z2), dZ1 = (dZ2 W2) silu'(Z1); then every layer's dW = dZ^T H and db in one launch
+  GemmArgs g = gemm(S.dZ3, S.wbT + SurrogateState::kW1 + SurrogateState::kW2, rows, kHid, kHid, S.err);
   g.gradOf = S.Z2, g.H = S.dZ2, g.HT = S.dZ2T;
   SG_CUDA(launchGemm(g, s));
-  // dW2 = dZ2^T H1, db2, dZ1 = (dZ2 W2) silu'(Z1)
-  g = gemm(S.dZ2T, S.H1T, kHid, kHid, rows, S.err);
-  g.C = S.grad + S.offOf(S.W2());
-  SG_CUDA(launchGemm(g, s));
-  colSumKernel<<<1, kHid, 0, s>>>(S.dZ2, rows, S.grad + S.offOf(S.b2()));
   g = gemm(S.dZ2, S.wbT + SurrogateState::kW1, rows, kHid, kHid, S.err);
   g.gradOf = S.Z1, g.H = S.dZ1, g.HT = S.dZ1T;
   SG_CUDA(launchGemm(g, s));
-  // dW1 = dZ1^T X, db1
-  g = gemm(S.dZ1T, S.XT, kHid, kIn, rows, S.err);
-  g.C = S.grad + S.offOf(S.W1());
-  SG_CUDA(launchGemm(g, s));
-  colSumKernel<<<1, kHid, 0, s>>>(S.dZ1, rows, S.grad + S.offOf(S.b1()));
-  return cudaGetLastError();
+  WeightGradArgs w{};
+  auto off = [&](const float* q) { return static_cast<uint32_t>(S.offOf(q)); };
+  w.layer[0] = {S.dZ3T, S.H2T, kHid, off(S.W3()), off(S.b3()), 0};
+  w.layer[1] = {S.dZ2T, S.H1T, kHid, off(S.W2()), off(S.b2()), 0};
+  w.layer[2] = {S.dZ1T, S.XT, kIn, off(S.W1()), off(S.b1()), 0};
+  w.rows = rows, w.perPart = rows <= kGradRows ? (blocks + kGradParts - 1) / kGradParts * 128 : rows, w.partStride = SurrogateState::kParams + 3;
+  w.part = S.gradPart, w.err = S.err;
+  return launchWeightGrads(w, (rows + w.perPart - 1) / w.perPart, S.grad, off(S.w4()), s);
 }
 
 cudaError_t adam(SurrogateState& S, float lr, float decay) {
@@ -325,19 +359,18 @@ cudaError_t surrogateEpoch(SurrogateState& S, const float* dx, const float* dy, 
                            bool train, double* loss) {
   const uint32_t rowsCap = (batch + 127) / 128 * 128;
   SG_CUDA(ensureWorkspace(S, rowsCap));
-  double total = 0.0;
-  std::vector<float> lp(rowsCap / 128);
+  SG_CUDA(cudaMemsetAsync(S.loss, 0, 8, S.stream));
   for (size_t b0 = 0; b0 < n; b0 += batch) {
     const uint32_t nb = static_cast<uint32_t>(std::min<size_t>(batch, n - b0)), rows = (nb + 127) / 128 * 128;
     prepareKernel<<<blocksOf(rows, 128), 128, 0, S.stream>>>(dx + b0 * kIn, dy + b0, nb, rows, S.scale, S.scale + 16, S.yMean,
                                                               1.0f / S.yScale, S.X, S.XT, S.ys);
-    SG_CUDA(forward(S, rows, true));
+    SG_CUDA(forward(S, rows));
     SG_CUDA(backward(S, nb, rows));
     if (train) SG_CUDA(adam(S, lr, decay));
-    SG_CUDA(cudaMemcpyAsync(lp.data(), S.lossPart, rows / 128 * 4, cudaMemcpyDeviceToHost, S.stream));
-    SG_CUDA(cudaStreamSynchronize(S.stream));
-    for (uint32_t i = 0; i < rows / 128; ++i) total += lp[i];
   }
+  double total = 0.0;
+  SG_CUDA(cudaMemcpyAsync(&total, S.loss, 8, cudaMemcpyDeviceToHost, S.stream));
+  SG_CUDA(cudaStreamSynchronize(S.stream));
   if (loss) *loss = total / static_cast<double>(n > 0 ? n : 1);
   return cudaSuccess;
 }
@@ -383,7 +416,7 @@ __device__ __forceinline__ bool groupAnd(bool v, uint32_t g) {
 // columns, activation tile and mbarrier, so four tiles' epilogues keep the SM busy.  Per tile, layer l is one
 // chain of K/16 MMAs (the same products, in the same order, as the layer-by-layer GEMMs), and its epilogue
 // (bias, SiLU, BF16) writes the activations straight into the next layer's A tile in shared memory; the last
-// epilogue evaluates the linear head as gemmKernel's fused head does.  The next tile's inputs load while the
+// epilogue evaluates the linear head, a row's columns in order.  The next tile's inputs load while the
 // tile's layers run.
 __global__ void __launch_bounds__(kMlpThreads, 1) mlpInferKernel(const bf16* __restrict__ X, const bf16* __restrict__ wb,
                                                                  const float* __restrict__ b1, const float* __restrict__ b2,

@@ -36,7 +36,8 @@ struct SurrogateState {
   unsigned char* ws = nullptr;
   bf16 *X = nullptr, *XT = nullptr, *Z1 = nullptr, *H1 = nullptr, *H1T = nullptr, *Z2 = nullptr, *H2 = nullptr, *H2T = nullptr;
   bf16 *Z3 = nullptr, *H3 = nullptr, *dZ3 = nullptr, *dZ3T = nullptr, *dZ2 = nullptr, *dZ2T = nullptr, *dZ1 = nullptr, *dZ1T = nullptr;
-  float *ys = nullptr, *pred = nullptr, *dOut = nullptr, *part = nullptr, *lossPart = nullptr;
+  float *ys = nullptr, *pred = nullptr, *dOut = nullptr, *part = nullptr, *lossPart = nullptr, *gradPart = nullptr;
+  double* loss = nullptr;  // the squared errors of an epoch so far
 
   float* W1() const { return p; }
   float* b1() const { return p + kW1; }

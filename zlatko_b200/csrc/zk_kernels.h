@@ -173,7 +173,7 @@ cudaError_t launchExerciseValues(const CubeArgs<R>& cb, const NsArgs<R>* nsArgs,
 
 // C = A B^T with A [M][K], B [N][K] bf16 row-major (K contiguous) and FP32 accumulation on the tensor cores
 // (mlp.cu); M % 128 == 0, N % 16 == 0, K % 16 == 0.  Epilogue: z = acc + bias[n], times silu'(gradOf[m][n])
-// when gradOf is given (back-propagation through a SiLU); C (fp32, or C += z when accumulate), Z = bf16(z),
+// when gradOf is given (back-propagation through a SiLU); C (fp32), Z = bf16(z),
 // H = bf16(act(z)) row-major, HT = bf16(act(z)) transposed [N][M]; any may be null.
 struct GemmArgs {
   const __nv_bfloat16* A;
@@ -186,14 +186,24 @@ struct GemmArgs {
   __nv_bfloat16* HT;
   const __nv_bfloat16* gradOf;  // [M][N] pre-activations of the SiLU being back-propagated, or null
   uint32_t act;         // 0 identity, 1 SiLU
-  uint32_t accumulate;
   uint32_t* err;
-  // Fused linear head (N = 128, one column tile): headOut[row] = sum_n bf16(h[row][n]) headW[n] + headB[0],
-  // summed over n in order; or null.
-  const float* headW;
-  const float* headB;
-  float* headOut;
 };
 cudaError_t launchGemm(const GemmArgs& g, cudaStream_t stream);
+
+// The gradients of the hidden layers' weights and biases from a batch of `rows` (a multiple of 128): per layer dZ^T [128][rows]
+// and the layer's inputs H^T [N][rows] (N = 128 or 16), into out[offW + j N + i] and out[offB + j] (out holds n values).  The rows go
+// in `parts` parts of perPart (a multiple of 128), each into part[p * partStride].
+struct WeightGradLayer {
+  const __nv_bfloat16* dZT;
+  const __nv_bfloat16* HT;
+  uint32_t N, offW, offB, pad;
+};
+struct WeightGradArgs {
+  WeightGradLayer layer[3];
+  uint32_t rows, perPart, partStride, pad;
+  float* part;
+  uint32_t* err;
+};
+cudaError_t launchWeightGrads(const WeightGradArgs& G, uint32_t parts, float* out, uint32_t n, cudaStream_t stream);
 
 }  // namespace zk
