@@ -7,11 +7,12 @@
 //
 // row statistics: one CTA per request.  Quantiles are the *exact* empirical quantile interpolated
 // between order statistics k = floor(p (n - 1)) and k + 1, as ccr::quantile does
-// (include/ccr/core/math.hpp:39-47), found without sorting the row: a min/max pass (on rows of 64K values or
-// more, over a 1/16 sample: it only sets the first histogram's range), a 4096-bin
+// (include/ccr/core/math.hpp:39-47), found without sorting the row.  Rows of 8K values or more: a 1/16 sample says in
+// which window of values the ranks lie, and one pass counts the values under it and keeps those in it, among which a radix
+// selection finds them.  Shorter rows, and rows whose window misses or overflows: a min/max pass, a 4096-bin
 // histogram pass that locates the bins of ranks k and k + 1, then either one pass that reads the
 // maximum of k's bin and the minimum of k+1's bin (different bins) or a gather of k's bin into
-// shared memory and a bitonic sort there (same bin; narrowed again if the bin holds more than
+// shared memory and a radix selection there (same bin; narrowed again if the bin holds more than
 // kCap values).  The reference's histogram kernel interpolates inside the final bin instead and
 // agrees with the exact quantile to about 5e-8 (README.md:182).
 #include <cfloat>
@@ -29,7 +30,7 @@ constexpr int kBins = 4096;
 constexpr int kCap = 4096;
 constexpr int kMaxRounds = 16;
 constexpr int kHistBins = 3072;  // the reference's histogram-request limit (kPfeBins)
-constexpr int kGather = 4096;    // values of the first histogram pass kept from the bins the sample points at
+constexpr int kGather = 4096;    // values kept from the bins the sample points at
 
 template <typename R>
 struct RowSmem {
@@ -38,11 +39,11 @@ struct RowSmem {
     R cand[kCap];
   };
   R gath[kGather];
-  uint32_t gathCount;
+  alignas(8) uint32_t digits[264];
   double dsum[kRowWarps];
   R rmin[kRowWarps], rmax[kRowWarps];
   uint32_t candCount;
-  uint32_t usum[kRowWarps];
+  uint32_t usum[kRowWarps], ukept[kRowWarps];
   uint32_t pick[4];
   double flo[kMaxRounds], finvw[kMaxRounds];
   uint32_t fb0[kMaxRounds], fb1[kMaxRounds];
@@ -119,57 +120,127 @@ __device__ __forceinline__ bool passes(const RowSmem<R>& s, int rounds, R v) {
   return true;
 }
 
-// Calls f(v, valid) for every value of the row, through max(x, 0) when pos, in warp-uniform steps (every lane
-// calls f the same number of times, so f may vote).  Rows that start on a 16-byte boundary with a length a
-// multiple of 16 bytes are read 16 bytes per load.
+// The 16-byte vectors of a row: the first aligned value and the number of whole vectors after it.
+template <typename R>
+struct RowVectors {
+  uint32_t head, count;
+};
+template <typename R>
+__device__ __forceinline__ RowVectors<R> vectorsOf(const R* X, uint32_t nP) {
+  constexpr uint32_t kVec = 16 / sizeof(R);
+  const uint32_t off = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(X) / sizeof(R)) % kVec, head = min((kVec - off) % kVec, nP);
+  return {head, (nP - head) / kVec};
+}
+
+// Calls f(v, valid) for every value of the row, through max(x, 0) when pos, 16 bytes per load; the values before the first
+// aligned one and after the last whole vector (rows of an odd number of paths start anywhere) one by one.
 template <typename R, typename F>
 __device__ __forceinline__ void forEachValue(const R* X, uint32_t nP, bool pos, F&& f) {
   const uint32_t tid = threadIdx.x;
   auto fix = [&](R x) { return pos ? fmax(x, R(0)) : x; };
   constexpr uint32_t kVec = 16 / sizeof(R);
-  if ((nP % kVec) == 0 && (reinterpret_cast<uintptr_t>(X) & 15u) == 0) {
-    const uint32_t nv = nP / kVec;
-#pragma unroll 2
-    for (uint32_t base = 0; base < nv; base += kRowThreads) {
-      const uint32_t i = base + tid;
-      const bool ok = i < nv;
-      if constexpr (sizeof(R) == 4) {
-        const float4 q = ok ? __ldg(reinterpret_cast<const float4*>(X) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-        f(fix(q.x), ok), f(fix(q.y), ok), f(fix(q.z), ok), f(fix(q.w), ok);
-      } else {
-        const double2 q = ok ? __ldg(reinterpret_cast<const double2*>(X) + i) : make_double2(0.0, 0.0);
-        f(fix(q.x), ok), f(fix(q.y), ok);
-      }
-    }
-  } else {
-    for (uint32_t base = 0; base < nP; base += kRowThreads) {
-      const uint32_t i = base + tid;
-      const bool ok = i < nP;
-      f(fix(ok ? X[i] : R(0)), ok);
+  const RowVectors<R> V = vectorsOf(X, nP);
+  const R* body = X + V.head;
+#pragma unroll 4
+  for (uint32_t base = 0; base < V.count; base += kRowThreads) {
+    const uint32_t i = base + tid;
+    const bool ok = i < V.count;
+    if constexpr (sizeof(R) == 4) {
+      const float4 q = ok ? __ldg(reinterpret_cast<const float4*>(body) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      f(fix(q.x), ok), f(fix(q.y), ok), f(fix(q.z), ok), f(fix(q.w), ok);
+    } else {
+      const double2 q = ok ? __ldg(reinterpret_cast<const double2*>(body) + i) : make_double2(0.0, 0.0);
+      f(fix(q.x), ok), f(fix(q.y), ok);
     }
   }
+  const uint32_t tail = V.head + V.count * kVec, loose = V.head + (nP - tail);
+  if (tid < loose) f(fix(__ldg(X + (tid < V.head ? tid : tail + tid - V.head))), true);
+}
+
+// Values of the row (through max(x, 0) when pos) below `from` counted, and those in [from, to] kept: each warp appends to its
+// own kGatherWarp slots by ballots (an atomic with its returned position stalls the warp at nearly every vector).  Returns
+// this thread's count below; `kept` the warp's values in the window, more than kGatherWarp when they did not fit.
+constexpr uint32_t kGatherWarp = kGather / kRowWarps;
+template <typename R>
+__device__ __forceinline__ uint32_t windowPass(const R* X, uint32_t nP, bool pos, R from, R to, R* gath, uint32_t& kept) {
+  constexpr uint32_t kVec = 16 / sizeof(R), kDeep = 4;
+  const uint32_t tid = threadIdx.x, below = (1u << (tid & 31u)) - 1u;
+  const RowVectors<R> V = vectorsOf(X, nP);
+  const R* body = X + V.head;
+  R* mine = gath + (tid >> 5) * kGatherWarp;
+  uint32_t under = 0, n = 0;
+  auto take = [&](const R (&v)[kVec], bool ok) {
+    bool in[kVec], any = false;
+#pragma unroll
+    for (uint32_t e = 0; e < kVec; ++e) {
+      const R x = pos ? fmax(v[e], R(0)) : v[e];
+      const bool up = x >= from;  // a NaN ranks below, as in the rounds' bin 0
+      under += ok && !up ? 1u : 0u;
+      in[e] = ok && up && x <= to, any = any || in[e];
+    }
+    if (__any_sync(0xFFFFFFFFu, any)) {
+#pragma unroll
+      for (uint32_t e = 0; e < kVec; ++e) {
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, in[e]), at = n + __popc(m & below);
+        if (in[e] && at < kGatherWarp) mine[at] = pos ? fmax(v[e], R(0)) : v[e];
+        n += __popc(m);
+      }
+    }
+  };
+  auto load = [&](uint32_t i, R (&v)[kVec]) {
+    if constexpr (sizeof(R) == 4) {
+      const float4 q = i < V.count ? __ldg(reinterpret_cast<const float4*>(body) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+    } else {
+      const double2 q = i < V.count ? __ldg(reinterpret_cast<const double2*>(body) + i) : make_double2(0.0, 0.0);
+      v[0] = q.x, v[1] = q.y;
+    }
+  };
+  for (uint32_t base = 0; base < V.count; base += kRowThreads * kDeep) {
+    R v[kDeep][kVec];
+#pragma unroll
+    for (uint32_t d = 0; d < kDeep; ++d) load(base + d * kRowThreads + tid, v[d]);
+#pragma unroll
+    for (uint32_t d = 0; d < kDeep; ++d) take(v[d], base + d * kRowThreads + tid < V.count);
+  }
+  // the values outside the whole vectors, fewer than eight: the first warp's
+  const uint32_t tail = V.head + V.count * kVec, loose = V.head + (nP - tail);
+  if (tid < 32) {
+    R v[kVec] = {};
+    if (tid < loose) v[0] = __ldg(X + (tid < V.head ? tid : tail + tid - V.head));
+    const uint32_t before = under;
+    const R x = pos ? fmax(v[0], R(0)) : v[0];
+    const bool ok = tid < loose, up = x >= from, in = ok && up && x <= to;
+    under = before + (ok && !up ? 1u : 0u);
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, in), at = n + __popc(m & below);
+    if (in && at < kGatherWarp) mine[at] = x;
+    n += __popc(m);
+  }
+  kept = n;
+  return under;
 }
 
 // A quantile's histogram needs a range, not the row's exact extremes: values outside it fall into the end bins,
 // and the ranks are still located exactly.  On long rows the range is the minimum and maximum of a sample,
 // every 16th block of 32 vectors (512 bytes, one 16-byte load per lane of a warp), about 1/16 of the row.
 constexpr uint32_t kSampleStride = 16;
-constexpr uint32_t kSampleMinVectors = 16384;  // rows of 64K floats or 32K doubles and more
+constexpr uint32_t kSampleMinVectors = 2048;  // rows of 8K floats or 4K doubles and more
 
 template <typename R>
 __device__ __forceinline__ bool canSample(const R* X, uint32_t nP) {
-  constexpr uint32_t kVec = 16 / sizeof(R);
-  return (nP % kVec) == 0 && (reinterpret_cast<uintptr_t>(X) & 15u) == 0 && nP / kVec >= kSampleMinVectors;
+  return vectorsOf(X, nP).count >= kSampleMinVectors;
 }
 
 template <typename R>
 __device__ __forceinline__ void sampleMinMax(const R* X, uint32_t nP, bool pos, R& lo, R& hi) {
-  constexpr uint32_t kVec = 16 / sizeof(R);
-  const uint32_t nv = nP / kVec, blocks = nv / 32, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const RowVectors<R> V = vectorsOf(X, nP);
+  const uint32_t blocks = V.count / 32, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  X += V.head;
   auto take = [&](R x) {
     x = pos ? fmax(x, R(0)) : x;
     lo = fmin(lo, x), hi = fmax(hi, x);
   };
+#pragma unroll 4
   for (uint32_t b = warp * kSampleStride; b < blocks; b += kRowWarps * kSampleStride) {
     const uint32_t i = b * 32 + lane;
     if constexpr (sizeof(R) == 4) {
@@ -187,12 +258,15 @@ __device__ __forceinline__ void sampleMinMax(const R* X, uint32_t nP, bool pos, 
 template <typename R>
 __device__ __forceinline__ uint32_t sampleHistogram(const R* X, uint32_t nP, bool pos, double dlo, double invw, uint32_t* hist) {
   constexpr uint32_t kVec = 16 / sizeof(R);
-  const uint32_t nv = nP / kVec, blocks = nv / 32, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const RowVectors<R> V = vectorsOf(X, nP);
+  const uint32_t blocks = V.count / 32, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  X += V.head;
   auto put = [&](R x) {  // bin 0 is filled afterwards (fillBinZero)
     x = pos ? fmax(x, R(0)) : x;
     const uint32_t b = binOf(x, dlo, invw);
     if (b != 0) atomicAdd(&hist[b], 1u);
   };
+#pragma unroll 4
   for (uint32_t b = warp * kSampleStride; b < blocks; b += kRowWarps * kSampleStride) {
     const uint32_t i = b * 32 + lane;
     if constexpr (sizeof(R) == 4) {
@@ -249,25 +323,71 @@ __device__ __forceinline__ void locateRanks(RowSmem<R>& s, uint32_t below, uint3
   }
 }
 
-// Bitonic sort of n (<= kCap) values in shared memory, padded with +inf to a power of two.
+__device__ __forceinline__ uint32_t orderKey(float v) { return floatKey(v); }
+__device__ __forceinline__ unsigned long long orderKey(double v) { return doubleKey(v); }
+__device__ __forceinline__ float fromKey(uint32_t k) { return keyFloat(k); }
+__device__ __forceinline__ double fromKey(unsigned long long k) { return keyDouble(k); }
+
+// The values of ranks r and r1 (r or r + 1, below n) among n values in shared memory, by their order-preserving integer keys:
+// a radix selection of 8 bits a pass finds rank r's value, and the next one is that value again or the least above it.  (A
+// bitonic sort of 2,048 values took 66 barriers and 45 us, four passes take 4.)  scratch: 256 + 8 words; every thread gets
+// both values.
 template <typename R>
-__device__ void bitonicSort(R* a, uint32_t n) {
-  uint32_t m = 1;
-  while (m < n) m <<= 1;
-  for (uint32_t i = n + threadIdx.x; i < m; i += kRowThreads) a[i] = R(INFINITY);
-  __syncthreads();
-  for (uint32_t size = 2; size <= m; size <<= 1)
-    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      for (uint32_t i = threadIdx.x; i < m; i += kRowThreads) {
-        const uint32_t partner = i ^ stride;
-        if (partner > i) {
-          const bool up = (i & size) == 0;
-          const R ai = a[i], ap = a[partner];
-          if ((ai > ap) == up) a[i] = ap, a[partner] = ai;
-        }
-      }
-      __syncthreads();
+__device__ __forceinline__ void selectRanks(const R* a, uint32_t n, uint32_t r, uint32_t r1, uint32_t* scratch, R& v, R& v1) {
+  using Key = decltype(orderKey(R(0)));
+  constexpr int kBits = 8 * static_cast<int>(sizeof(R));
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  static_assert(kRowThreads == 256, "a thread per digit");
+  Key prefix = 0, mask = 0;
+  uint32_t rank = r, same = n;  // rank among the values with the prefix; how many those are
+  for (int shift = kBits - 8; shift >= 0; shift -= 8) {
+    scratch[tid] = 0;
+    __syncthreads();
+    for (uint32_t i = tid; i < n; i += kRowThreads) {
+      const Key key = orderKey(a[i]);
+      if ((key & mask) == prefix) atomicAdd(&scratch[static_cast<uint32_t>(key >> shift) & 255u], 1u);
     }
+    __syncthreads();
+    // The digit whose running count passes the rank: each thread scans its digit's count over the CTA.
+    const uint32_t own = scratch[tid];
+    uint32_t incl = own;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    __syncthreads();  // scratch has been read
+    if (lane == 31) scratch[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0;
+    for (uint32_t w = 0; w < warp; ++w) before += scratch[w];
+    const uint32_t lo = before + incl - own;
+    if (own > 0 && lo <= rank && rank < lo + own) scratch[16] = tid, scratch[17] = lo, scratch[18] = own;
+    __syncthreads();
+    prefix |= static_cast<Key>(scratch[16]) << shift, mask |= static_cast<Key>(255) << shift;
+    rank -= scratch[17], same = scratch[18];
+    __syncthreads();
+  }
+  v = fromKey(prefix);
+  v1 = v;
+  if (r1 == r || rank + 1 < same) return;  // rank r + 1 is the same value
+  // The least value above: its key minimum over the CTA, two words for a double's.
+  Key best = ~static_cast<Key>(0);
+  for (uint32_t i = tid; i < n; i += kRowThreads) {
+    const Key key = orderKey(a[i]);
+    if (key > prefix && key < best) best = key;
+  }
+#pragma unroll
+  for (uint32_t o = 16; o > 0; o >>= 1) {
+    const Key t = __shfl_xor_sync(0xFFFFFFFFu, best, o);
+    best = t < best ? t : best;
+  }
+  Key* keys = reinterpret_cast<Key*>(scratch);
+  if (lane == 0) keys[warp] = best;
+  __syncthreads();
+  for (uint32_t w = 0; w < static_cast<uint32_t>(kRowWarps); ++w) best = keys[w] < best ? keys[w] : best;
+  v1 = fromKey(best);
+  __syncthreads();
 }
 
 template <typename R>
@@ -362,14 +482,14 @@ __global__ void __launch_bounds__(kRowThreads, 6) rowStatsKernel(const RowJob<R>
   int rounds = 0;
   R vk = lo, vk1 = lo;
   bool done = false;
-  // On a sampled row the sample's own histogram (same bins as round 0's) says where ranks k, k1 lie to within the
-  // sample's rank error: round 0 then keeps the row's values of the bins holding sample ranks k_s -+ (3 sd + 4) and,
-  // when those hold every value of the bins of k and k1, the quantile is read from them without another pass.
-  uint32_t winLo = 1, winHi = 0;
+  // On a sampled row the sample's own histogram says where ranks k, k1 lie to within the sample's rank error: one pass
+  // counts the row's values under the bins of sample ranks k_s -+ (3 sd + 4) and keeps the values in them, and when the
+  // ranks fall among those (the counts prove it) they are selected there.  No histogram of the row: a shared-memory
+  // atomic per value had bound the pass (100 netting sets, 121 rows each of 250,000 paths: 5.05 ms, 33,333 odd paths x 12
+  // 282 us; now 3.97 ms and 156 us).  Else the rounds below.
   if (sampled) {
     const double dlo0 = static_cast<double>(lo), invw0 = scaleOf(lo, hi);
     for (uint32_t b = tid; b < kBins; b += kRowThreads) s.hist[b] = 0;
-    if (tid == 0) s.gathCount = 0;
     __syncthreads();
     const uint32_t ns = sampleHistogram(X, nP, pos, dlo0, invw0, s.hist);
     __syncthreads();
@@ -379,7 +499,31 @@ __global__ void __launch_bounds__(kRowThreads, 6) rowStatsKernel(const RowJob<R>
     const uint32_t rlo = static_cast<uint32_t>(fmax(ks - sd, 0.0)), rhi = static_cast<uint32_t>(fmin(ks + sd + 1.0, ns - 1.0));
     if (tid < 32) locateRanks(s, 0u, rlo, rhi, tid);
     __syncthreads();
-    winLo = s.pick[0], winHi = s.pick[1];
+    const uint32_t winLo = s.pick[0], winHi = s.pick[1];
+    // The window's edges as values, half a bin outside the bins' centres (the ends open): any edges serve, the counts decide.
+    const R from = winLo == 0 ? R(-INFINITY) : static_cast<R>(dlo0 + (static_cast<double>(winLo) - 0.5) / invw0);
+    const R to = winHi + 1 >= static_cast<uint32_t>(kBins) ? R(INFINITY) : static_cast<R>(dlo0 + (static_cast<double>(winHi) + (sizeof(R) == 4 ? 0.5 : 1.0)) / invw0);
+    uint32_t kept;
+    uint32_t under = windowPass(X, nP, pos, from, to, s.gath, kept);
+    under = __reduce_add_sync(0xFFFFFFFFu, under);
+    __syncthreads();
+    if ((tid & 31u) == 0) s.usum[tid >> 5] = under, s.ukept[tid >> 5] = kept;
+    __syncthreads();
+    uint32_t at = 0, total = 0;
+    bool fit = true;
+    under = 0;
+    for (int w = 0; w < kRowWarps; ++w) {
+      if (w == static_cast<int>(tid >> 5)) at = total;
+      fit = fit && s.ukept[w] <= kGatherWarp;
+      under += s.usum[w], total += s.ukept[w];
+    }
+    if (fit && under <= k && k1 - under < total) {  // the ranks are among the kept values: together in s.cand, and selected
+      for (uint32_t i = tid & 31u; i < kept; i += 32) s.cand[at + i] = s.gath[(tid >> 5) * kGatherWarp + i];
+      __syncthreads();
+      selectRanks(s.cand, total, k - under, k1 - under, s.digits, vk, vk1);
+      done = true;
+    }
+    __syncthreads();
   }
   while (!done) {
     if (rounds >= static_cast<int>(maxRounds)) {
@@ -401,46 +545,16 @@ __global__ void __launch_bounds__(kRowThreads, 6) rowStatsKernel(const RowJob<R>
     const double dlo = static_cast<double>(lo), invw = scaleOf(lo, hi);
     for (uint32_t b = tid; b < kBins; b += kRowThreads) s.hist[b] = 0;
     __syncthreads();
-    const bool gather = rounds == 0 && winLo <= winHi;
-    const uint32_t winSpan = winHi - winLo;
     forEachValue(X, nP, pos, [&](R x, bool ok) {
       const bool in = ok && passes(s, rounds, x);
       const uint32_t b = binOf(x, dlo, invw);
       if (in && b != 0) atomicAdd(&s.hist[b], 1u);  // bin 0 is filled afterwards (fillBinZero)
-      if (gather && in && b - winLo <= winSpan) {
-        const uint32_t at = atomicAdd(&s.gathCount, 1u);
-        if (at < static_cast<uint32_t>(kGather)) s.gath[at] = x;
-      }
     });
     __syncthreads();
     fillBinZero(s.hist, binned, s.usum);
     if (tid < 32) locateRanks(s, below, k, k1, tid);
     __syncthreads();
     const uint32_t b0 = s.pick[0], b1 = s.pick[1], below0 = s.pick[2], c0 = s.pick[3];
-    if (gather && winLo <= b0 && b1 <= winHi && s.gathCount <= static_cast<uint32_t>(kGather)) {
-      // Every value of bins b0..b1 was kept (no bin between them holds one): sort them, read ranks k and k1.
-      if (tid == 0) s.candCount = 0;
-      __syncthreads();
-      const uint32_t ng = s.gathCount;
-      for (uint32_t i = tid; i < ng; i += kRowThreads) {
-        const R v = s.gath[i];
-        const uint32_t b = binOf(v, dlo, invw);
-        if (b >= b0 && b <= b1) {
-          const uint32_t at = atomicAdd(&s.candCount, 1u);
-          if (at < static_cast<uint32_t>(kCap)) s.cand[at] = v;
-        }
-      }
-      __syncthreads();
-      const uint32_t n = s.candCount;
-      if (n <= static_cast<uint32_t>(kCap) && k1 - below0 < n) {
-        bitonicSort(s.cand, n);
-        vk = s.cand[k - below0];
-        vk1 = s.cand[k1 - below0];
-        done = true;
-        continue;
-      }
-      // more than kCap values: the passes below
-    }
     if (b0 != b1) {
       // k is the largest value of bin b0, k + 1 the smallest of bin b1.
       R mx = R(-INFINITY), mn = R(INFINITY);
@@ -461,9 +575,7 @@ __global__ void __launch_bounds__(kRowThreads, 6) rowStatsKernel(const RowJob<R>
       });
       __syncthreads();
       const uint32_t n = s.candCount;
-      bitonicSort(s.cand, n);
-      vk = s.cand[k - below0];
-      vk1 = s.cand[min(k1 - below0, n - 1)];
+      selectRanks(s.cand, n, k - below0, min(k1 - below0, n - 1), s.digits, vk, vk1);
       done = true;
     } else {
       if (tid == 0) s.flo[rounds] = dlo, s.finvw[rounds] = invw, s.fb0[rounds] = b0, s.fb1[rounds] = b0;
@@ -482,23 +594,46 @@ __global__ void __launch_bounds__(kRowThreads, 6) rowStatsKernel(const RowJob<R>
 // sum completes the binary tree of the warp sums ((w0 + w1) + (w2 + w3) for one path per thread, w0 + w1 for
 // two, w0 for four), absent warps past the last path counting as 0, so it has the same bits for every tile
 // shape; the groups are then summed in path order with a compensated double sum.
-template <typename R, int PPT>
-__global__ void reduceKernel(const ReduceJob<R>* __restrict__ jobs) {
+//
+// One CTA per 32 columns (date, statistic), kSegs warps over consecutive segments of the groups, each a compensated sum of
+// its own with four groups' loads in flight; the segments are added in order, compensated too.  (One thread walked all groups
+// of a column: 129 us for 12 netting sets at 33,333 paths and 1,155 us for 100 at
+// 250,000; now 18 and 889.)
+template <typename R, int PPT, int kSegs>
+__global__ void __launch_bounds__(32 * kSegs) reduceKernel(const ReduceJob<R>* __restrict__ jobs) {
+  __shared__ double segSum[kSegs][32], segComp[kSegs][32];
   const ReduceJob<R> J = jobs[blockIdx.y];
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= J.n) return;
+  const uint32_t lane = threadIdx.x & 31u, seg = threadIdx.x >> 5, i = blockIdx.x * 32u + lane;
+  if (blockIdx.x * 32u >= J.n) return;
   // A job with pad 1 or 2 has partials of 32 or 64 paths whatever the batch's shape (the basis kernel's: 64).
   const uint32_t ppt = J.pad == 1u || J.pad == 2u ? J.pad : static_cast<uint32_t>(PPT);
-  const uint32_t kUnits = 4 / ppt, kUnitPaths = 32 * ppt;
-  auto unit = [&](uint32_t u) { return u * kUnitPaths < J.nP ? J.partials[static_cast<size_t>(u) * J.n + i] : R(0); };
+  const uint32_t units = 4 / ppt, unitPaths = 32 * ppt, col = min(i, J.n - 1);
+  const uint32_t count = (J.nP + unitPaths - 1) / unitPaths;  // partials
   double sum = 0.0, comp = 0.0;
-  for (uint32_t t = 0; t < J.numTiles; ++t) {
-    const uint32_t u0 = t * kUnits;
-    R g;
-    if (ppt == 1) g = (unit(u0) + unit(u0 + 1)) + (unit(u0 + 2) + unit(u0 + 3));
-    else if (ppt == 2) g = unit(u0) + unit(u0 + 1);
-    else g = unit(u0);
+  auto add = [&](R g) {
     const double yv = static_cast<double>(g) - comp;
+    const double tv = sum + yv;
+    comp = (tv - sum) - yv;
+    sum = tv;
+  };
+  const uint32_t t0 = static_cast<uint32_t>(static_cast<uint64_t>(J.numTiles) * seg / kSegs);
+  const uint32_t t1 = static_cast<uint32_t>(static_cast<uint64_t>(J.numTiles) * (seg + 1) / kSegs);
+  const R* __restrict__ P = J.partials + col;
+  auto unit = [&](uint32_t u) { return u < count ? __ldg(P + static_cast<size_t>(u) * J.n) : R(0); };
+#pragma unroll 4
+  for (uint32_t t = t0; t < t1; ++t) {
+    const uint32_t u = t * units;
+    R g;
+    if (ppt == 1) g = (unit(u) + unit(u + 1)) + (unit(u + 2) + unit(u + 3));
+    else if (ppt == 2) g = unit(u) + unit(u + 1);
+    else g = unit(u);
+    add(g);
+  }
+  segSum[seg][lane] = sum, segComp[seg][lane] = comp;
+  __syncthreads();
+  if (seg != 0 || i >= J.n) return;
+  for (int s = 1; s < kSegs; ++s) {  // sum - comp is the segment's sum to more than double precision
+    const double yv = (segSum[s][lane] - segComp[s][lane]) - comp;
     const double tv = sum + yv;
     comp = (tv - sum) - yv;
     sum = tv;
@@ -511,11 +646,14 @@ __global__ void reduceKernel(const ReduceJob<R>* __restrict__ jobs) {
 template <typename R>
 cudaError_t launchReduce(const ReduceJob<R>* jobs, uint32_t numJobs, uint32_t maxN, int ppt, cudaStream_t stream) {
   if (numJobs == 0 || maxN == 0) return cudaSuccess;
-  const dim3 grid((maxN + 255) / 256, numJobs);
+  const dim3 grid((maxN + 31) / 32, numJobs);
+  // 32 segments where the columns alone leave the GPU idle, 8 where they fill it.
+  const bool few = static_cast<uint64_t>(grid.x) * grid.y < 148u * 8u;
+  auto go = [&](auto kernel, int segs) { kernel<<<grid, 32 * segs, 0, stream>>>(jobs); };
   switch (ppt) {
-    case 1: reduceKernel<R, 1><<<grid, 256, 0, stream>>>(jobs); break;
-    case 2: reduceKernel<R, 2><<<grid, 256, 0, stream>>>(jobs); break;
-    case 4: reduceKernel<R, 4><<<grid, 256, 0, stream>>>(jobs); break;
+    case 1: few ? go(reduceKernel<R, 1, 32>, 32) : go(reduceKernel<R, 1, 8>, 8); break;
+    case 2: few ? go(reduceKernel<R, 2, 32>, 32) : go(reduceKernel<R, 2, 8>, 8); break;
+    case 4: few ? go(reduceKernel<R, 4, 32>, 32) : go(reduceKernel<R, 4, 8>, 8); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
