@@ -149,7 +149,7 @@ zk_status zk_amc_states(zk_context* ctx, const zk_plan_view* plan, float* x, flo
 /* Replaces the Longstaff-Schwartz fit that the reference's gpu::compile runs on its CPU kernels (fitAmc,
  * src/gpu/fused_exposure.cpp:103-156): the AMC state pass on the GPU, then the policy regression of every
  * exercise (in-the-money paths, backwards) and the continuation regression of every date, in double
- * precision with FP64 Cholesky solves, one thread-block cluster per Bermudan.  terms_out (terms_len =
+ * precision with FP64 Cholesky solves, every regression over the whole GPU.  terms_out (terms_len =
  * plan->terms_len) receives the plan's term table with the fitted policy and continuation records;
  * degrees[b] (<= 3) is the regression degree of Bermudan b, num_bermudans the plan's count (header[27]). */
 zk_status zk_fit_amc(zk_context* ctx, const zk_plan_view* plan, const uint32_t* degrees, size_t num_bermudans, float* terms_out,
