@@ -482,10 +482,10 @@ __device__ __forceinline__ void revalueDate(const NsArgs<R>& A, const CubeArgs<R
     for (int i = 0; i < PPT; ++i) value[i] = fma(fma(r.x, fix(slot, i), r.y), termExp(r.z, x[i]), value[i]);
   }
 #pragma unroll 2
-  for (uint32_t u = d0.y; u < d0.z; ++u) {  // bonds, two per record
+  for (uint32_t u = d0.y; u < d0.z; ++u) {  // bonds, two per record (which product is fused is written out: kernels differed in FP64)
     const R4 r = ld4(table + 4 * u);
 #pragma unroll
-    for (int i = 0; i < PPT; ++i) value[i] += r.x * termExp(r.y, x[i]) + r.z * termExp(r.w, x[i]);
+    for (int i = 0; i < PPT; ++i) value[i] += fma(r.x, termExp(r.y, x[i]), r.z * termExp(r.w, x[i]));
   }
   for (uint32_t u = d0.z; u < d0.w; ++u) {  // asset forwards: (c, A, asset)
     const R4 r = ld4(table + 4 * u);
