@@ -3,10 +3,14 @@ and beyond the tables that this package's compiler writes.  A book in waves has 
 kernels revalue it."""
 from __future__ import annotations
 
+import copy
+
 import numpy as np
 import pytest
 
+from oracle import restated
 from setups import bermudan, gpu_model, swap_book
+from test_gpu_parity import check_sums
 from zlatko_b200 import gpu
 from zlatko_b200 import spec as S
 
@@ -14,6 +18,7 @@ pytestmark = pytest.mark.gpu
 
 TRADES = [S.Swap(1e6, 0.028, True, S.vanilla_schedule(0.0, 5.0, 2)), S.Forward(0, 5e5, 1.12, 3.0), S.Option(0, True, -4e5, 1.15, 2.0)]
 CSA = S.Csa(2e4, 2e4, 5e3)
+FIXED_FLOAT, SET_FIXING = 1, 3  # kinds: the low four bits of a record's code
 
 
 def walked(ctx, run, plan):
@@ -40,3 +45,34 @@ def test_double_precision(ctx, book, paths):
         p = ctx.fit_amc_f64(p)
     got = ctx.run_f64(p)
     assert np.isfinite(got[0]).all() and same(got, walked(ctx, ctx.run_f64, p))
+
+
+def with_fields(plan, kinds, field):
+    """The plan with `field` added to the codes of its records of `kinds`."""
+    p = copy.copy(plan)
+    p.tables64 = dict(plan.tables64)
+
+    def coded(terms):
+        t = terms.reshape(-1, 8).copy()
+        hit = np.isin(t[:, 0], kinds)
+        assert hit.any()
+        t[hit, 0] += field
+        return t.reshape(-1)
+
+    p.terms, p.tables64["terms"] = coded(plan.terms), coded(plan.tables64["terms"])
+    return p
+
+
+@pytest.mark.parametrize("kinds", [(FIXED_FLOAT,), (SET_FIXING,), (FIXED_FLOAT, SET_FIXING)])
+@pytest.mark.parametrize("field", [1 << 4, 15 << 4, 3 << 12])
+@pytest.mark.parametrize("paths", [129, 4100])
+def test_fixings_among_the_generic_records(ctx, kinds, field, paths):
+    """The trade-group field of a code means nothing outside the per-trade views: a coupon or fixing with a group there is
+    priced like the bare one.  It is among the generic records, and a run of dates that starts after the fixing has to find
+    it all the same."""
+    plan = gpu.compile(gpu_model(paths), S.NettingSet(TRADES, CSA), S.Options(pfe_quantile=0.975))
+    p = with_fields(plan, kinds, field)
+    got = ctx.run(p)
+    assert same(got, walked(ctx, ctx.run, p))
+    assert same(ctx.run_f64(p), walked(ctx, ctx.run_f64, p))
+    check_sums(p, got[0], restated.run_plan(p)[0], 2e-4)

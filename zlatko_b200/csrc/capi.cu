@@ -943,18 +943,18 @@ void planSplit(Batch<R>& B, typename Batch<R>::Launch& L) {
       std::vector<uint8_t> read(P.nSlots, P.im ? 1 : 0), fresh(P.nSlots, 0);  // the margin's start reads every fixing
       for (uint32_t j = j0; j < j1; ++j) {
         const uint32_t* d = &P.dates[8 * static_cast<size_t>(j)];
-        for (uint32_t u = d[0]; u < d[1]; ++u) {
-          const uint32_t q = asUint(P.table[4 * static_cast<size_t>(u) + 3]);
-          if (!fresh[q]) read[q] = 1;
+        auto word = [&](uint32_t u, uint32_t w) { return asUint(P.table[4 * static_cast<size_t>(u) + w]); };
+        auto use = [&](uint32_t q) { read[q] = read[q] || !fresh[q]; };
+        // in the order of the kernel: coupons, generic records (coupons and fixings among them whose code has more than
+        // its kind), fixings
+        for (uint32_t u = d[0]; u < d[1]; ++u) use(word(u, 3));
+        for (uint32_t u = d[3]; u < d[4]; u += 2) {
+          const uint32_t kind = word(u, 0) & 15u, q = word(u, 1);
+          if (kind == kBermBond && q >= kBlockMark) u += 2 * ((q - kBlockMark + 1) / 2);
+          if (kind == kBermFloat || kind == kFixedFloat) use(q);
+          if (kind == kSetFixing) fresh[q] = 1, now[q] = make_uint2(u, j | kGenericFixing);
         }
-        for (uint32_t t = P.v.indices[j]; t < P.v.indices[j + 1]; ++t) {
-          const R* r = P.v.terms + static_cast<size_t>(t) * kTermStride;
-          if ((static_cast<uint32_t>(r[0]) & 15u) == kBermFloat && !fresh[static_cast<uint32_t>(r[1])]) read[static_cast<uint32_t>(r[1])] = 1;
-        }
-        for (uint32_t u = d[4]; u < d[5]; ++u) {
-          const uint32_t q = asUint(P.table[4 * static_cast<size_t>(u) + 3]);
-          fresh[q] = 1, now[q] = make_uint2(u, j);
-        }
+        for (uint32_t u = d[4]; u < d[5]; ++u) fresh[word(u, 3)] = 1, now[word(u, 3)] = make_uint2(u, j);
       }
       for (uint32_t q = 0; q < P.nSlots; ++q)
         if (read[q] && set[q].x != kNoRow) S.pre.push_back(set[q]);

@@ -443,6 +443,12 @@ __device__ __forceinline__ double mulRn(double a, double b) { return __dmul_rn(a
 __device__ __forceinline__ float addRn(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double addRn(double a, double b) { return __dadd_rn(a, b); }
 
+// The fixing that a generic record (1 / the period's length in c) sets from its date's short rate.
+template <typename R>
+__device__ __forceinline__ R genericFixing(const R (&rec)[8], R x) {
+  return (rec[3] * fastExp(-rec[4] * x) - R(1)) / rec[2];
+}
+
 // The netting set's value on date j of a thread's PPT paths (value), from the date's lowered runs [d0, d1), and the
 // fixings and exercise states the date sets.  state: the fixings [slot][PPT][kTile]; the exercise index of Bermudan b
 // (-1: not exercised) in bytes exS[b][PPT][kTile] when exBytes, else in registers ex.  kGiven: the decisions are those
@@ -545,7 +551,7 @@ __device__ __forceinline__ void revalueDate(const NsArgs<R>& A, const CubeArgs<R
         break;
       case kSetFixing:
 #pragma unroll
-        for (int i = 0; i < PPT; ++i) fix(slot, i) = (rec[3] * fastExp(nB * x[i]) - R(1)) / c;
+        for (int i = 0; i < PPT; ++i) fix(slot, i) = genericFixing(rec, x[i]);
         break;
       case kOption: {
         const R p3 = rec[7];
@@ -1090,9 +1096,16 @@ __global__ void __launch_bounds__(kTile, (sizeof(R) == 8 ? 4 : kLean ? 8 : 6)) v
     for (int i = 0; i < PPT; ++i) state[(q * PPT + i) * kTile + tid] = R(0);
   for (uint32_t q = I.preBegin; q < I.preEnd; ++q) {
     const uint2 f = __ldg(pre + q);  // fixing record, date
-    const auto r = ld4(A.table + 4 * static_cast<size_t>(f.x));
     R x[PPT];
-    load(static_cast<size_t>(f.y) * nP, x);
+    load(static_cast<size_t>(f.y & ~kGenericFixing) * nP, x);
+    if (f.y & kGenericFixing) {
+      R rec[8];
+      loadTerm(A.table + 4 * static_cast<size_t>(f.x), rec);
+#pragma unroll
+      for (int i = 0; i < PPT; ++i) state[(asUint(rec[1]) * PPT + i) * kTile + tid] = genericFixing(rec, x[i]);
+      continue;
+    }
+    const auto r = ld4(A.table + 4 * static_cast<size_t>(f.x));
 #pragma unroll
     for (int i = 0; i < PPT; ++i) state[(asUint(r.w) * PPT + i) * kTile + tid] = (r.x * termExp(r.y, x[i]) - R(1)) * r.z;
   }

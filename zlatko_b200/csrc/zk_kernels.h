@@ -29,9 +29,10 @@ cudaError_t launchRevalue(const CubeArgs<R>& cb, const NsArgs<R>* nsArgs, uint32
 size_t revalueSmemBytes(size_t stateWordsMax, bool perTrade, bool f64, int ppt);
 
 // The revaluation split over the dates (valueKernel and the kernels beside it): a run of dates [j0, j1) of netting set ns,
-// the fixings set before it that it reads -- (record of the lowered table, date) pairs pre[preBegin, preEnd) -- and per
-// Bermudan the number of exercises decided before it, exFirst[exAt + b]; and per Bermudan the records of its exercise
+// the fixings set before it that it reads -- (record of the lowered table, date) pairs pre[preBegin, preEnd), the date with
+// kGenericFixing for a generic record -- and per Bermudan the number of exercises decided before it, exFirst[exAt + b]; and per Bermudan the records of its exercise
 // dates in `decideTable` [begin, end), in units of 4 values: a record (kBond, date) before each date's; codes by their bits.
+constexpr uint32_t kGenericFixing = 0x80000000u;
 struct ValueItem {
   uint32_t ns, j0, j1, preBegin, preEnd, exAt, pad[2];
 };
