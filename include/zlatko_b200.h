@@ -91,7 +91,9 @@ zk_status zk_context_set_stream(zk_context* ctx, void* stream);
  * default: all netting sets at once while that takes under 70% of the free device memory, else 60% of it).  A
  * book whose rows exceed it runs its netting sets in waves that reuse one region: each wave's reduce and row
  * statistics follow its revalue launch, and the outputs are the same bits as in one wave.  (The reference's
- * kernels keep every netting set's rows, EXPO[rows][P], at once: fused_exposure.hpp:214-216.) */
+ * kernels keep every netting set's rows, EXPO[rows][P], at once: fused_exposure.hpp:214-216.)  The values of a
+ * revaluation split over the dates take what the budget leaves beside the rows, in fewer paths at a time, and where it
+ * leaves too little the netting sets are revalued date after date without them: the same bits either way. */
 zk_status zk_context_set_row_budget(zk_context* ctx, uint64_t bytes);
 /* Which netting sets of a call or batch run on the tensor-core basis kernel: single-precision plans of bonds,
  * floating coupons, FX forwards and options, with no CSA or a cash CSA looking back at most one date and no rows

@@ -76,3 +76,79 @@ def test_fixings_among_the_generic_records(ctx, kinds, field, paths):
     assert same(got, walked(ctx, ctx.run, p))
     assert same(ctx.run_f64(p), walked(ctx, ctx.run_f64, p))
     check_sums(p, got[0], restated.run_plan(p)[0], 2e-4)
+
+
+def rows_and_partials(plans, size=4):
+    up = lambda b: (b + 255) // 256 * 256  # noqa: E731
+    return sum(up(p.rows_total * p.num_paths * size) + up((p.num_paths + 31) // 32 * p.num_dates * p.stats_per_date * size) for p in plans)
+
+
+def kernels(ctx, plans):
+    b = ctx.batch(plans)
+    try:
+        return b.info().kernels_per_execute
+    finally:
+        b.close()
+
+
+def books(paths, seed=7):
+    """Netting sets with Bermudans and margin calls that look back, and one without: the same dates."""
+    m = gpu_model(paths, seed)
+    m.base_grid = [k / 8.0 for k in range(1, 41)]
+    csa = S.Csa(1e4, 1e4, 1e3, 500.0, 0.3)
+    return [gpu.compile(m, S.NettingSet(TRADES[:1 + k % 3] + [bermudan(fixed=0.02 + 0.004 * k, pay=bool(k % 2))] * (k > 0), csa),
+                        S.Options(collateral_bands=True)) for k in range(4)]
+
+
+@pytest.mark.parametrize("paths", [1001, 1024])
+@pytest.mark.parametrize("slabs", [1, 2, 4])
+def test_slabs_within_the_row_budget(ctx, paths, slabs):
+    """The values of the split take what the budget leaves beside the rows: slabs of 512 or 256 paths, or the walk."""
+    plans = [ctx.fit_amc(p) if p.amc_degrees else p for p in books(paths)]
+    tile = len(plans) * plans[0].num_dates * 4 * 256
+    rows = rows_and_partials(plans) + len(plans) * 1280  # a byte per path and Bermudan
+    whole = ctx.run_many(plans)
+    assert kernels(ctx, plans) == 1 + 1 + 3 + 2  # simulate; decide; values with and without Bermudans, settle; statistics
+    try:
+        ctx.set_row_budget(rows + tile * (4 // slabs) + tile // 2)
+        assert kernels(ctx, plans) == 1 + 1 + 3 * slabs + 2
+        assert all(same(a, b) for a, b in zip(whole, ctx.run_many(plans)))
+        ctx.set_row_budget(rows + tile // 2)
+        assert kernels(ctx, plans) == 1 + 1 + 2  # revalueKernel
+        assert all(same(a, b) for a, b in zip(whole, ctx.run_many(plans)))
+    finally:
+        ctx.set_row_budget(0)
+
+
+@pytest.mark.parametrize("slabs", [1, 2, 4])
+def test_slabs_in_double_precision(ctx, slabs):
+    p = ctx.fit_amc_f64(books(1001)[1])
+    whole = ctx.run_f64(p)
+    try:
+        ctx.set_row_budget(rows_and_partials([p], 8) + 1280 + p.num_dates * 8 * (256 * (4 // slabs) + 128))
+        assert same(whole, ctx.run_f64(p))
+    finally:
+        ctx.set_row_budget(0)
+
+
+def test_a_margin_plan_stays_within_the_row_budget(ctx):
+    """Plans of the nested margin never run in waves; their split's values count against the budget like the others'."""
+    p = gpu.compile(gpu_model(257), S.NettingSet(TRADES, CSA), S.Options(im_quantile=0.99, im_inner_paths=32, im_margin_period=0.25))
+    whole = ctx.run(p)
+    assert kernels(ctx, [p]) == 1 + 2 + 1 + 2  # simulate; values, settle; the inner paths; statistics
+    try:
+        ctx.set_row_budget(1)
+        assert kernels(ctx, [p]) == 1 + 1 + 1 + 2
+        assert same(whole, ctx.run(p))
+    finally:
+        ctx.set_row_budget(0)
+
+
+def test_scenarios_share_the_scratch(ctx):
+    """Two scenarios in one call, each split over the dates: each has the bits of its own call."""
+    plans = [ctx.fit_amc(p) if p.amc_degrees else p for seed in (7, 8) for p in books(777, seed)]
+    assert kernels(ctx, plans) == 2 * (1 + 1 + 3) + 2
+    both = ctx.run_many(plans)
+    for first in (0, 4):
+        alone = ctx.run_many(plans[first:first + 4])
+        assert all(same(a, b) for a, b in zip(alone, both[first:]))

@@ -133,7 +133,7 @@ struct zk_context {
   // quantile's narrowing rounds.
   uint64_t failAtLaunch = 0, launchCount = 0;
   uint32_t rowRounds = 16;
-  // Device bytes a batch may give to per-path rows and warp partials at once (zk_context_set_row_budget); 0: all
+  // Device bytes a batch may give to per-path rows, warp partials and the split's scratch (zk_context_set_row_budget); 0: all
   // of its netting sets at once while that takes under 70% of the free device memory, else waves in 60% of it.
   uint64_t rowBudget = 0;
   // Which netting sets run on the tensor-core basis kernel (zk_context_set_basis): 0 groups of at least
@@ -883,9 +883,11 @@ bool exercisePrograms(const Plan<R>& P, uint32_t ns, std::vector<std::vector<uin
 }
 
 // Sets up the split over the dates of a launch's netting sets [basisCount, n) (Launch::split), or leaves it off where
-// a plan needs revalueKernel: per-trade views, or Bermudans whose exercise indices do not follow their dates.
+// a plan needs revalueKernel -- per-trade views, or Bermudans whose exercise indices do not follow their dates -- or its
+// scratch would take more than `most` bytes.
 template <typename R>
-void planSplit(Batch<R>& B, typename Batch<R>::Launch& L) {
+void planSplit(Batch<R>& B, typename Batch<R>::Launch& L, size_t most) {
+  L.split = {};
   const size_t nb = L.basisCount, n = L.planIdx.size() - nb;
   if (n == 0 || n > 16384) return;
   const uint32_t nP = L.sc.nP, nT = L.sc.nT;
@@ -909,10 +911,13 @@ void planSplit(Batch<R>& B, typename Batch<R>::Launch& L) {
   bool anyFull = false;
   for (size_t k = 0; k < n; ++k) anyFull = anyFull || full(B.plans[L.planIdx[nb + k]]);
   if (!anyFull && static_cast<uint64_t>(nP) * n > (1u << 20)) return;
-  // One slab's values take at most 1 GB (slabs of 64 MB, which would stay in the L2, cost 15% in their tails).
-  const size_t perPath = n * nT * sizeof(R), most = size_t(1) << 30;
-  S.slab = static_cast<uint32_t>(std::min<size_t>((nP + 255u) / 256u * 256u, std::max<size_t>(most / perPath / 256 * 256, 256)));
-  S.valsBytes = perPath * S.slab;
+  // One slab's values take 1 GB, or 256 paths' where those are more (slabs of 64 MB, which would stay in the L2, cost 15% in
+  // their tails), and less where `most` leaves less.
+  const size_t tile = n * nT * sizeof(R) * 256, tiles = std::min<size_t>((nP + 255u) / 256u, std::max<size_t>((size_t(1) << 30) / tile, 1));
+  const size_t fit = most > S.indexBytes ? std::min<size_t>((most - S.indexBytes) / tile, tiles) : 0;
+  if (fit == 0) return;
+  S.slab = static_cast<uint32_t>(fit) * 256u;
+  S.valsBytes = tile * fit;
   // Runs of dates of about equal work, enough of them for several CTAs per SM and slab: an item's cost counts its term
   // records (a generic record as three) and a date's own work.
   auto cost = [](const uint32_t* d) { return (d[2] - d[0]) + (d[3] - d[2]) + 3 * (d[4] - d[3]) / 2 + (d[5] - d[4]) + 6; };
@@ -925,7 +930,7 @@ void planSplit(Batch<R>& B, typename Batch<R>::Launch& L) {
   // 32 paths per CTA of settleKernel while they run in one wave (11.5 us against 20 at 2,000 paths), 64 beyond (384 against
   // 412 us at 12 x 33,333).
   S.settlePaths = static_cast<uint64_t>((nP + 31) / 32) * n <= 148 * 6 ? 32 : 64;
-  const uint64_t tiles = (S.slab + kTile * S.ppt - 1) / (kTile * S.ppt), want = std::min<uint64_t>(std::max<uint64_t>((148ull * 64) / tiles, 1), 32768);
+  const uint64_t ctas = (S.slab + kTile * S.ppt - 1) / (kTile * S.ppt), want = std::min<uint64_t>(std::max<uint64_t>((148ull * 64) / ctas, 1), 32768);
   const uint64_t each = std::max<uint64_t>(total / want, 1);
   std::vector<std::pair<uint64_t, ValueItem>> order;
   for (size_t k = 0; k < n; ++k) {
@@ -1008,6 +1013,7 @@ struct BuildOpts {
   const std::vector<std::vector<uint32_t>>* maps = nullptr;
   const Presim* presim = nullptr;  // the first plan's scenario already simulated (single precision, counter normals)
   bool ctxArena = false;  // the batch goes into the context's arena
+  bool factors = false;   // only the factor paths: nothing is revalued
 };
 
 // parsed: the plans already validated and lowered (their views' tables stay the caller's), else parsed from views.
@@ -1092,10 +1098,6 @@ std::unique_ptr<Batch<R>> build(zk_context* ctx, std::vector<View<R>> views, boo
     return alignUp(static_cast<size_t>(std::max<uint32_t>(P.v.rows_total, 1)) * P.nP * sizeof(R)) +
            alignUp(static_cast<size_t>(warps) * P.nT * P.nS * sizeof(R));
   };
-  // Whether the batch may run split over the dates: with a context (the no-alloc entry has a fixed array), not the AMC
-  // state pass, not the re-run of chosen paths (its plans run side by side on worker streams).
-  if (ctx && !sink && !opts.maps)
-    for (auto& L : B->launches) planSplit(*B, L);
   // The AMC state pass reads the exercises' records alone; x and the deflator stay in the factor cube.
   if (sink) {
     auto& S = B->launches[0].split;
@@ -1135,13 +1137,6 @@ std::unique_ptr<Batch<R>> build(zk_context* ctx, std::vector<View<R>> views, boo
     }
   }
   B->basisArgsOff = take(B->numGroups * sizeof(BasisArgs));
-  for (auto& L : B->launches) {
-    auto& S = L.split;
-    if (sink && B->sinkPrograms) S.oDecides = take(S.decides.size() * sizeof(DecideJob)), S.oTable = take(S.table.size() * sizeof(R));
-    if (!S.on) continue;
-    S.oItems = take(S.items.size() * sizeof(ValueItem)), S.oPre = take(S.pre.size() * sizeof(uint2)), S.oFirst = take(S.exFirst.size());
-    S.oDecides = take(S.decides.size() * sizeof(DecideJob)), S.oTable = take(S.table.size() * sizeof(R));
-  }
   B->reduceOff = take(nPlans * sizeof(ReduceJob<R>));
   for (const auto& P : B->plans) B->numRowJobs += static_cast<uint32_t>(P.nReq);
   B->rowOff = take(B->numRowJobs * sizeof(RowJob<R>));
@@ -1154,48 +1149,78 @@ std::unique_ptr<Batch<R>> build(zk_context* ctx, std::vector<View<R>> views, boo
     const auto& P = B->plans[0];
     B->normalsOff = take(static_cast<size_t>(P.nT - 1) * P.nNormals * streams * sizeof(R));
   }
-  B->inputBytes = off;
-  for (auto& L : B->launches)
-    if (!L.presim) L.cubeOff = take(static_cast<size_t>(L.numFields) * L.sc.nT * L.sc.nP * sizeof(R));
   // Rows and warp partials: one region per plan, or -- when they exceed the row budget -- waves of netting sets
   // (in each launch's order) that reuse one region, sized by the largest wave.
-  size_t allRows = 0;
-  bool anyIm = false;
-  for (const auto& P : B->plans) allRows += rowsBytes(P), anyIm = anyIm || P.im;
-  size_t splitBytes = 0;
-  for (const auto& L : B->launches)
-    if (L.split.on) splitBytes += alignUp(L.split.valsBytes) + alignUp(std::max<size_t>(L.split.indexBytes, 16));
-  uint64_t budget = ctx ? ctx->rowBudget : 0;
-  // Asking the driver for the free memory takes 0.1 ms, and milliseconds when other processes keep it busy: only a batch
-  // that may run in waves asks, and not when the context's arena already holds it whole (no memory is taken then).
-  size_t whole = off + allRows + splitBytes;  // the arena of the batch in one wave
   auto sized = [](size_t bytes) { return alignUp(std::max<size_t>(bytes, 16)); };
+  size_t allRows = 0, fixed = off;  // fixed: the arena of the batch in one wave without the split's tables and scratch
+  bool anyIm = false;
   for (const auto& P : B->plans) {
-    whole += sized(static_cast<size_t>(P.nT) * P.nS * sizeof(R)) + sized(static_cast<size_t>(std::max<uint32_t>(P.v.num_outputs, 1)) * sizeof(R));
-    if (opts.exact && !P.guard.empty()) whole += sized(static_cast<size_t>((P.nP + 31) / 32) * 4);
+    allRows += rowsBytes(P), anyIm = anyIm || P.im;
+    fixed += sized(static_cast<size_t>(P.nT) * P.nS * sizeof(R)) + sized(static_cast<size_t>(std::max<uint32_t>(P.v.num_outputs, 1)) * sizeof(R));
+    if (opts.exact && !P.guard.empty()) fixed += sized(static_cast<size_t>((P.nP + 31) / 32) * 4);
+    if (P.im && !sink) fixed += sized(static_cast<size_t>(P.nR) * (5 + P.nSlots) * P.nP * sizeof(R));
   }
-  const bool mayWave = !sink && !anyIm && !normals && !(opts.ctxArena && ctx && whole <= ctx->arenaBytes);
-  if (ctx && budget == 0 && mayWave) {
+  for (const auto& L : B->launches)
+    if (!L.presim) fixed += sized(static_cast<size_t>(L.numFields) * L.sc.nT * L.sc.nP * sizeof(R));
+  fixed += allRows;
+  // Whether the batch may run split over the dates: with a context (the no-alloc entry has a fixed array), not the AMC
+  // state pass, not the re-run of chosen paths (its plans run side by side on worker streams).  The launches run one after
+  // the other, so one region of scratch serves them all: within what an explicit budget leaves beside the rows and what
+  // the device has left.
+  const bool maySplit = ctx && !sink && !opts.maps && !opts.factors, mayWave = !sink && !anyIm && !normals && !opts.factors;
+  uint64_t budget = ctx ? ctx->rowBudget : 0;
+  size_t tables = 0, scratch = 0;
+  auto planSplits = [&](size_t most) {
+    tables = scratch = 0;
+    for (auto& L : B->launches) {
+      planSplit(*B, L, most);
+      const auto& S = L.split;
+      if (!S.on) continue;
+      tables += sized(S.items.size() * sizeof(ValueItem)) + sized(S.pre.size() * sizeof(uint2)) + sized(S.exFirst.size()) +
+                sized(S.decides.size() * sizeof(DecideJob)) + sized(S.table.size() * sizeof(R));
+      scratch = std::max(scratch, alignUp(S.valsBytes) + sized(S.indexBytes));
+    }
+  };
+  if (maySplit) planSplits(budget == 0 ? SIZE_MAX : budget > allRows ? budget - allRows : 0);
+  // Asking the driver for the free memory takes 0.1 ms, and milliseconds when other processes keep it busy: only a batch
+  // that may run in waves or split asks, and not when the context's arena already holds it whole (no memory is taken then).
+  const bool held = opts.ctxArena && ctx && fixed + tables + scratch <= ctx->arenaBytes;
+  if (ctx && !held && ((budget == 0 && mayWave) || scratch > 0)) {
     size_t freeB = 0, totalB = 0;
     if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess) {
       cudaGetLastError();
     } else {
-      if (allRows > freeB / 10 * 7) budget = freeB / 10 * 6;
-      if (whole > freeB / 10 * 9)  // no room for the split's values
-        for (auto& L : B->launches) L.split.on = false;
+      if (budget == 0 && mayWave && allRows > freeB / 10 * 7) budget = freeB / 10 * 6;
+      const size_t room = (freeB + (opts.ctxArena ? ctx->arenaBytes : 0)) / 10 * 9;  // an arena too small is given back first
+      if (scratch > 0 && fixed + tables + scratch > room) planSplits(room > fixed + tables ? room - fixed - tables : 0);
     }
   }
-  B->waved = budget > 0 && allRows > budget && !sink && !anyIm && !normals;
+  B->waved = budget > 0 && allRows > budget && mayWave;
+  if (B->waved)
+    for (auto& L : B->launches) L.split.on = false;
+  for (auto& L : B->launches) {
+    auto& S = L.split;
+    if (sink && B->sinkPrograms) S.oDecides = take(S.decides.size() * sizeof(DecideJob)), S.oTable = take(S.table.size() * sizeof(R));
+    if (!S.on) continue;
+    S.oItems = take(S.items.size() * sizeof(ValueItem)), S.oPre = take(S.pre.size() * sizeof(uint2)), S.oFirst = take(S.exFirst.size());
+    S.oDecides = take(S.decides.size() * sizeof(DecideJob)), S.oTable = take(S.table.size() * sizeof(R));
+  }
+  B->inputBytes = off;
+  for (auto& L : B->launches)
+    if (!L.presim) L.cubeOff = take(static_cast<size_t>(L.numFields) * L.sc.nT * L.sc.nP * sizeof(R));
   auto placeRows = [&](size_t i, auto&& takeFn) {
     const auto& P = B->plans[i];
     const uint32_t warps = (P.nP + 31) / 32;
     B->dev[i].expo = takeFn(static_cast<size_t>(std::max<uint32_t>(P.v.rows_total, 1)) * P.nP * sizeof(R));
     B->dev[i].partials = takeFn(static_cast<size_t>(warps) * P.nT * P.nS * sizeof(R));
   };
-  if (B->waved)
-    for (auto& L : B->launches) L.split.on = false;
-  for (auto& L : B->launches)
-    if (L.split.on) L.split.oVals = take(L.split.valsBytes), L.split.oIndex = take(L.split.indexBytes);
+  size_t region = 0;
+  for (const auto& L : B->launches)
+    if (L.split.on) region = std::max(region, alignUp(L.split.valsBytes) + sized(L.split.indexBytes));
+  if (region > 0) {
+    const size_t at = take(region);
+    for (auto& L : B->launches) L.split.oVals = at, L.split.oIndex = at + alignUp(L.split.valsBytes);
+  }
   if (!B->waved) {
     for (size_t i = 0; i < nPlans; ++i) {
       const auto& P = B->plans[i];
@@ -2798,7 +2823,9 @@ zk_status zk_factor_paths_f64(zk_context* ctx, const zk_plan_view_f64* plan, con
   try {
     requireCtx(ctx);
     if (!plan || !out) throw fail(ZK_ERR_INVALID_ARGUMENT, "null argument");
-    auto B = build<double>(ctx, {viewOf(*plan)}, false, normals, streams);
+    BuildOpts bo;
+    bo.ctxArena = bo.factors = true;
+    auto B = build<double>(ctx, {viewOf(*plan)}, false, normals, streams, bo);
     const auto& L = B->launches.front();
     const size_t n = static_cast<size_t>(2 + L.sc.nA) * L.sc.nT * L.sc.nP;
     if (out_len != n) throw fail(ZK_ERR_INVALID_ARGUMENT, "out must hold (2 + nA) nT nP = %zu values", n);
