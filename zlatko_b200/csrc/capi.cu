@@ -2030,11 +2030,14 @@ zk_status fitAmc(zk_context* ctx, const ViewT* plan, const double* normals, size
     if (numBermudans == 0) return ZK_OK;
     upload(*B, ctx, true, normals, streams);
     execute(*B);
-    // Bermudans in groups whose realised values after each exercise (nE rows each) take at most 2 GB; the continuations'
-    // swap rates (two regressors) at most 512 MB of rows at a time.
+    // The realised values (rows of nP doubles) and the swap rates (two regressors) take at most kFitScratch bytes each, or as
+    // much as the states themselves (eight Bermudans on a million paths in one group: 6.0 ms against 7.0), and less under an
+    // explicit row budget.  A Bermudan whose realised values after each exercise fit keeps them, and its
+    // continuations, which nothing waits for, run after the chain; else it has one row, updated in place, and a date's
+    // continuation runs in the chain as soon as the exercises after it are in the row.  Bermudans go in groups that fit.
+    // Where the device has not even that much left, one Bermudan and one continuation at a time.
+    constexpr size_t kFitScratch = size_t(256) << 20;
     const size_t rowBytes = static_cast<size_t>(P.nP) * 8;
-    const size_t group = std::max<size_t>(1, std::min<size_t>(numBermudans, (size_t(2) << 30) / (rowBytes * maxE)));
-    const uint32_t contAtOnce = static_cast<uint32_t>(std::max<size_t>(1, std::min<size_t>(any2 ? (size_t(512) << 20) / rowBytes : 65535, 65535)));
     struct FitLaunch {
       uint32_t first, count;
       bool gram, dates;  // dates: items of `shared`
@@ -2042,88 +2045,109 @@ zk_status fitAmc(zk_context* ctx, const ViewT* plan, const double* normals, size
     std::vector<FitItem> items;
     std::vector<FitDate> shared;
     std::vector<FitLaunch> launches;
-    for (size_t b0 = 0; b0 < numBermudans; b0 += group) {
-      const size_t b1 = std::min(numBermudans, b0 + group);
-      auto realisedRow = [&](size_t b, uint32_t s) { return s == 0 ? kNoRow : static_cast<uint32_t>((b - b0) * maxE + s - 1); };
-      auto swapRow = [&](size_t b, uint32_t s) { return static_cast<uint32_t>((b - b0) * 2 + (s & 1u)); };
-      // The chain, all Bermudans of the group in step: step s fits the policy of exercise nE - 1 - s on the realised values
-      // after the s later ones; one more step leaves those after the first exercise.
-      for (uint32_t s = 0; s <= maxE; ++s) {
-        const uint32_t first = static_cast<uint32_t>(items.size());
-        bool fits = false;
-        for (size_t b = b0; b < b1; ++b) {
-          const uint32_t nE = static_cast<uint32_t>(decide[b].size());
-          if (nE == 0 || s > nE) continue;
-          FitItem I{};
-          const uint32_t k = nE - 1 - s;  // s == nE: only the update
-          const bool fit = s < nE;
-          I.date = fit ? decide[b][k].second : 0u, I.eRow = fit ? eRow[b] + k : kNoRow, I.slot = fit ? slotBase[b] + k : kNoRow;
-          I.degree = degrees[b], I.twoD = twoD[b] > 0 ? 1u : 0u;
-          I.prevSlot = s > 0 ? slotBase[b] + k + 1 : kNoRow, I.prevDate = s > 0 ? decide[b][k + 1].second : 0u;
-          I.prevERow = s > 0 ? eRow[b] + k + 1 : 0u;
-          I.realisedIn = s > 0 ? realisedRow(b, s - 1) : kNoRow, I.realisedOut = realisedRow(b, s);
-          I.swapRow = swapRow(b, s), I.prevSwapRow = swapRow(b, s + 1);
-          if (fit && I.twoD) I.bonds = coterm.at(decide[b][k].first);
-          items.push_back(I);
-          fits = fits || fit;
-        }
-        std::stable_partition(items.begin() + first, items.end(), [](const FitItem& I) { return I.slot != kNoRow; });
-        if (items.size() > first) launches.push_back({first, static_cast<uint32_t>(items.size()) - first, fits, false});
-      }
-      // The continuations: on a date whose next exercise is k the realised values after exercise k's policy.
-      uint32_t first = static_cast<uint32_t>(items.size());
-      const size_t firstDate = shared.size();
-      std::map<std::pair<uint32_t, uint32_t>, size_t> open;  // (date, degree): its item with room
-      for (size_t b = b0; b < b1; ++b) {
-        const uint32_t nE = static_cast<uint32_t>(decide[b].size());
-        for (uint32_t i = 0; i < cont[b].size(); ++i) {
-          const uint32_t jc = cont[b][i].first;
-          uint32_t k = 0;
-          while (k < nE && decide[b][k].second <= jc) ++k;
-          if (k == nE) continue;  // no exercise ahead
-          if (twoD[b] <= 0) {
-            auto [at, fresh] = open.try_emplace({jc, degrees[b]}, shared.size());
-            if (fresh || shared[at->second].count == static_cast<uint32_t>(kFitShared)) {
-              at->second = shared.size();
-              shared.push_back({jc, 0u, degrees[b], 0u, {}, {}});
-            }
-            FitDate& T = shared[at->second];
-            T.slot[T.count] = slotBase[b] + nE + i, T.realisedIn[T.count++] = realisedRow(b, nE - k);
-            continue;
-          }
-          FitItem I{};
-          I.date = jc, I.eRow = kNoRow, I.slot = slotBase[b] + nE + i, I.degree = degrees[b], I.twoD = twoD[b] > 0 ? 1u : 0u;
-          I.realisedIn = realisedRow(b, nE - k), I.realisedOut = kNoRow, I.prevSlot = kNoRow;
-          I.swapRow = static_cast<uint32_t>(2 * group + (items.size() - first));
-          if (I.twoD) I.bonds = coterm.at(cont[b][i].second);
-          items.push_back(I);
-          if (items.size() - first == contAtOnce) {
-            launches.push_back({first, contAtOnce, true, false});
-            first = static_cast<uint32_t>(items.size());
-          }
-        }
-      }
-      if (items.size() > first) launches.push_back({first, static_cast<uint32_t>(items.size()) - first, true, false});
-      for (size_t at = firstDate; at < shared.size(); at += 65535)
-        launches.push_back({static_cast<uint32_t>(at), static_cast<uint32_t>(std::min<size_t>(shared.size() - at, 65535)), true, true});
-    }
     // CTAs per regression, at least a path per thread: a step of the chain in about one wave (its CTAs are few and short),
     // the continuations in two.
     auto chunksOf = [&](uint32_t count, bool dates) {
       return std::max(1u, std::min({(P.nP + 255u) / 256u, (148u * (dates ? 8u : 4u) + count - 1) / count, 296u}));
     };
-    uint32_t maxItems = 1;
-    size_t parts = 1;
-    for (const auto& l : launches) maxItems = std::max(maxItems, l.count), parts = std::max<size_t>(parts, static_cast<size_t>(l.count) * chunksOf(l.count, l.dates));
-    // Device scratch: one image of the items and bonds, then the records, counters, partials, realised values and swap rates.
-    size_t off = 0;
+    size_t off = 0, oItems = 0, oBonds = 0, oShared = 0, imageBytes = 0, oFit = 0, oCount = 0, zeroEnd = 0, oPart = 0, oRealised = 0, oSwap = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off = alignUp(off + std::max<size_t>(bytes, 16)); return o; };
-    const size_t oItems = take(items.size() * sizeof(FitItem)), oBonds = take(bonds.size() * sizeof(double4)), oShared = take(shared.size() * sizeof(FitDate));
-    const size_t imageBytes = off;
-    const size_t oFit = take(static_cast<size_t>(slots) * kFitOut * 8), oCount = take(maxItems * 4), zeroEnd = off;
-    const size_t oPart = take(parts * kFitSums * 8), oRealised = take(group * maxE * rowBytes);
-    const size_t oSwap = take(any2 ? (2 * group + std::min<size_t>(contAtOnce, items.size())) * rowBytes : 0);
+    auto layOut = [&](size_t bytes) {
+      items.clear(), shared.clear(), launches.clear(), off = 0;
+      const size_t atMost = bytes / rowBytes;  // rows
+      const bool inPlace = atMost < maxE;
+      const uint32_t each = inPlace ? 1u : maxE;  // rows per Bermudan
+      const size_t group = std::max<size_t>(1, std::min<size_t>(numBermudans, atMost / each));
+      const uint32_t contAtOnce = static_cast<uint32_t>(std::max<size_t>(1, std::min<size_t>(any2 ? atMost : 65535, 65535)));
+      for (size_t b0 = 0; b0 < numBermudans; b0 += group) {
+        const size_t b1 = std::min(numBermudans, b0 + group);
+        // the row of the realised values after the s last policies
+        auto realisedRow = [&](size_t b, uint32_t s) { return s == 0 ? kNoRow : static_cast<uint32_t>((b - b0) * each + (inPlace ? 0 : s - 1)); };
+        auto swapRow = [&](size_t b, uint32_t s) { return static_cast<uint32_t>((b - b0) * 2 + (s & 1u)); };
+        // The continuations whose realised values are those after the last s policies (kNoRow: all): on a date whose next
+        // exercise is k, those after exercise k's policy.
+        auto continuations = [&](uint32_t s) {
+          uint32_t first = static_cast<uint32_t>(items.size());
+          const size_t firstDate = shared.size();
+          std::map<std::pair<uint32_t, uint32_t>, size_t> open;  // (date, degree): its item with room
+          for (size_t b = b0; b < b1; ++b) {
+            const uint32_t nE = static_cast<uint32_t>(decide[b].size());
+            for (uint32_t i = 0; i < cont[b].size(); ++i) {
+              const uint32_t jc = cont[b][i].first;
+              uint32_t k = 0;
+              while (k < nE && decide[b][k].second <= jc) ++k;
+              if (k == nE || (s != kNoRow && nE - k != s)) continue;  // no exercise ahead; another step's
+              if (twoD[b] <= 0) {
+                auto [at, fresh] = open.try_emplace({jc, degrees[b]}, shared.size());
+                if (fresh || shared[at->second].count == static_cast<uint32_t>(kFitShared)) {
+                  at->second = shared.size();
+                  shared.push_back({jc, 0u, degrees[b], 0u, {}, {}});
+                }
+                FitDate& T = shared[at->second];
+                T.slot[T.count] = slotBase[b] + nE + i, T.realisedIn[T.count++] = realisedRow(b, nE - k);
+                continue;
+              }
+              FitItem I{};
+              I.date = jc, I.eRow = kNoRow, I.slot = slotBase[b] + nE + i, I.degree = degrees[b], I.twoD = 1u;
+              I.realisedIn = realisedRow(b, nE - k), I.realisedOut = kNoRow, I.prevSlot = kNoRow;
+              I.swapRow = static_cast<uint32_t>(2 * group + (items.size() - first));
+              I.bonds = coterm.at(cont[b][i].second);
+              items.push_back(I);
+              if (items.size() - first == contAtOnce) {
+                launches.push_back({first, contAtOnce, true, false});
+                first = static_cast<uint32_t>(items.size());
+              }
+            }
+          }
+          if (items.size() > first) launches.push_back({first, static_cast<uint32_t>(items.size()) - first, true, false});
+          for (size_t at = firstDate; at < shared.size(); at += 65535)
+            launches.push_back({static_cast<uint32_t>(at), static_cast<uint32_t>(std::min<size_t>(shared.size() - at, 65535)), true, true});
+        };
+        // The chain, all Bermudans of the group in step: step s fits the policy of exercise nE - 1 - s on the realised values
+        // after the s later ones; one more step leaves those after the first exercise.
+        for (uint32_t s = 0; s <= maxE; ++s) {
+          const uint32_t first = static_cast<uint32_t>(items.size());
+          bool fits = false;
+          for (size_t b = b0; b < b1; ++b) {
+            const uint32_t nE = static_cast<uint32_t>(decide[b].size());
+            if (nE == 0 || s > nE) continue;
+            FitItem I{};
+            const uint32_t k = nE - 1 - s;  // s == nE: only the update
+            const bool fit = s < nE;
+            I.date = fit ? decide[b][k].second : 0u, I.eRow = fit ? eRow[b] + k : kNoRow, I.slot = fit ? slotBase[b] + k : kNoRow;
+            I.degree = degrees[b], I.twoD = twoD[b] > 0 ? 1u : 0u;
+            I.prevSlot = s > 0 ? slotBase[b] + k + 1 : kNoRow, I.prevDate = s > 0 ? decide[b][k + 1].second : 0u;
+            I.prevERow = s > 0 ? eRow[b] + k + 1 : 0u;
+            I.realisedIn = s > 0 ? realisedRow(b, s - 1) : kNoRow, I.realisedOut = realisedRow(b, s);
+            I.swapRow = swapRow(b, s), I.prevSwapRow = swapRow(b, s + 1);
+            if (fit && I.twoD) I.bonds = coterm.at(decide[b][k].first);
+            items.push_back(I);
+            fits = fits || fit;
+          }
+          std::stable_partition(items.begin() + first, items.end(), [](const FitItem& I) { return I.slot != kNoRow; });
+          if (items.size() > first) launches.push_back({first, static_cast<uint32_t>(items.size()) - first, fits, false});
+          if (inPlace && s > 0) continuations(s);
+        }
+        if (!inPlace) continuations(kNoRow);
+      }
+      uint32_t maxItems = 1;
+      size_t parts = 1;
+      for (const auto& l : launches) maxItems = std::max(maxItems, l.count), parts = std::max<size_t>(parts, static_cast<size_t>(l.count) * chunksOf(l.count, l.dates));
+      // Device scratch: one image of the items and bonds, then the records, counters, partials, realised values and swap rates.
+      oItems = take(items.size() * sizeof(FitItem)), oBonds = take(bonds.size() * sizeof(double4)), oShared = take(shared.size() * sizeof(FitDate));
+      imageBytes = off;
+      oFit = take(static_cast<size_t>(slots) * kFitOut * 8), oCount = take(maxItems * 4), zeroEnd = off;
+      oPart = take(parts * kFitSums * 8), oRealised = take(group * each * rowBytes);
+      oSwap = take(any2 ? (2 * group + std::min<size_t>(contAtOnce, items.size())) * rowBytes : 0);
+    };
+    const size_t most = std::max(kFitScratch, B->totalBytes);
+    layOut(ctx->rowBudget > 0 ? std::min<size_t>(most, ctx->rowBudget) : most);
     dmem = takeBlock(ctx, off, dmemBytes);
+    if (!dmem) {
+      cudaGetLastError();
+      layOut(0);
+      dmem = takeBlock(ctx, off, dmemBytes);
+    }
     if (!dmem) throw fail(ZK_ERR_OUT_OF_MEMORY, "AMC fit: %zu bytes of device memory", off);
     unsigned char* d = static_cast<unsigned char*>(dmem);
     std::vector<unsigned char> image(imageBytes, 0);
