@@ -30,21 +30,26 @@ constexpr int kBins = 4096;
 constexpr int kCap = 4096;
 constexpr int kMaxRounds = 16;
 constexpr int kHistBins = 3072;  // the reference's histogram-request limit (kPfeBins)
-constexpr int kGather = 4096;    // values kept from the bins the sample points at
+constexpr int kPool = 8192;      // values kept from the window the sample points at
+// A window of the sample holds about 16 times its values in the row, give or take a few hundred, spread over the warps'
+// shares of kPool: the pass is made where it expects to keep at most this many.  (With a pool of half the size, and the pass
+// made whether it fitted or not, 97.5% of a million paths took 1.96 ms in four netting sets and 0.55 now, 99% of two million
+// 3.10 and 0.96, a median of 500,000 in twelve 4.18 and 3.95.)
+constexpr uint32_t kWindowKept = 7000;
 
 template <typename R>
 struct RowSmem {
   union {  // the histogram is read up to the choice of the bins; the candidates are gathered after it
     uint32_t hist[kBins];
     R cand[kCap];
+    R pool[kPool];
   };
-  R gath[kGather];
   alignas(8) uint32_t digits[264];
   double dsum[kRowWarps];
   R rmin[kRowWarps], rmax[kRowWarps];
   uint32_t candCount;
   uint32_t usum[kRowWarps], ukept[kRowWarps];
-  uint32_t pick[4];
+  uint32_t pick[5];
   double flo[kMaxRounds], finvw[kMaxRounds];
   uint32_t fb0[kMaxRounds], fb1[kMaxRounds];
 };
@@ -158,16 +163,16 @@ __device__ __forceinline__ void forEachValue(const R* X, uint32_t nP, bool pos, 
 }
 
 // Values of the row (through max(x, 0) when pos) below `from` counted, and those in [from, to] kept: each warp appends to its
-// own kGatherWarp slots by ballots (an atomic with its returned position stalls the warp at nearly every vector).  Returns
-// this thread's count below; `kept` the warp's values in the window, more than kGatherWarp when they did not fit.
-constexpr uint32_t kGatherWarp = kGather / kRowWarps;
+// own kPoolWarp slots by ballots (an atomic with its returned position stalls the warp at nearly every vector).  Returns
+// this thread's count below; `kept` the warp's values in the window, more than kPoolWarp when they did not fit.
+constexpr uint32_t kPoolWarp = kPool / kRowWarps;
 template <typename R>
-__device__ __forceinline__ uint32_t windowPass(const R* X, uint32_t nP, bool pos, R from, R to, R* gath, uint32_t& kept) {
+__device__ __forceinline__ uint32_t windowPass(const R* X, uint32_t nP, bool pos, R from, R to, R* pool, uint32_t& kept) {
   constexpr uint32_t kVec = 16 / sizeof(R), kDeep = 4;
   const uint32_t tid = threadIdx.x, below = (1u << (tid & 31u)) - 1u;
   const RowVectors<R> V = vectorsOf(X, nP);
   const R* body = X + V.head;
-  R* mine = gath + (tid >> 5) * kGatherWarp;
+  R* mine = pool + (tid >> 5) * kPoolWarp;
   uint32_t under = 0, n = 0;
   auto take = [&](const R (&v)[kVec], bool ok) {
     bool in[kVec], any = false;
@@ -182,7 +187,7 @@ __device__ __forceinline__ uint32_t windowPass(const R* X, uint32_t nP, bool pos
 #pragma unroll
       for (uint32_t e = 0; e < kVec; ++e) {
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, in[e]), at = n + __popc(m & below);
-        if (in[e] && at < kGatherWarp) mine[at] = pos ? fmax(v[e], R(0)) : v[e];
+        if (in[e] && at < kPoolWarp) mine[at] = pos ? fmax(v[e], R(0)) : v[e];
         n += __popc(m);
       }
     }
@@ -213,7 +218,7 @@ __device__ __forceinline__ uint32_t windowPass(const R* X, uint32_t nP, bool pos
     const bool ok = tid < loose, up = x >= from, in = ok && up && x <= to;
     under = before + (ok && !up ? 1u : 0u);
     const uint32_t m = __ballot_sync(0xFFFFFFFFu, in), at = n + __popc(m & below);
-    if (in && at < kGatherWarp) mine[at] = x;
+    if (in && at < kPoolWarp) mine[at] = x;
     n += __popc(m);
   }
   kept = n;
@@ -281,8 +286,8 @@ __device__ __forceinline__ uint32_t sampleHistogram(const R* X, uint32_t nP, boo
 }
 
 // The bins of ranks k and k1 >= k among the candidates counted in s.hist, `below` values ranking under bin 0:
-// pick = {bin of k, bin of k1, values under k's bin, count of k's bin}, as a walk over the bins in order would
-// find them.  One warp: lane l owns bins [128 l, 128 l + 128) (read skewed by l, free of bank conflicts), a
+// pick = {bin of k, bin of k1, values under k's bin, count of k's bin, values up to k1's bin}, as a walk over the bins in
+// order would find them.  One warp: lane l owns bins [128 l, 128 l + 128) (read skewed by l, free of bank conflicts), a
 // warp scan of the lanes' counts finds the lane holding each rank, and that lane walks its own bins.
 template <typename R>
 __device__ __forceinline__ void locateRanks(RowSmem<R>& s, uint32_t below, uint32_t k, uint32_t k1, uint32_t lane) {
@@ -319,7 +324,7 @@ __device__ __forceinline__ void locateRanks(RowSmem<R>& s, uint32_t below, uint3
     uint32_t b1, under1;
     walk(k1, b1, under1);
     if (!m1) b1 = kBins - 1;
-    s.pick[1] = b1;
+    s.pick[1] = b1, s.pick[4] = under1 + s.hist[b1];
   }
 }
 
@@ -328,12 +333,13 @@ __device__ __forceinline__ unsigned long long orderKey(double v) { return double
 __device__ __forceinline__ float fromKey(uint32_t k) { return keyFloat(k); }
 __device__ __forceinline__ double fromKey(unsigned long long k) { return keyDouble(k); }
 
-// The values of ranks r and r1 (r or r + 1, below n) among n values in shared memory, by their order-preserving integer keys:
+// The values of ranks r and r1 (r or r + 1, below n) among n values, by their order-preserving integer keys (each(f) calls
+// f(value) for this thread's share of the values):
 // a radix selection of 8 bits a pass finds rank r's value, and the next one is that value again or the least above it.  (A
 // bitonic sort of 2,048 values took 66 barriers and 45 us, four passes take 4.)  scratch: 256 + 8 words; every thread gets
 // both values.
-template <typename R>
-__device__ __forceinline__ void selectRanks(const R* a, uint32_t n, uint32_t r, uint32_t r1, uint32_t* scratch, R& v, R& v1) {
+template <typename R, typename Each>
+__device__ __forceinline__ void selectRanks(Each&& each, uint32_t n, uint32_t r, uint32_t r1, uint32_t* scratch, R& v, R& v1) {
   using Key = decltype(orderKey(R(0)));
   constexpr int kBits = 8 * static_cast<int>(sizeof(R));
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -343,10 +349,10 @@ __device__ __forceinline__ void selectRanks(const R* a, uint32_t n, uint32_t r, 
   for (int shift = kBits - 8; shift >= 0; shift -= 8) {
     scratch[tid] = 0;
     __syncthreads();
-    for (uint32_t i = tid; i < n; i += kRowThreads) {
-      const Key key = orderKey(a[i]);
+    each([&](R x) {
+      const Key key = orderKey(x);
       if ((key & mask) == prefix) atomicAdd(&scratch[static_cast<uint32_t>(key >> shift) & 255u], 1u);
-    }
+    });
     __syncthreads();
     // The digit whose running count passes the rank: each thread scans its digit's count over the CTA.
     const uint32_t own = scratch[tid];
@@ -373,10 +379,10 @@ __device__ __forceinline__ void selectRanks(const R* a, uint32_t n, uint32_t r, 
   if (r1 == r || rank + 1 < same) return;  // rank r + 1 is the same value
   // The least value above: its key minimum over the CTA, two words for a double's.
   Key best = ~static_cast<Key>(0);
-  for (uint32_t i = tid; i < n; i += kRowThreads) {
-    const Key key = orderKey(a[i]);
+  each([&](R x) {
+    const Key key = orderKey(x);
     if (key > prefix && key < best) best = key;
-  }
+  });
 #pragma unroll
   for (uint32_t o = 16; o > 0; o >>= 1) {
     const Key t = __shfl_xor_sync(0xFFFFFFFFu, best, o);
@@ -486,7 +492,8 @@ __global__ void __launch_bounds__(kRowThreads, 6) rowStatsKernel(const RowJob<R>
   // counts the row's values under the bins of sample ranks k_s -+ (3 sd + 4) and keeps the values in them, and when the
   // ranks fall among those (the counts prove it) they are selected there.  No histogram of the row: a shared-memory
   // atomic per value had bound the pass (100 netting sets, 121 rows each of 250,000 paths: 5.05 ms, 33,333 odd paths x 12
-  // 282 us; now 3.97 ms and 156 us).  Else the rounds below.
+  // 282 us; now 3.97 ms and 156 us).  A window too full for the pool (a median of many paths, equal values) would waste the
+  // pass, 4 to 20% of such a row: the sample's count says so beforehand.  Else the rounds below.
   if (sampled) {
     const double dlo0 = static_cast<double>(lo), invw0 = scaleOf(lo, hi);
     for (uint32_t b = tid; b < kBins; b += kRowThreads) s.hist[b] = 0;
@@ -499,31 +506,28 @@ __global__ void __launch_bounds__(kRowThreads, 6) rowStatsKernel(const RowJob<R>
     const uint32_t rlo = static_cast<uint32_t>(fmax(ks - sd, 0.0)), rhi = static_cast<uint32_t>(fmin(ks + sd + 1.0, ns - 1.0));
     if (tid < 32) locateRanks(s, 0u, rlo, rhi, tid);
     __syncthreads();
-    const uint32_t winLo = s.pick[0], winHi = s.pick[1];
-    // The window's edges as values, half a bin outside the bins' centres (the ends open): any edges serve, the counts decide.
-    const R from = winLo == 0 ? R(-INFINITY) : static_cast<R>(dlo0 + (static_cast<double>(winLo) - 0.5) / invw0);
-    const R to = winHi + 1 >= static_cast<uint32_t>(kBins) ? R(INFINITY) : static_cast<R>(dlo0 + (static_cast<double>(winHi) + (sizeof(R) == 4 ? 0.5 : 1.0)) / invw0);
-    uint32_t kept;
-    uint32_t under = windowPass(X, nP, pos, from, to, s.gath, kept);
-    under = __reduce_add_sync(0xFFFFFFFFu, under);
-    __syncthreads();
-    if ((tid & 31u) == 0) s.usum[tid >> 5] = under, s.ukept[tid >> 5] = kept;
-    __syncthreads();
-    uint32_t at = 0, total = 0;
-    bool fit = true;
-    under = 0;
-    for (int w = 0; w < kRowWarps; ++w) {
-      if (w == static_cast<int>(tid >> 5)) at = total;
-      fit = fit && s.ukept[w] <= kGatherWarp;
-      under += s.usum[w], total += s.ukept[w];
-    }
-    if (fit && under <= k && k1 - under < total) {  // the ranks are among the kept values: together in s.cand, and selected
-      for (uint32_t i = tid & 31u; i < kept; i += 32) s.cand[at + i] = s.gath[(tid >> 5) * kGatherWarp + i];
+    const uint32_t winLo = s.pick[0], winHi = s.pick[1], sampledIn = s.pick[4] - s.pick[2];
+    if (static_cast<uint64_t>(sampledIn) * nP <= static_cast<uint64_t>(kWindowKept) * ns) {
+      // The window's edges as values, half a bin outside the bins' centres (the ends open): any edges serve, the counts decide.
+      const R from = winLo == 0 ? R(-INFINITY) : static_cast<R>(dlo0 + (static_cast<double>(winLo) - 0.5) / invw0);
+      const R to = winHi + 1 >= static_cast<uint32_t>(kBins) ? R(INFINITY) : static_cast<R>(dlo0 + (static_cast<double>(winHi) + (sizeof(R) == 4 ? 0.5 : 1.0)) / invw0);
+      uint32_t kept;
+      uint32_t under = windowPass(X, nP, pos, from, to, s.pool, kept);
+      under = __reduce_add_sync(0xFFFFFFFFu, under);
+      if ((tid & 31u) == 0) s.usum[tid >> 5] = under, s.ukept[tid >> 5] = kept;
       __syncthreads();
-      selectRanks(s.cand, total, k - under, k1 - under, s.digits, vk, vk1);
-      done = true;
+      uint32_t total = 0;
+      bool fit = true;
+      under = 0;
+      for (int w = 0; w < kRowWarps; ++w) fit = fit && s.ukept[w] <= kPoolWarp, under += s.usum[w], total += s.ukept[w];
+      if (fit && under <= k && k1 - under < total) {  // the ranks are among the kept values
+        selectRanks([&](auto&& f) {  // each warp its own
+          for (uint32_t i = tid & 31u; i < kept; i += 32) f(s.pool[(tid >> 5) * kPoolWarp + i]);
+        }, total, k - under, k1 - under, s.digits, vk, vk1);
+        done = true;
+      }
+      __syncthreads();
     }
-    __syncthreads();
   }
   while (!done) {
     if (rounds >= static_cast<int>(maxRounds)) {
@@ -575,7 +579,9 @@ __global__ void __launch_bounds__(kRowThreads, 6) rowStatsKernel(const RowJob<R>
       });
       __syncthreads();
       const uint32_t n = s.candCount;
-      selectRanks(s.cand, n, k - below0, min(k1 - below0, n - 1), s.digits, vk, vk1);
+      selectRanks([&](auto&& f) {
+        for (uint32_t i = tid; i < n; i += kRowThreads) f(s.cand[i]);
+      }, n, k - below0, min(k1 - below0, n - 1), s.digits, vk, vk1);
       done = true;
     } else {
       if (tid == 0) s.flo[rounds] = dlo, s.finvw[rounds] = invw, s.fb0[rounds] = b0, s.fb1[rounds] = b0;
