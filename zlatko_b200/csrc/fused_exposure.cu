@@ -5,8 +5,9 @@
 // src/gpu/fused_reference.cpp:198-422), organised for a B200 and for books of many netting sets:
 //
 //   simulateKernel   producer warps draw the counter-based normals and correlate them, ahead of the warps that
-//                    step Hull-White, the lognormal assets and the CIR++ intensities once per date, writing
-//                    the factor state (x, D, S, Q; lnS and y when probes read them) path-major to HBM.
+//                    step Hull-White, the lognormal assets and the CIR++ intensities once per date (simulateWalkKernel:
+//                    a thread does all of a path or pair, where those fill the GPU), writing the factor state (x, D, S,
+//                    Q; lnS and y when probes read them) path-major to HBM.
 //                    Every netting set of the launch reuses it: the reference re-simulates per plan.
 //                    Only factors are stored, never the paths x dates x trades value cube.
 //   revalueKernel    one CTA per (tile of kTile paths, netting set).  CTA ids run tile-major, so the
@@ -203,6 +204,148 @@ __device__ __forceinline__ void stPaths(R* p, const R (&v)[PPT]) {
   }
 }
 
+namespace {
+
+// The Brownian-bridge coefficients of the CIR sub-steps, the same for every path: the CTA computes them once.
+template <typename R>
+__device__ __forceinline__ void bridgeTable(const ScenarioArgs<R>& sc, R* bridge) {
+  const uint32_t nB = sc.substeps - 1;
+  for (uint32_t jj = threadIdx.x + 1; jj < sc.nT; jj += blockDim.x) {
+    const R dt = sc.steps[static_cast<size_t>(jj) * sc.stepStride + 6], h = dt / static_cast<R>(sc.substeps);
+    R remT = dt;
+    for (uint32_t q = 0; q < nB; ++q) {
+      bridge[(static_cast<size_t>(jj) * nB + q) * 2] = h / remT;
+      bridge[(static_cast<size_t>(jj) * nB + q) * 2 + 1] = rsqrt_(fmax(h * (remT - h) / remT, R(0)));
+      remT -= h;
+    }
+  }
+  __syncthreads();
+}
+
+// The rates and assets of a thread's PPL paths.  The deflator's exponent -sum of the integrated short rate accumulates in
+// double precision in both modes (the reference's kernel sums it in single precision, fused_kernels.cpp:250-253);
+// D = exp(lnD) is then taken in R.
+template <typename R, int PPL>
+struct RateState {
+  R x[PPL], D[PPL], S[4][PPL], lnS[4][PPL], xf[2][PPL];  // xf: stochastic foreign short-rate states of assets 0 and 1
+  double lnD[PPL];
+  __device__ __forceinline__ explicit RateState(const ScenarioArgs<R>& sc) {
+#pragma unroll
+    for (int i = 0; i < PPL; ++i) {
+      x[i] = R(0), D[i] = R(1), lnD[i] = 0.0, xf[0][i] = xf[1][i] = R(0);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) S[a][i] = sc.spots[a], lnS[a][i] = R(0);
+    }
+  }
+};
+
+// One date's step, from the drivers at buf[m * cols].
+template <typename R, int PPL, uint32_t cols>
+__device__ __forceinline__ void stepRates(const ScenarioArgs<R>& sc, uint32_t j, const R* buf, const R (&sign)[PPL], RateState<R, PPL>& st) {
+  const R* step = sc.steps + static_cast<size_t>(j) * sc.stepStride;
+  const R s0 = __ldg(step), s1 = __ldg(step + 1), s2 = __ldg(step + 2), s3 = __ldg(step + 3), s4 = __ldg(step + 4), s5 = __ldg(step + 5);
+  const R w0 = buf[0], zI = buf[sc.nCorr * cols];
+  R integratedRate[PPL], carry[4][PPL];
+#pragma unroll
+  for (int i = 0; i < PPL; ++i) {
+    const R w = sign[i] * w0, z = sign[i] * zI;
+    integratedRate[i] = fma(s3, z, fma(st.x[i], s5, s2 * w)) + s4;
+    st.x[i] = fma(st.x[i], s0, s1 * w);
+    st.lnD[i] -= static_cast<double>(integratedRate[i]);
+    st.D[i] = rexp(static_cast<R>(st.lnD[i]));
+  }
+  // Stochastic foreign rates: the exact Hull-White step of x_f (with its quanto drift) and of its integral, on
+  // driver 1 + nA + nC + f and the independent normal nCorr + 1 + f; the asset's carry is then the simulated
+  // integral of r_f instead of the deterministic one.
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int i = 0; i < PPL; ++i) carry[a][i] = __ldg(step + 8 + a);
+#pragma unroll
+  for (int f = 0; f < 2; ++f) {
+    if (static_cast<uint32_t>(f) < sc.nF) {
+      const R* fs = step + kStepStride + 8 * f;
+      const R wf0 = buf[(1 + sc.nA + sc.nC + f) * cols], zf0 = buf[(sc.nCorr + 1 + f) * cols];
+#pragma unroll
+      for (int i = 0; i < PPL; ++i) {
+        const R wf = sign[i] * wf0, zf = sign[i] * zf0;
+        carry[f][i] = fma(__ldg(fs + 3), zf, fma(st.xf[f][i], __ldg(fs + 5), __ldg(fs + 2) * wf)) + __ldg(fs + 4) + __ldg(fs + 7);
+        st.xf[f][i] = fma(st.xf[f][i], __ldg(fs), __ldg(fs + 1) * wf) + __ldg(fs + 6);
+      }
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    if (static_cast<uint32_t>(a) < sc.nA) {
+      const R drift = __ldg(step + 16 + a), vol = __ldg(step + 12 + a), wa = buf[(1 + a) * cols];
+#pragma unroll
+      for (int i = 0; i < PPL; ++i) {
+        st.lnS[a][i] = st.lnS[a][i] + fma(vol, sign[i] * wa, integratedRate[i] - carry[a][i] - drift);
+        st.S[a][i] = sc.spots[a] * rexp(st.lnS[a][i]);
+      }
+    }
+  }
+}
+
+template <typename R, int PPL, typename Put>
+__device__ __forceinline__ void writeRates(const ScenarioArgs<R>& sc, const CubeArgs<R>& cb, uint32_t j, const RateState<R, PPL>& st, const Put& put) {
+  put(0, j, st.x);
+  put(1, j, st.D);
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+    if (static_cast<uint32_t>(a) < sc.nA) put(cb.fS + a, j, st.S[a]);
+#pragma unroll
+  for (int f = 0; f < 2; ++f)
+    if (static_cast<uint32_t>(f) < sc.nF) put(cb.fXf + f, j, st.xf[f]);
+  if (cb.probes)
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+      if (static_cast<uint32_t>(a) < sc.nA) put(cb.fLnS + a, j, st.lnS[a]);
+}
+
+// One CIR++ intensity of a thread's PPL paths, and where a date's drivers hold its increments (values from the column's first).
+template <typename R, int PPL>
+struct CreditState {
+  R y[PPL], Y[PPL], Q[PPL], kappa, theta, xi;
+  uint32_t at, last;
+  __device__ __forceinline__ CreditState(const ScenarioArgs<R>& sc, const SimLayout& L, uint32_t c, uint32_t cols)
+      : kappa(sc.cir[4 * c]), theta(sc.cir[4 * c + 1]), xi(sc.cir[4 * c + 2]),
+        at((sc.nCorr + 1 + sc.nF + c * (sc.substeps - 1)) * cols), last((L.need + c) * cols) {
+#pragma unroll
+    for (int i = 0; i < PPL; ++i) y[i] = sc.cir[4 * c + 3], Y[i] = R(0), Q[i] = R(1);
+  }
+};
+
+template <typename R, int PPL, uint32_t cols>
+__device__ __forceinline__ void stepCredit(const ScenarioArgs<R>& sc, uint32_t c, uint32_t j, const R* buf, const R (&sign)[PPL],
+                                           CreditState<R, PPL>& st) {
+  const uint32_t nB = sc.substeps - 1;
+  const R* step = sc.steps + static_cast<size_t>(j) * sc.stepStride;
+  const R h = __ldg(step + 6) / static_cast<R>(sc.substeps), shift = __ldg(step + 20 + c);
+  auto subStep = [&](R dW0) {
+#pragma unroll
+    for (int i = 0; i < PPL; ++i) {
+      const R dW = sign[i] * dW0, yp = fmax(st.y[i], R(0));
+      const R yn = fma(st.xi * rsqrt_(yp), dW, fma(st.kappa * (st.theta - yp), h, st.y[i]));
+      st.Y[i] = fma(R(0.5) * (yp + fmax(yn, R(0))), h, st.Y[i]);
+      st.y[i] = yn;
+    }
+  };
+#pragma unroll 4
+  for (uint32_t s = 0; s < nB; ++s) subStep(buf[st.at + s * cols]);
+  subStep(buf[st.last]);
+#pragma unroll
+  for (int i = 0; i < PPL; ++i) st.Q[i] = rexp(-st.Y[i] - shift);
+}
+
+template <typename R, int PPL, typename Put>
+__device__ __forceinline__ void writeCredit(const CubeArgs<R>& cb, uint32_t c, uint32_t j, const CreditState<R, PPL>& st, const Put& put) {
+  put(cb.fQ + c, j, st.Q);
+  if (cb.probes) put(cb.fY + c, j, st.y);
+}
+
+}  // namespace
+
 // ---------------------------------------------------------------------------------------------
 // Risk factors of every path and date (the transitions of the reference's ScenarioGenerator:
 // hull_white.cpp:40-68, lognormal_asset.cpp:17-22, cir_intensity.cpp:49-66, in the statement order
@@ -215,8 +358,8 @@ __device__ __forceinline__ void stPaths(R* p, const R (&v)[PPT]) {
 // they are produced once per pair: with 32 streams a lane steps both paths of its stream (PPL = 2: two independent
 // chains of the CIR++ sub-steps' square roots, which bind), with 16 streams adjacent lanes share one and a producer pass
 // covers two dates.  Without pairs a stream is a path.
-// Before (one thread drew and stepped a path): 389 us at 2,000 paths x 121 dates, 4 factors, 1,159 us at 100,000 x 169,
-// 6 factors, 4,800 us at 500,000.  16 streams: 80, 991 and 4,433 us; 32: 108, 735 and 3,475 us.
+// Against one thread that draws and steps a path: 389 us at 2,000 paths x 121 dates, 4 factors, and 1,159 us at 100,000 x 169,
+// 6 factors; 16 streams take 80 and 991 us, 32 take 108 and 735.
 template <typename R, int PPL, uint32_t cols>
 __global__ void __launch_bounds__(kSimThreads, sizeof(R) == 4 ? 4 : 2) simulateKernel(const ScenarioArgs<R> sc, const CubeArgs<R> cb,
                                                                                      const SimLayout L) {
@@ -224,8 +367,7 @@ __global__ void __launch_bounds__(kSimThreads, sizeof(R) == 4 ? 4 : 2) simulateK
   R* ring = reinterpret_cast<R*>(simRaw);
   const uint32_t bufLen = L.dates * L.slots * cols;
   R* bridge = ring + 2 * static_cast<size_t>(bufLen);
-  // The Brownian-bridge coefficients of the CIR sub-steps are the same for every path: with L.table the CTA computes
-  // them once.
+  // bridgeTable in line: as a call it costs the credits' loops 3%.
   const uint32_t nB = sc.substeps - 1, nP = sc.nP, nT = sc.nT;
   if (L.table) {
     for (uint32_t jj = threadIdx.x + 1; jj < nT; jj += blockDim.x) {
@@ -284,82 +426,16 @@ __global__ void __launch_bounds__(kSimThreads, sizeof(R) == 4 ? 4 : 2) simulateK
     }
   };
   if (role == 0) {
-    // The deflator's exponent -sum of the integrated short rate accumulates in double precision in both modes (the
-    // reference's kernel sums it in single precision, fused_kernels.cpp:250-253); D = exp(lnD) is then taken in R.
-    R x[PPL], D[PPL], S[4][PPL], lnS[4][PPL], xf[2][PPL];  // xf: stochastic foreign short-rate states of assets 0 and 1
-    double lnD[PPL];
-#pragma unroll
-    for (int i = 0; i < PPL; ++i) {
-      x[i] = R(0), D[i] = R(1), lnD[i] = 0.0, xf[0][i] = xf[1][i] = R(0);
-#pragma unroll
-      for (int a = 0; a < 4; ++a) S[a][i] = sc.spots[a], lnS[a][i] = R(0);
-    }
-    auto write = [&](uint32_t j) {
-      put(0, j, x);
-      put(1, j, D);
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-        if (static_cast<uint32_t>(a) < sc.nA) put(cb.fS + a, j, S[a]);
-#pragma unroll
-      for (int f = 0; f < 2; ++f)
-        if (static_cast<uint32_t>(f) < sc.nF) put(cb.fXf + f, j, xf[f]);
-      if (cb.probes)
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-          if (static_cast<uint32_t>(a) < sc.nA) put(cb.fLnS + a, j, lnS[a]);
-    };
-    write(0);
+    RateState<R, PPL> st(sc);
+    writeRates<R, PPL>(sc, cb, 0, st, put);
     for (uint32_t b = 0; b <= blocks; ++b) {
       if (b > 0) {
         const uint32_t j0 = 1 + (b - 1) * L.dates, j1 = min(j0 + L.dates, nT);
         const R* buf = ring + ((b - 1) & 1u) * bufLen + col;
 #pragma unroll 1
         for (uint32_t j = j0; j < j1; ++j, buf += L.slots * cols) {
-          const R* step = sc.steps + static_cast<size_t>(j) * sc.stepStride;
-          const R s0 = __ldg(step), s1 = __ldg(step + 1), s2 = __ldg(step + 2), s3 = __ldg(step + 3), s4 = __ldg(step + 4),
-                  s5 = __ldg(step + 5);
-          const R w0 = buf[0], zI = buf[sc.nCorr * cols];
-          R integratedRate[PPL], carry[4][PPL];
-#pragma unroll
-          for (int i = 0; i < PPL; ++i) {
-            const R w = sign[i] * w0, z = sign[i] * zI;
-            integratedRate[i] = fma(s3, z, fma(x[i], s5, s2 * w)) + s4;
-            x[i] = fma(x[i], s0, s1 * w);
-            lnD[i] -= static_cast<double>(integratedRate[i]);
-            D[i] = rexp(static_cast<R>(lnD[i]));
-          }
-          // Stochastic foreign rates: the exact Hull-White step of x_f (with its quanto drift) and of its integral, on
-          // driver 1 + nA + nC + f and the independent normal nCorr + 1 + f; the asset's carry is then the simulated
-          // integral of r_f instead of the deterministic one.
-#pragma unroll
-          for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int i = 0; i < PPL; ++i) carry[a][i] = __ldg(step + 8 + a);
-#pragma unroll
-          for (int f = 0; f < 2; ++f) {
-            if (static_cast<uint32_t>(f) < sc.nF) {
-              const R* fs = step + kStepStride + 8 * f;
-              const R wf0 = buf[(1 + sc.nA + sc.nC + f) * cols], zf0 = buf[(sc.nCorr + 1 + f) * cols];
-#pragma unroll
-              for (int i = 0; i < PPL; ++i) {
-                const R wf = sign[i] * wf0, zf = sign[i] * zf0;
-                carry[f][i] = fma(__ldg(fs + 3), zf, fma(xf[f][i], __ldg(fs + 5), __ldg(fs + 2) * wf)) + __ldg(fs + 4) + __ldg(fs + 7);
-                xf[f][i] = fma(xf[f][i], __ldg(fs), __ldg(fs + 1) * wf) + __ldg(fs + 6);
-              }
-            }
-          }
-#pragma unroll
-          for (int a = 0; a < 4; ++a) {
-            if (static_cast<uint32_t>(a) < sc.nA) {
-              const R drift = __ldg(step + 16 + a), vol = __ldg(step + 12 + a), wa = buf[(1 + a) * cols];
-#pragma unroll
-              for (int i = 0; i < PPL; ++i) {
-                lnS[a][i] = lnS[a][i] + fma(vol, sign[i] * wa, integratedRate[i] - carry[a][i] - drift);
-                S[a][i] = sc.spots[a] * rexp(lnS[a][i]);
-              }
-            }
-          }
-          write(j);
+          stepRates<R, PPL, cols>(sc, j, buf, sign, st);
+          writeRates<R, PPL>(sc, cb, j, st, put);
         }
       }
       __syncthreads();
@@ -367,40 +443,63 @@ __global__ void __launch_bounds__(kSimThreads, sizeof(R) == 4 ? 4 : 2) simulateK
     return;
   }
   const uint32_t c = role - 1;  // this warp's credit
-  const R kappa = sc.cir[4 * c], theta = sc.cir[4 * c + 1], xi = sc.cir[4 * c + 2];
-  R y[PPL], Y[PPL], Q[PPL];
-#pragma unroll
-  for (int i = 0; i < PPL; ++i) y[i] = sc.cir[4 * c + 3], Y[i] = R(0), Q[i] = R(1);
-  put(cb.fQ + c, 0, Q);
-  if (cb.probes) put(cb.fY + c, 0, y);
-  const uint32_t at = (sc.nCorr + 1 + sc.nF + c * nB) * cols, last = (L.need + c) * cols;
+  CreditState<R, PPL> st(sc, L, c, cols);
+  writeCredit<R, PPL>(cb, c, 0, st, put);
   for (uint32_t b = 0; b <= blocks; ++b) {
     if (b > 0) {
       const uint32_t j0 = 1 + (b - 1) * L.dates, j1 = min(j0 + L.dates, nT);
       const R* buf = ring + ((b - 1) & 1u) * bufLen + col;
 #pragma unroll 1
       for (uint32_t j = j0; j < j1; ++j, buf += L.slots * cols) {
-        const R* step = sc.steps + static_cast<size_t>(j) * sc.stepStride;
-        const R h = __ldg(step + 6) / static_cast<R>(sc.substeps), shift = __ldg(step + 20 + c);
-        auto subStep = [&](R dW0) {
-#pragma unroll
-          for (int i = 0; i < PPL; ++i) {
-            const R dW = sign[i] * dW0, yp = fmax(y[i], R(0));
-            const R yn = fma(xi * rsqrt_(yp), dW, fma(kappa * (theta - yp), h, y[i]));
-            Y[i] = fma(R(0.5) * (yp + fmax(yn, R(0))), h, Y[i]);
-            y[i] = yn;
-          }
-        };
-#pragma unroll 4
-        for (uint32_t s = 0; s < nB; ++s) subStep(buf[at + s * cols]);
-        subStep(buf[last]);
-#pragma unroll
-        for (int i = 0; i < PPL; ++i) Q[i] = rexp(-Y[i] - shift);
-        put(cb.fQ + c, j, Q);
-        if (cb.probes) put(cb.fY + c, j, y);
+        stepCredit<R, PPL, cols>(sc, c, j, buf, sign, st);
+        writeCredit<R, PPL>(cb, c, j, st, put);
       }
     }
     __syncthreads();
+  }
+}
+
+// The same states by threads that each draw and step their PPL paths (2: an antithetic pair) date after date: where the paths
+// alone fill the GPU it is the faster one (launchSimulate has the rule and the times).  Its working set is a thread's drivers
+// of one date; what binds it is the issue of the normals and exponentials.
+template <typename R, int PPL>
+__global__ void __launch_bounds__(kSimThreads) simulateWalkKernel(const ScenarioArgs<R> sc, const CubeArgs<R> cb, const SimLayout L) {
+  extern __shared__ __align__(16) unsigned char simRaw[];
+  R* col = reinterpret_cast<R*>(simRaw) + threadIdx.x;
+  R* bridge = reinterpret_cast<R*>(simRaw) + static_cast<size_t>(L.slots) * kSimThreads;
+  if (L.table) bridgeTable(sc, bridge);
+  const uint32_t nP = sc.nP, p0 = (blockIdx.x * kSimThreads + threadIdx.x) * PPL;
+  if (p0 >= nP) return;
+  const uint32_t po = sc.pathMap ? sc.pathMap[p0] : p0, pathStream = sc.antithetic ? po >> 1u : po;
+  const uint32_t injectedStream = sc.nStreams > 0 ? min(pathStream, sc.nStreams - 1) : 0u;
+  const uint32_t stream = pcg(pcg(sc.seed) ^ pcg(pathStream + 0x9E3779B9u));
+  R sign[PPL];
+#pragma unroll
+  for (int i = 0; i < PPL; ++i) sign[i] = PPL == 2 ? (i == 0 ? R(1) : R(-1)) : sc.antithetic && (po & 1u) ? R(-1) : R(1);
+  auto put = [&](uint32_t field, uint32_t j, const R (&v)[PPL]) {
+    R* dst = cb.data + (static_cast<size_t>(field) * sc.nT + j) * nP + p0;
+    if (PPL == 2 && nP % 2u == 0u) {
+      stPaths<R, PPL>(dst, v);
+    } else {
+#pragma unroll
+      for (int i = 0; i < PPL; ++i)
+        if (p0 + i < nP) dst[i] = v[i];
+    }
+  };
+  RateState<R, PPL> st(sc);
+  CreditState<R, PPL> cr[2] = {CreditState<R, PPL>(sc, L, 0, kSimThreads), CreditState<R, PPL>(sc, L, 1, kSimThreads)};
+  for (uint32_t j = 0; j < sc.nT; ++j) {
+    if (j > 0) {
+      drawDate<R, kSimThreads>(sc, L, stream, j, injectedStream, bridge, col);
+      stepRates<R, PPL, kSimThreads>(sc, j, col, sign, st);
+    }
+    writeRates<R, PPL>(sc, cb, j, st, put);
+#pragma unroll
+    for (uint32_t c = 0; c < 2; ++c)
+      if (c < sc.nC) {
+        if (j > 0) stepCredit<R, PPL, kSimThreads>(sc, c, j, col, sign, cr[c]);
+        writeCredit<R, PPL>(cb, c, j, cr[c], put);
+      }
   }
 }
 
@@ -1613,7 +1712,16 @@ cudaError_t launchSimulate(const ScenarioArgs<R>& sc, const CubeArgs<R>& cb, cud
   const size_t date = static_cast<size_t>(L.slots) * cols * sizeof(R);
   L.dates = L.slots <= 8 ? 2 * round : round;
   L.dates = std::min(L.dates, std::max(static_cast<uint32_t>(96 * 1024 / (2 * date)), 1u));
-  size_t smem = 2 * L.dates * date;
+  // Threads that draw and step for themselves once they fill the GPU: the ring's stepping warps hold 64 paths (32 unpaired) of
+  // a CTA's 256 threads, and each credit adds a stepping warp.  Ring against threads in us, 61 dates: unpaired, no assets nor
+  // credits 73 / 76 at 33,333 paths, 185 / 96 at 100,000, 1,558 / 668 at a million; pairs, two stochastic FX rates and a credit
+  // of 8 sub-steps 282 / 329 at 100,000, 547 / 462 at 200,000, 2,623 / 1,966 at a million; the same in double precision 769 /
+  // 731 (whole calls) at 65,536; two credits of 4 sub-steps unpaired 650 / 677 at 200,000, 1,642 / 1,512 at 500,000, of one 392 /
+  // 330 at 200,000.
+  const uint32_t threads = paired ? (sc.nP + 1) / 2 : sc.nP;
+  const uint32_t chains = sc.substeps <= 2 ? sc.nC : sc.nC == 2 ? 12u : 2u * sc.nC;  // several sub-steps: the credits' chains bind
+  const bool walk = threads >= (2u + chains) * 148u * (sizeof(R) == 4 ? 128u : 64u);
+  size_t smem = walk ? static_cast<size_t>(L.slots) * kSimThreads * sizeof(R) : 2 * L.dates * date;
   const size_t table = static_cast<size_t>(sc.nT) * (sc.substeps - 1) * 2 * sizeof(R);
   L.table = sc.nC > 0 && sc.substeps > 1 && table <= 32 * 1024;
   if (L.table) smem += table;
@@ -1625,6 +1733,7 @@ cudaError_t launchSimulate(const ScenarioArgs<R>& sc, const CubeArgs<R>& cb, cud
     kernel<<<(sc.nP + paths - 1) / paths, kSimThreads, smem, stream>>>(sc, cb, L);
     return cudaGetLastError();
   };
+  if (walk) return paired ? go(simulateWalkKernel<R, 2>, 2 * kSimThreads) : go(simulateWalkKernel<R, 1>, kSimThreads);
   return small ? go(simulateKernel<R, 1, 16>, 32) : paired ? go(simulateKernel<R, 2, 32>, 64) : go(simulateKernel<R, 1, 32>, 32);
 }
 
