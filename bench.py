@@ -468,14 +468,19 @@ def xva_batch_leg(ctx, a):
                                             q.num_outputs, q.times, q.reporting)
     fit_s = time.perf_counter() - t0
     # The tile shape: the autotuner's choice on the same batch at 65,536 paths, pinned on the full batch (tuning at
-    # full size would take six executes of the whole batch).
+    # full size would take six executes of the whole batch).  In waves like the full batch: in one wave it would be
+    # split over the dates and have no tile shape.
     small = []
     for p in csa + plain:
         h = p.header.copy()
         h[0], h[15] = min(65536, a.xva_paths), (min(65536, a.xva_paths) + 63) // 64
         small.append(gpu.Plan.from_arrays(h, p.indices, p.params, p.steps, p.terms, p.requests, p.rows_total, p.num_outputs,
                                           p.times, p.reporting))
-    tb = ctx.batch(small)
+    ctx.set_row_budget(sum(p.rows_total * p.num_paths * 4 for p in small) // 10)
+    try:
+        tb = ctx.batch(small)
+    finally:
+        ctx.set_row_budget(0)
     try:
         tb.execute()
         tile = int(tb.info().tile_paths)

@@ -265,7 +265,9 @@ typedef struct zk_batch_info {
   uint64_t table_bytes;          /* bytes of plan tables on the device                            */
   uint64_t row_bytes;            /* bytes of per-path rows (PFE inputs) written per execute        */
   uint64_t kernels_per_execute;  /* kernel launches of one zk_batch_execute                         */
-  uint64_t tile_paths;           /* paths per revalue CTA, chosen by the autotuner at creation     */
+  uint64_t tile_paths;           /* paths per CTA of the walk over the dates (revalueKernel): the autotuner's choice, or
+                                  * the default of 256 in a batch that other kernels revalue (on the tensor cores, or
+                                  * split over the dates), which has none                          */
   uint64_t graph_replay;         /* 1 once executes replay a captured CUDA graph, 0 while eager    */
   uint64_t num_waves;            /* waves of netting sets within the row budget (1 per launch group without) */
   uint64_t num_basis_netting_sets; /* netting sets revalued by the tensor-core basis kernel (zk_context_set_basis) */
@@ -275,7 +277,8 @@ typedef struct zk_batch_info {
 } zk_batch_info;
 
 /* Uploads the plans.  The first zk_batch_execute autotunes the tile shape (paths per revalue CTA) on
- * them, a few timed runs, unless zk_batch_set_tile_paths pinned one. */
+ * them, a few timed runs, unless zk_batch_set_tile_paths pinned one or no netting set is walked.  To time the
+ * shape for a larger batch that will run in waves, create the small one under a row budget that it exceeds too. */
 zk_status zk_batch_create(zk_context* ctx, const zk_plan_view* plans, size_t n, zk_batch** out);
 /* After the tile shape is settled, the execute sequence is captured once in a CUDA graph and replayed (the
  * context's stream must be capturable; otherwise executes stay eager). */

@@ -152,3 +152,24 @@ def test_scenarios_share_the_scratch(ctx):
     for first in (0, 4):
         alone = ctx.run_many(plans[first:first + 4])
         assert all(same(a, b) for a, b in zip(alone, both[first:]))
+
+
+def test_the_tile_shape_is_the_walks(ctx):
+    """A batch that no walk revalues has no tile shape to report; under a row budget it is walked, and tuned."""
+    plans = [ctx.fit_amc(p) if p.amc_degrees else p for p in books(20_000)]
+
+    def tile(budget):
+        ctx.set_row_budget(budget)
+        try:
+            b = ctx.batch(plans)
+        finally:
+            ctx.set_row_budget(0)
+        try:
+            b.execute()
+            return b.info().tile_paths, b.info().num_waves, b.timings()
+        finally:
+            b.close()
+
+    assert tile(0)[:2] == (256, 1)
+    shape, waves, _ = tile(rows_and_partials(plans) // 2)
+    assert waves >= 2 and shape in (128, 256, 512)

@@ -2893,15 +2893,6 @@ zk_status zk_batch_execute(zk_batch* b) {
       bool termByTerm = false;
       for (const auto& L : b->b->launches) termByTerm = termByTerm || (L.basisCount < L.planIdx.size() && !L.split.on);
       if (termByTerm) autotune(*b->b);
-      // A batch split over the dates has no walk to time, but callers take its shape for a larger batch, whose waves are
-      // walked: the shape that the walk of such plans is fastest at (24 netting sets with Bermudans and their uncollateralised
-      // twins, 65,536 paths: 68 ms at 512 paths a CTA; the large XVA batch 9.5 s at 512 and 12.3 s at 256).
-      bool bermudans = !termByTerm, fits = true;
-      for (const auto& L : b->b->launches) {
-        bermudans = bermudans && L.split.on && !L.lean;
-        fits = fits && revalueSmemBytes(L.stateWordsMax, L.perTrade, false, 4) <= 200 * 1024;
-      }
-      if (bermudans && fits) setTileShape(*b->b, 4);
       b->tuned = true;
     }
     if (!b->eager && (!b->graph || b->graphPpt != b->b->ppt) && !captureExecute(b)) b->eager = true;

@@ -204,7 +204,8 @@ class Batch:
         check(lib().zk_batch_execute(self.handle), self.ctx.handle)
 
     def set_tile_paths(self, tile_paths: int) -> None:
-        """Pins the tile shape (paths per revalue CTA: 128, 256 or 512) instead of the autotuned one."""
+        """Pins the tile shape of the walk over the dates (paths per revalue CTA: 128, 256 or 512) instead of the
+        autotuned one; kernels without one ignore it."""
         check(lib().zk_batch_set_tile_paths(self.handle, tile_paths), self.ctx.handle)
 
     def timings(self) -> np.ndarray:
