@@ -2,8 +2,8 @@
 // src/gpu/fused_kernels.cpp:538-563 and :565-771; CPU mirror finishFused,
 // src/gpu/fused_reference.cpp:468-607).
 //
-// reduce: one thread per (date, statistic) sums the per-tile partials in tile order with a
-// compensated double-precision sum, so the result does not depend on scheduling.
+// reduce: the per-tile partials of each (date, statistic) in tile order, in 32 segments of compensated double-precision
+// sums added in order, so the result depends neither on scheduling nor on the launch's other plans.
 //
 // row statistics: one CTA per request.  Quantiles are the *exact* empirical quantile interpolated
 // between order statistics k = floor(p (n - 1)) and k + 1, as ccr::quantile does
@@ -601,43 +601,47 @@ __global__ void __launch_bounds__(kRowThreads, 6) rowStatsKernel(const RowJob<R>
 // two, w0 for four), absent warps past the last path counting as 0, so it has the same bits for every tile
 // shape; the groups are then summed in path order with a compensated double sum.
 //
-// One CTA per 32 columns (date, statistic), kSegs warps over consecutive segments of the groups, each a compensated sum of
-// its own with four groups' loads in flight; the segments are added in order, compensated too.  (One thread walked all groups
+// One CTA per 32 columns (date, statistic), the groups in kSegs consecutive segments, each a compensated sum of its own with
+// four groups' loads in flight; the segments are added in order, compensated too.  Always kSegs of them, so that a plan's
+// sums do not depend on what else is in the launch; kWarps warps share them.  (One thread walked all groups
 // of a column: 129 us for 12 netting sets at 33,333 paths and 1,155 us for 100 at
 // 250,000; now 18 and 889.)
-template <typename R, int PPT, int kSegs>
-__global__ void __launch_bounds__(32 * kSegs) reduceKernel(const ReduceJob<R>* __restrict__ jobs) {
+constexpr int kSegs = 32;
+template <typename R, int PPT, int kWarps>
+__global__ void __launch_bounds__(32 * kWarps) reduceKernel(const ReduceJob<R>* __restrict__ jobs) {
   __shared__ double segSum[kSegs][32], segComp[kSegs][32];
   const ReduceJob<R> J = jobs[blockIdx.y];
-  const uint32_t lane = threadIdx.x & 31u, seg = threadIdx.x >> 5, i = blockIdx.x * 32u + lane;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, i = blockIdx.x * 32u + lane;
   if (blockIdx.x * 32u >= J.n) return;
   // A job with pad 1 or 2 has partials of 32 or 64 paths whatever the batch's shape (the basis kernel's: 64).
   const uint32_t ppt = J.pad == 1u || J.pad == 2u ? J.pad : static_cast<uint32_t>(PPT);
   const uint32_t units = 4 / ppt, unitPaths = 32 * ppt, col = min(i, J.n - 1);
   const uint32_t count = (J.nP + unitPaths - 1) / unitPaths;  // partials
-  double sum = 0.0, comp = 0.0;
-  auto add = [&](R g) {
-    const double yv = static_cast<double>(g) - comp;
-    const double tv = sum + yv;
-    comp = (tv - sum) - yv;
-    sum = tv;
-  };
-  const uint32_t t0 = static_cast<uint32_t>(static_cast<uint64_t>(J.numTiles) * seg / kSegs);
-  const uint32_t t1 = static_cast<uint32_t>(static_cast<uint64_t>(J.numTiles) * (seg + 1) / kSegs);
   const R* __restrict__ P = J.partials + col;
   auto unit = [&](uint32_t u) { return u < count ? __ldg(P + static_cast<size_t>(u) * J.n) : R(0); };
+#pragma unroll 1
+  for (uint32_t seg = warp * (kSegs / kWarps); seg < (warp + 1) * (kSegs / kWarps); ++seg) {
+    double sum = 0.0, comp = 0.0;
+    const uint32_t t0 = static_cast<uint32_t>(static_cast<uint64_t>(J.numTiles) * seg / kSegs);
+    const uint32_t t1 = static_cast<uint32_t>(static_cast<uint64_t>(J.numTiles) * (seg + 1) / kSegs);
 #pragma unroll 4
-  for (uint32_t t = t0; t < t1; ++t) {
-    const uint32_t u = t * units;
-    R g;
-    if (ppt == 1) g = (unit(u) + unit(u + 1)) + (unit(u + 2) + unit(u + 3));
-    else if (ppt == 2) g = unit(u) + unit(u + 1);
-    else g = unit(u);
-    add(g);
+    for (uint32_t t = t0; t < t1; ++t) {
+      const uint32_t u = t * units;
+      R g;
+      if (ppt == 1) g = (unit(u) + unit(u + 1)) + (unit(u + 2) + unit(u + 3));
+      else if (ppt == 2) g = unit(u) + unit(u + 1);
+      else g = unit(u);
+      const double yv = static_cast<double>(g) - comp;
+      const double tv = sum + yv;
+      comp = (tv - sum) - yv;
+      sum = tv;
+    }
+    // An infinite last group leaves the sum infinite and its compensation NaN, which no later group takes up.
+    segSum[seg][lane] = sum, segComp[seg][lane] = seg == kSegs - 1 && isinf(sum) ? 0.0 : comp;
   }
-  segSum[seg][lane] = sum, segComp[seg][lane] = comp;
   __syncthreads();
-  if (seg != 0 || i >= J.n) return;
+  if (warp != 0 || i >= J.n) return;
+  double sum = segSum[0][lane], comp = segComp[0][lane];
   for (int s = 1; s < kSegs; ++s) {  // sum - comp is the segment's sum to more than double precision
     const double yv = (segSum[s][lane] - segComp[s][lane]) - comp;
     const double tv = sum + yv;
@@ -653,9 +657,9 @@ template <typename R>
 cudaError_t launchReduce(const ReduceJob<R>* jobs, uint32_t numJobs, uint32_t maxN, int ppt, cudaStream_t stream) {
   if (numJobs == 0 || maxN == 0) return cudaSuccess;
   const dim3 grid((maxN + 31) / 32, numJobs);
-  // 32 segments where the columns alone leave the GPU idle, 8 where they fill it.
+  // 32 warps, a segment each, where the columns alone leave the GPU idle, 8 where they fill it.
   const bool few = static_cast<uint64_t>(grid.x) * grid.y < 148u * 8u;
-  auto go = [&](auto kernel, int segs) { kernel<<<grid, 32 * segs, 0, stream>>>(jobs); };
+  auto go = [&](auto kernel, int warps) { kernel<<<grid, 32 * warps, 0, stream>>>(jobs); };
   switch (ppt) {
     case 1: few ? go(reduceKernel<R, 1, 32>, 32) : go(reduceKernel<R, 1, 8>, 8); break;
     case 2: few ? go(reduceKernel<R, 2, 32>, 32) : go(reduceKernel<R, 2, 8>, 8); break;
