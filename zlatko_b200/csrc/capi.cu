@@ -904,13 +904,27 @@ void planSplit(Batch<R>& B, typename Batch<R>::Launch& L, size_t most) {
     S.bermsMax = std::max(S.bermsMax, P.nBerm);
   }
   if (S.decides.size() > 65535) return;
+  // An item's cost counts its term records (a generic record as three) and a date's own work.
+  auto cost = [](const uint32_t* d) { return (d[2] - d[0]) + (d[3] - d[2]) + 3 * (d[4] - d[3]) / 2 + (d[5] - d[4]) + 6; };
+  uint64_t total = 0;
+  bool anyFull = false, anyCsa = false;
+  for (size_t k = 0; k < n; ++k) {
+    const auto& P = B.plans[L.planIdx[nb + k]];
+    anyFull = anyFull || full(P), anyCsa = anyCsa || P.hasCsa;
+    for (uint32_t j = 0; j < nT; ++j) total += cost(&P.dates[8 * static_cast<size_t>(j)]);
+  }
   // revalueKernel fills the GPU with a CTA per 128 to 512 paths of every netting set, and writes no values: without AMC
-  // terms it is the faster one from about a million paths x netting sets on (12 netting sets: 1,490 us against 1,026 here
-  // at 33,333 paths, 3.1 ms both at 100,000, 12.4 ms against 15.4 at 500,000).  With AMC terms it never is (24 + 24 netting
-  // sets, 800 trades, 65,536 paths: 66 ms against 28).
-  bool anyFull = false;
-  for (size_t k = 0; k < n; ++k) anyFull = anyFull || full(B.plans[L.planIdx[nb + k]]);
-  if (!anyFull && static_cast<uint64_t>(nP) * n > (1u << 20)) return;
+  // terms it is the faster one from some number of paths x netting sets on -- later the more a date has to compute (the
+  // split's extra traffic weighs less, and one CTA's walk over it more), and later without margin calls.  Where the two met
+  // on 121 dates with margin calls, and the line: 150,000 (3 trades in one netting set; 150,000), 450,000 (30 in one;
+  // 335,000), 550,000 (36 in 12; 560,000), 700,000 (150 in one; 690,000), a million (119 in 12; 740,000); without, on 61 dates,
+  // from 180,000 (3 in one) to beyond two million (120 in 40).  Between the line and where they meet either is within 10%; with
+  // one line at a million, 3 trades on 700,000 paths took 956 us split and 655 walked.  In double precision the split is
+  // ahead up to there (3 trades on 800,000 paths 12.9 ms against 13.2, 30 trades on 100,000 2.5 against 3.0).  With AMC
+  // terms the walk never is faster (24 + 24 netting sets, 800 trades, 65,536 paths: 66 ms against 28).
+  double line = 1048576.0;
+  if (sizeof(R) == 4) line = std::min(line, (anyCsa ? 5e4 : 1e5) * std::sqrt(static_cast<double>(total) / nT));
+  if (!anyFull && static_cast<double>(nP) * static_cast<double>(n) > line) return;
   // One slab's values take 1 GB, or 256 paths' where those are more (slabs of 64 MB, which would stay in the L2, cost 15% in
   // their tails), and less where `most` leaves less.
   const size_t tile = n * nT * sizeof(R) * 256, tiles = std::min<size_t>((nP + 255u) / 256u, std::max<size_t>((size_t(1) << 30) / tile, 1));
@@ -918,14 +932,7 @@ void planSplit(Batch<R>& B, typename Batch<R>::Launch& L, size_t most) {
   if (fit == 0) return;
   S.slab = static_cast<uint32_t>(fit) * 256u;
   S.valsBytes = tile * fit;
-  // Runs of dates of about equal work, enough of them for several CTAs per SM and slab: an item's cost counts its term
-  // records (a generic record as three) and a date's own work.
-  auto cost = [](const uint32_t* d) { return (d[2] - d[0]) + (d[3] - d[2]) + 3 * (d[4] - d[3]) / 2 + (d[5] - d[4]) + 6; };
-  uint64_t total = 0;
-  for (size_t k = 0; k < n; ++k) {
-    const auto& P = B.plans[L.planIdx[nb + k]];
-    for (uint32_t j = 0; j < nT; ++j) total += cost(&P.dates[8 * static_cast<size_t>(j)]);
-  }
+  // Runs of dates of about equal work, enough of them for several CTAs per SM and slab.
   S.ppt = static_cast<uint64_t>(S.slab) * total < (1ull << 25) ? 1 : 2;
   // 32 paths per CTA of settleKernel while they run in one wave (11.5 us against 20 at 2,000 paths), 64 beyond (384 against
   // 412 us at 12 x 33,333).
