@@ -542,11 +542,16 @@ __device__ __forceinline__ double mulRn(double a, double b) { return __dmul_rn(a
 __device__ __forceinline__ float addRn(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double addRn(double a, double b) { return __dadd_rn(a, b); }
 
-// The fixing that a generic record (1 / the period's length in c) sets from its date's short rate.
+// The fixing that a generic record (c, A, B) sets from its date's short rate.
 template <typename R>
-__device__ __forceinline__ R genericFixing(const R (&rec)[8], R x) {
-  return (rec[3] * fastExp(-rec[4] * x) - R(1)) / rec[2];
+__device__ __forceinline__ R genericFixing(R c, R A, R B, R x) {
+  return (A * fastExp(-B * x) - R(1)) / c;
 }
+
+// a e + b f with one product fused, the same one in every kernel (left to the compiler, the walk and the split differed in
+// double precision).
+__device__ __forceinline__ float bondPair(float a, float e, float b, float f) { return fmaf(a, e, b * f); }
+__device__ __forceinline__ double bondPair(double a, double e, double b, double f) { return fma(b, f, a * e); }
 
 // The netting set's value on date j of a thread's PPT paths (value), from the date's lowered runs [d0, d1), and the
 // fixings and exercise states the date sets.  state: the fixings [slot][PPT][kTile]; the exercise index of Bermudan b
@@ -587,10 +592,10 @@ __device__ __forceinline__ void revalueDate(const NsArgs<R>& A, const CubeArgs<R
     for (int i = 0; i < PPT; ++i) value[i] = fma(fma(r.x, fix(slot, i), r.y), termExp(r.z, x[i]), value[i]);
   }
 #pragma unroll 2
-  for (uint32_t u = d0.y; u < d0.z; ++u) {  // bonds, two per record (which product is fused is written out: kernels differed in FP64)
+  for (uint32_t u = d0.y; u < d0.z; ++u) {  // bonds, two per record
     const R4 r = ld4(table + 4 * u);
 #pragma unroll
-    for (int i = 0; i < PPT; ++i) value[i] += fma(r.x, termExp(r.y, x[i]), r.z * termExp(r.w, x[i]));
+    for (int i = 0; i < PPT; ++i) value[i] += bondPair(r.x, termExp(r.y, x[i]), r.z, termExp(r.w, x[i]));
   }
   for (uint32_t u = d0.z; u < d0.w; ++u) {  // asset forwards: (c, A, asset)
     const R4 r = ld4(table + 4 * u);
@@ -650,7 +655,7 @@ __device__ __forceinline__ void revalueDate(const NsArgs<R>& A, const CubeArgs<R
         break;
       case kSetFixing:
 #pragma unroll
-        for (int i = 0; i < PPT; ++i) fix(slot, i) = genericFixing(rec, x[i]);
+        for (int i = 0; i < PPT; ++i) fix(slot, i) = genericFixing(c, rec[3], rec[4], x[i]);
         break;
       case kOption: {
         const R p3 = rec[7];
@@ -1195,16 +1200,15 @@ __global__ void __launch_bounds__(kTile, (sizeof(R) == 8 ? 4 : kLean ? 8 : 6)) v
     for (int i = 0; i < PPT; ++i) state[(q * PPT + i) * kTile + tid] = R(0);
   for (uint32_t q = I.preBegin; q < I.preEnd; ++q) {
     const uint2 f = __ldg(pre + q);  // fixing record, date
+    const auto r = ld4(A.table + 4 * static_cast<size_t>(f.x));
     R x[PPT];
     load(static_cast<size_t>(f.y & ~kGenericFixing) * nP, x);
-    if (f.y & kGenericFixing) {
-      R rec[8];
-      loadTerm(A.table + 4 * static_cast<size_t>(f.x), rec);
+    if (f.y & kGenericFixing) {  // (code, slot, c, A), (B, ...)
+      const R B = __ldg(A.table + 4 * static_cast<size_t>(f.x) + 4);
 #pragma unroll
-      for (int i = 0; i < PPT; ++i) state[(asUint(rec[1]) * PPT + i) * kTile + tid] = genericFixing(rec, x[i]);
+      for (int i = 0; i < PPT; ++i) state[(asUint(r.y) * PPT + i) * kTile + tid] = genericFixing(r.z, r.w, B, x[i]);
       continue;
     }
-    const auto r = ld4(A.table + 4 * static_cast<size_t>(f.x));
 #pragma unroll
     for (int i = 0; i < PPT; ++i) state[(asUint(r.w) * PPT + i) * kTile + tid] = (r.x * termExp(r.y, x[i]) - R(1)) * r.z;
   }
