@@ -173,3 +173,16 @@ def test_the_tile_shape_is_the_walks(ctx):
     assert tile(0)[:2] == (256, 1)
     shape, waves, _ = tile(rows_and_partials(plans) // 2)
     assert waves >= 2 and shape in (128, 256, 512)
+
+
+def test_exercises_out_of_date_order_are_walked(ctx):
+    """A plan whose exercise indices do not follow their dates cannot be decided ahead of the values: it takes the walk."""
+    p = ctx.fit_amc(books(1001)[1])
+    t = p.terms.reshape(-1, 8).copy()
+    code = t[:, 0].astype(np.int64)
+    hit = np.isin(code & 15, (6, 8, 9))  # policies, and the bonds and coupons after an exercise
+    last = (code[hit] >> 12).max()
+    t[hit, 0] = (code[hit] & 0xFFF) | ((last - (code[hit] >> 12)) << 12)
+    p.terms = t.reshape(-1)
+    assert last == 2 and kernels(ctx, [p]) == 1 + 1 + 2
+    check_sums(p, ctx.run(p)[0], restated.run_plan(p)[0], 2e-4)
