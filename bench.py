@@ -869,7 +869,8 @@ def main():
             "roofline_row_stats": {"bound": "hbm", "achieved": row_bytes / (float(np.mean(rows_ms)) / 1e3) / 1e9, "peak": peak,
                                    "unit": "GB/s", "frac": row_bytes / (float(np.mean(rows_ms)) / 1e3) / 1e9 / peak,
                                    "note": "row-statistics kernel: algorithmic bytes = every exposure row read once; the exact "
-                                           "quantile reads a row up to three times (min/max of a sample, histogram, bracket)"},
+                                           "quantile reads a row once and a sixteenth of it twice (a window placed by a sample), twice where the "
+                                           "window would not fit, three times where it misses"},
             # the term-by-term kernel's SFU rate (one ex2 per bond-like term and path); with the basis kernel the
             # book's exponentials are the basis columns', far fewer, and this rate does not describe the kernel
             "roofline_mufu": ({"bound": "sfu", "achieved": exp_per_launch / fused_s / 1e9 if C_ex2 else None,

@@ -28,8 +28,7 @@ namespace {
 
 constexpr int kFitThreads = 256;
 constexpr int kFitWarps = kFitThreads / 32;
-constexpr int kMoments1 = 4;     // count, sum x, sum x^2, sum y
-constexpr int kMoments2 = 6;     // count, sum x, sum x^2, sum s, sum s^2, sum y
+constexpr int kMoments2 = 6;     // count, sum x, sum x^2, sum s, sum s^2, sum y (one regressor: count, sum x, sum x^2, sum y)
 constexpr int kGram1 = 14;       // 10 Gram entries (lower triangle, degree 3) + 4 right-hand sides
 // The two-regressor basis: its Gram entries are the mixed moments sum z^a w^b, a + b <= 6 (28 of them, where the
 // lower triangle of 10 functions has 55 entries), plus the 10 right-hand sides: one pass of 38 sums.

@@ -18,9 +18,11 @@ namespace zk {
 
 namespace {
 
-// Parts of a batch in the weight gradients (three layers: 144 CTAs), up to kGradRows rows.  The tensor core's FP32 accumulation
-// over one chain and over parts differ by about 1e-9 of the gradient's norm per row (9e-6 at 8,192 rows, 1.5e-5 at 12,288); larger batches keep the
-// one chain, and with it their results (131,072 rows: 29.3 ms before, 4.4 now).
+// Parts of a batch in the weight gradients (three layers: 144 CTAs), up to kGradRows rows; a larger batch is one part, one
+// CTA and one chain of FP32 accumulation per layer.  Parts are the faster and the more exact form at every size: against the
+// FP64 network at the same bf16 roundings the largest error of a layer's gradient is 2.6e-5 (chain) and 2.4e-5 (parts) of its
+// norm at 9,217 rows, 2.3e-4 and 7.9e-6 at 131,072 (4.4 ms and 1.15).  The line only keeps the results of larger batches what
+// they were: there the two forms differ by more than 2e-5 of the norm.
 constexpr uint32_t kGradParts = 48, kGradRows = 9216;
 
 // A row of 128 bf16 as 16-byte loads, f(j, value) in order.

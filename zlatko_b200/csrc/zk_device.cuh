@@ -140,7 +140,8 @@ struct NsArgs {
   uint32_t manyBerm;       // more than 4 Bermudans: exercise indices in shared memory, bytes [nBerm][PPT][kTile]
   uint32_t stepStride;     // values per row of `steps`
   uint32_t moreRows;       // some row besides the exposure rows and the exercise rows
-  // AMC state pass (zk_amc_states, zk_fit_amc): x / deflator [date][path] and exercise values [row][path].
+  // AMC state pass (zk_amc_states, zk_fit_amc): x / deflator [date][path] and exercise values [row][path].  The exercise
+  // programs (decideKernel) write sinkEx only: x and the deflator stay in the factor cube, where sinkX and sinkD then point.
   R* sinkX;
   R* sinkD;
   R* sinkEx;
