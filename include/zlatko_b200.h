@@ -93,7 +93,8 @@ zk_status zk_context_set_stream(zk_context* ctx, void* stream);
  * statistics follow its revalue launch, and the outputs are the same bits as in one wave.  (The reference's
  * kernels keep every netting set's rows, EXPO[rows][P], at once: fused_exposure.hpp:214-216.)  The values of a
  * revaluation split over the dates take what the budget leaves beside the rows, in fewer paths at a time, and where it
- * leaves too little the netting sets are revalued date after date without them: the same bits either way. */
+ * leaves too little the netting sets are revalued date after date without them: the same bits either way.  The
+ * fit's realised values (zk_fit_amc) keep within it too, down to one row per Bermudan. */
 zk_status zk_context_set_row_budget(zk_context* ctx, uint64_t bytes);
 /* Which netting sets of a call or batch run on the tensor-core basis kernel: single-precision plans of bonds,
  * floating coupons, FX forwards and options, with no CSA or a cash CSA looking back at most one date and no rows

@@ -291,8 +291,8 @@ class Context:
         return sums, values, r[: plan.rows_total * plan.num_paths].reshape(plan.rows_total, plan.num_paths)
 
     def set_row_budget(self, nbytes: int) -> None:
-        """zk_context_set_row_budget: device bytes for per-path rows and partials at once (0: automatic); books
-        beyond it run in waves of netting sets with the same results."""
+        """zk_context_set_row_budget: device bytes for per-path rows, partials and the scratch of the split revaluation
+        and of the AMC fit at once (0: automatic); books beyond it run in waves of netting sets with the same results."""
         check(lib().zk_context_set_row_budget(self.handle, int(nbytes)), self.handle)
 
     BASIS_AUTO, BASIS_OFF, BASIS_ALL = 0, 1, 2
